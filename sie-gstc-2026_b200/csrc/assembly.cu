@@ -50,6 +50,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "phase.cuh"
 
 namespace sieb200 {
 
@@ -147,12 +148,6 @@ __global__ void near_pairs_kernel(const FaceGeom* __restrict__ geom, int nf, flo
     }
 }
 
-template <int NK, bool TK>
-struct Moments {
-    cplx S0[NK], Sp[NK][3], Sq[NK][3], Spq[NK];
-    cplx T0[TK ? NK : 1], Tp[TK ? NK : 1][3], Tq[TK ? NK : 1][3], Tpq[TK ? NK : 1][3];
-};
-
 __device__ __forceinline__ void warp_sum(double& v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -191,344 +186,415 @@ __device__ __forceinline__ void green_reg(double R, double k, cplx& G, cplx& g) 
     g = K * i4p;
 }
 
-template <int NK, bool TK>
-__device__ __forceinline__ void accumulate(Moments<NK, TK>& M, const d3& pl, const d3& ql,
-                                           double pq, const d3& pxq, double ww, int a,
-                                           cplx G, cplx g) {
-    const cplx Gw = G * ww;
-    M.S0[a] += Gw;
-    M.Sp[a][0] += Gw * pl.x; M.Sp[a][1] += Gw * pl.y; M.Sp[a][2] += Gw * pl.z;
-    M.Sq[a][0] += Gw * ql.x; M.Sq[a][1] += Gw * ql.y; M.Sq[a][2] += Gw * ql.z;
-    M.Spq[a] += Gw * pq;
-    if (TK) {
-        const cplx gw = g * ww;
-        M.T0[a] += gw;
-        M.Tp[a][0] += gw * pl.x; M.Tp[a][1] += gw * pl.y; M.Tp[a][2] += gw * pl.z;
-        M.Tq[a][0] += gw * ql.x; M.Tq[a][1] += gw * ql.y; M.Tq[a][2] += gw * ql.z;
-        M.Tpq[a][0] += gw * pxq.x; M.Tpq[a][1] += gw * pxq.y; M.Tpq[a][2] += gw * pxq.z;
-    }
+__device__ __forceinline__ d3 normalize3(d3 a) {
+    const double inv = 1.0 / sqrt(dot3(a, a));
+    return a * inv;
 }
 
-// Regular (or extracted-kernel) double quadrature of all face pairs (m, n)
-// with m in [m0, m1). Output blocks: NB = NK (TL only) or 2*NK (TL then TK),
-// each 3x3 complex, per pair at pairs[((m-m0)*nf + n) * NB*9].
-// SPLIT: blockIdx.y picks one of the NK wavenumbers and the CTA accumulates
-// that one only. The geometry of a point pair (R, 1/R, p.q, p x q) is then
-// formed once per wavenumber instead of once, but the moments of one
-// wavenumber (18 complex) fit in half the registers, so two CTAs share an SM
-// and the FP64 pipe sees twice the warps; each wavenumber's sums run in the
-// same order as without the split.
-template <int NK, bool TK, bool SPLIT = false>
-__global__ void __launch_bounds__(kWarps * 32, SPLIT ? 2 : 1)
-pair_regular_kernel(const FaceGeom* __restrict__ geom, const d3* __restrict__ qp,
-                    const float* __restrict__ qw_g, int Q, int nf, int m0, double k0, double k1,
-                    float thr, cplx* __restrict__ pairs) {
-    constexpr int NB = TK ? 2 * NK : NK;
-    constexpr int NKC = SPLIT ? 1 : NK;  // wavenumbers accumulated by this CTA
-    const int a_base = SPLIT ? (int)blockIdx.y : 0;
-    __shared__ d3 s_tp[kMaxQ], s_tl[kMaxQ];
-    __shared__ double s_w[kMaxQ];
-    __shared__ d3 s_sp[kWarps][kMaxQ], s_sl[kWarps][kMaxQ];
+__device__ __forceinline__ d3 face_normal(const FaceGeom& g) {
+    return normalize3(cross3(g.v[1] - g.v[0], g.v[2] - g.v[0]));
+}
 
-    const int m = m0 + blockIdx.x;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const FaceGeom& gm = geom[m];
-    const d3 cm = gm.c;
-    for (int t = threadIdx.x; t < Q; t += blockDim.x) {
-        const d3 r = qp[(size_t)m * Q + t];
-        s_tp[t] = r;
-        s_tl[t] = r - cm;
-        s_w[t] = (double)qw_g[t];
+// The line form's unit normal: cross product divided by its length
+// (dunavant_quadrature.cuh:521-525), and twice the area.
+__device__ __forceinline__ d3 face_normal_div(const FaceGeom& g) {
+    const d3 c = cross3(g.v[1] - g.v[0], g.v[2] - g.v[0]);
+    const double l = sqrt(dot3(c, c));
+    return mk3(c.x / l, c.y / l, c.z / l);
+}
+
+// ------------------------------------------------- regular quadrature ----
+// Double quadrature of the Green kernel over a face pair (m test, n source).
+// Inner sums per test point p, in source coordinates q about the centroid:
+//   S0 = sum_q w G, Sq = sum_q w G q,  T0 = sum_q w g, Tq = sum_q w g q
+// (g R is the gradient factor, R = r_p - r_q). Everything the 3 x 3 blocks
+// need is linear in these, so the test point is folded in once per p, into
+// one of two sets of moments:
+//   RWG testing (TL, TK):
+//     TL_ji = l_j l_i [ 1/4 (Spq - Sp.B_i - A_j.Sq + (A_j.B_i) S0) - S0/k^2 ]
+//     TK_ji = l_j l_i / 4 [ Tpq.d - Tp.(B x d) - Tq.(d x A) + ((A x B).d) T0 ],
+//     d = v_j - v_i; Tpq = sum p x Tq, the others plain products with w_p, p.
+//   n x RWG testing (surface form B of nTL / nTK, dunavant_quadrature.cuh:342-480),
+//   tau_j = t_p - t_j, t_p = p x n_m, t_j = A_j x n_m:
+//     nTL = 1/4 (tau . rho_ni) G - 1/(2 k^2) tau . (g R),
+//     nTK = 1/4 (tau x rho_ni) . (g R)   (not on the coincident face);
+//     sum G tau.rho       = Stq - St.B - t_j.Sq + (t_j.B) S0
+//     sum g tau.R         = TtR - t_j.TR
+//     sum g (tau x rho).R = U0 - B.V1 - t_j.V2 + (t_j x B).TR
+//   with, per p and P = r_p - c_n: TR = T0 P - Tq, U0 = (P x t_p).Tq,
+//   V1 = TR x t_p, V2 = Tq x P.
+// NT: number of T sums: 0 (TL only), NK (one per wavenumber), or 1 with
+// NK = 2, where the consumer needs TK1 + TK2 only (T-PMCHWT) and the two
+// wavenumbers' g are added before they are accumulated.
+template <int NK, int NT>
+struct PointSums {
+    cplx S0[NK], Sq[NK][3];
+    cplx T0[NT ? NT : 1], Tq[NT ? NT : 1][3];
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int a = 0; a < NK; ++a) S0[a] = Sq[a][0] = Sq[a][1] = Sq[a][2] = cx(0, 0);
+#pragma unroll
+        for (int a = 0; a < (NT ? NT : 1); ++a) T0[a] = Tq[a][0] = Tq[a][1] = Tq[a][2] = cx(0, 0);
     }
-    __syncthreads();
-    const double kall[2] = {k0, k1};
-    double kk[NKC];
+    // G and g of wavenumber a already carry the source weight.
+    __device__ __forceinline__ void add(const cplx (&G)[NK], const cplx (&g)[NK], double qx, double qy, double qz) {
 #pragma unroll
-    for (int a = 0; a < NKC; ++a) kk[a] = kall[a_base + a];
-    const int QQ = Q * Q;
-
-    for (int n = warp; n < nf; n += kWarps) {
-        const FaceGeom& gn = geom[n];
-        const d3 cn = gn.c;
-        for (int t = lane; t < Q; t += 32) {
-            const d3 r = ldg3(&qp[(size_t)n * Q + t]);
-            s_sp[warp][t] = r;
-            s_sl[warp][t] = r - cn;
+        for (int a = 0; a < NK; ++a) {
+            S0[a] += G[a];
+            Sq[a][0].re = fma(G[a].re, qx, Sq[a][0].re); Sq[a][0].im = fma(G[a].im, qx, Sq[a][0].im);
+            Sq[a][1].re = fma(G[a].re, qy, Sq[a][1].re); Sq[a][1].im = fma(G[a].im, qy, Sq[a][1].im);
+            Sq[a][2].re = fma(G[a].re, qz, Sq[a][2].re); Sq[a][2].im = fma(G[a].im, qz, Sq[a][2].im);
         }
-        __syncwarp();
-        const bool regular = centroid_distance(gm, gn) < thr;  // warp-uniform
-        const bool coinc = gm.idx[0] == gn.idx[0] && gm.idx[1] == gn.idx[1] &&
-                           gm.idx[2] == gn.idx[2];
-
-        Moments<NKC, TK> M;
 #pragma unroll
-        for (int a = 0; a < NKC; ++a) {
-            M.S0[a] = cx(0, 0); M.Spq[a] = cx(0, 0);
+        for (int t = 0; t < NT; ++t) {
+            cplx s = g[t];
+            if (NT < NK) {
 #pragma unroll
-            for (int c = 0; c < 3; ++c) { M.Sp[a][c] = cx(0, 0); M.Sq[a][c] = cx(0, 0); }
-            if (TK) {
-                M.T0[a] = cx(0, 0);
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    M.Tp[a][c] = cx(0, 0); M.Tq[a][c] = cx(0, 0); M.Tpq[a][c] = cx(0, 0);
-                }
+                for (int a = 1; a < NK; ++a) s += g[a];
             }
+            T0[t] += s;
+            Tq[t][0].re = fma(s.re, qx, Tq[t][0].re); Tq[t][0].im = fma(s.im, qx, Tq[t][0].im);
+            Tq[t][1].re = fma(s.re, qy, Tq[t][1].re); Tq[t][1].im = fma(s.im, qy, Tq[t][1].im);
+            Tq[t][2].re = fma(s.re, qz, Tq[t][2].re); Tq[t][2].im = fma(s.im, qz, Tq[t][2].im);
         }
+    }
+};
 
-        for (int idx = lane; idx < QQ; idx += 32) {
-            const int p = idx / Q, q = idx - p * Q;
-            const d3 rp = s_tp[p], rq = s_sp[warp][q];
-            const d3 pl = s_tl[p], ql = s_sl[warp][q];
-            const double ww = s_w[p] * s_w[q];
-            const d3 Rv = rp - rq;
-            const double R = sqrt(Rv.x * Rv.x + Rv.y * Rv.y + Rv.z * Rv.z);
-            const double pq = dot3(pl, ql);
-            const d3 pxq = TK ? cross3(pl, ql) : mk3(0, 0, 0);
-            if (!regular) {
-                if (R < 1e-12) continue;
-                const double inv_R = 1.0 / R;
-                const double i4pR = 1.0 / (4.0 * kPi * R);
+// Totals of one pair: S = S0, Sp (St), Sq, Spq (Stq); T = T0, Tp, Tq, Tpq
+// (RWG) or TR, TtR, U0, V1, V2 (n x RWG).
+template <int NK, int NT, bool ROT>
+struct PairSums {
+    static constexpr int NTM = ROT ? 11 : 10;
+    cplx S[NK][8], T[NT ? NT : 1][NTM];
+    __device__ __forceinline__ void clear() {
 #pragma unroll
-                for (int a = 0; a < NKC; ++a) {
-                    cplx G, g;
-                    green_std(R, inv_R, i4pR, kk[a], G, g);
-                    accumulate<NKC, TK>(M, pl, ql, pq, pxq, ww, a, G, g);
-                }
+        for (int a = 0; a < NK; ++a)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) S[a][e] = cx(0, 0);
+#pragma unroll
+        for (int a = 0; a < (NT ? NT : 1); ++a)
+#pragma unroll
+            for (int e = 0; e < NTM; ++e) T[a][e] = cx(0, 0);
+    }
+    // Folds test point p in: u = p (RWG) or t_p (n x RWG), P = r_p - c_n.
+    __device__ __forceinline__ void fold(const PointSums<NK, NT>& I, double w, d3 u, d3 P) {
+#pragma unroll
+        for (int a = 0; a < NK; ++a) {
+            const cplx s0 = I.S0[a] * w, qx = I.Sq[a][0] * w, qy = I.Sq[a][1] * w, qz = I.Sq[a][2] * w;
+            S[a][0] += s0;
+            S[a][1] += s0 * u.x; S[a][2] += s0 * u.y; S[a][3] += s0 * u.z;
+            S[a][4] += qx; S[a][5] += qy; S[a][6] += qz;
+            S[a][7] += qx * u.x + qy * u.y + qz * u.z;
+        }
+#pragma unroll
+        for (int a = 0; a < NT; ++a) {
+            const cplx t0 = I.T0[a] * w, qx = I.Tq[a][0] * w, qy = I.Tq[a][1] * w, qz = I.Tq[a][2] * w;
+            if (!ROT) {
+                T[a][0] += t0;
+                T[a][1] += t0 * u.x; T[a][2] += t0 * u.y; T[a][3] += t0 * u.z;
+                T[a][4] += qx; T[a][5] += qy; T[a][6] += qz;
+                T[a][7] += qz * u.y - qy * u.z;
+                T[a][8] += qx * u.z - qz * u.x;
+                T[a][9] += qy * u.x - qx * u.y;
             } else {
-#pragma unroll
-                for (int a = 0; a < NKC; ++a) {
-                    cplx G, g;
-                    green_reg(R, kk[a], G, g);
-                    accumulate<NKC, TK>(M, pl, ql, pq, pxq, ww, a, G, g);
-                }
+                const cplx rx = t0 * P.x - qx, ry = t0 * P.y - qy, rz = t0 * P.z - qz;
+                const d3 c = cross3(P, u);
+                T[a][0] += rx; T[a][1] += ry; T[a][2] += rz;
+                T[a][3] += rx * u.x + ry * u.y + rz * u.z;
+                T[a][4] += qx * c.x + qy * c.y + qz * c.z;
+                T[a][5] += ry * u.z - rz * u.y;
+                T[a][6] += rz * u.x - rx * u.z;
+                T[a][7] += rx * u.y - ry * u.x;
+                T[a][8] += qy * P.z - qz * P.y;
+                T[a][9] += qz * P.x - qx * P.z;
+                T[a][10] += qx * P.y - qy * P.x;
             }
         }
-        // Butterfly: every lane ends with the totals.
+    }
+    // Sums over groups of 2^lg neighbouring lanes (every lane gets the total).
+    __device__ __forceinline__ void reduce(int lg) {
+        for (int o = 1; o < (1 << lg); o <<= 1) {
 #pragma unroll
-        for (int a = 0; a < NKC; ++a) {
-            warp_sum(M.S0[a]); warp_sum(M.Spq[a]);
+            for (int a = 0; a < NK; ++a)
 #pragma unroll
-            for (int c = 0; c < 3; ++c) { warp_sum(M.Sp[a][c]); warp_sum(M.Sq[a][c]); }
-            if (TK) {
-                warp_sum(M.T0[a]);
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    warp_sum(M.Tp[a][c]); warp_sum(M.Tq[a][c]); warp_sum(M.Tpq[a][c]);
+                for (int e = 0; e < 8; ++e) {
+                    S[a][e].re += __shfl_xor_sync(0xffffffffu, S[a][e].re, o);
+                    S[a][e].im += __shfl_xor_sync(0xffffffffu, S[a][e].im, o);
                 }
+#pragma unroll
+            for (int a = 0; a < NT; ++a)
+#pragma unroll
+                for (int e = 0; e < NTM; ++e) {
+                    T[a][e].re += __shfl_xor_sync(0xffffffffu, T[a][e].re, o);
+                    T[a][e].im += __shfl_xor_sync(0xffffffffu, T[a][e].im, o);
+                }
+        }
+    }
+    // Values of local edges (j, i): tl per wavenumber, tk per T sum.
+    __device__ __forceinline__ void expand(const FaceGeom& gm, const FaceGeom& gn, int j, int i, d3 nm, bool coinc,
+                                           bool form_a, const double (&kk)[NK], cplx (&tl)[NK],
+                                           cplx (&tk)[NT ? NT : 1]) const {
+        const d3 B = gn.A[i];
+        const d3 A = ROT ? cross3(gm.A[j], nm) : gm.A[j];  // t_j for n x RWG testing
+        const double scale = gm.len[j] * gn.len[i];
+        const double AB = dot3(A, B);
+#pragma unroll
+        for (int a = 0; a < NK; ++a) {
+            cplx s = S[a][7];
+            s = s - (S[a][1] * B.x + S[a][2] * B.y + S[a][3] * B.z);
+            s = s - (S[a][4] * A.x + S[a][5] * A.y + S[a][6] * A.z);
+            s += S[a][0] * AB;
+            if (!ROT) {
+                tl[a] = (s * 0.25 - S[a][0] * (1.0 / (kk[a] * kk[a]))) * scale;
+            } else if (form_a) {
+                tl[a] = s * (0.25 * scale);
+            } else {
+                // (ROT keeps one T sum per wavenumber)
+                const cplx* t = T[NT == NK ? a : 0];
+                const cplx g = t[3] - (t[0] * A.x + t[1] * A.y + t[2] * A.z);
+                tl[a] = (s * 0.25 + g * (-0.5 / (kk[a] * kk[a]))) * scale;
             }
         }
-        if (lane < 9) {
-            const int j = lane / 3, i = lane - 3 * j;
-            const d3 A = gm.A[j], B = gn.A[i];
-            const d3 d = gm.fv[j] - gn.fv[i];
-            const double scale = gm.len[j] * gn.len[i];
-            const double AB = dot3(A, B);
-            cplx* out = pairs + ((size_t)blockIdx.x * nf + n) * (NB * 9);
 #pragma unroll
-            for (int a = 0; a < NKC; ++a) {
-                // TL_ji = l_j l_i [ 1/4 (Spq - Sp.B - A.Sq + (A.B) S0) - S0 / k^2 ]
-                cplx t = M.Spq[a];
-                t = t - (M.Sp[a][0] * B.x + M.Sp[a][1] * B.y + M.Sp[a][2] * B.z);
-                t = t - (M.Sq[a][0] * A.x + M.Sq[a][1] * A.y + M.Sq[a][2] * A.z);
-                t += M.S0[a] * AB;
-                const cplx tl = (t * 0.25 - M.S0[a] * (1.0 / (kk[a] * kk[a]))) * scale;
-                out[(a_base + a) * 9 + lane] = tl;
-                if (TK) {
-                    cplx tk = cx(0, 0);
-                    if (!coinc) {
-                        // TK_ji = l_j l_i / 4 [ Tpq.d - (Tp x B).d - (A x Tq).d + ((A x B).d) T0 ]
-                        const d3 BxD = cross3(B, d);   // (Tp x B).d = Tp . (B x d)
-                        const d3 DxA = cross3(d, A);   // (A x Tq).d = Tq . (d x A)
-                        const double axbd = dot3(cross3(A, B), d);
-                        cplx u = M.Tpq[a][0] * d.x + M.Tpq[a][1] * d.y + M.Tpq[a][2] * d.z;
-                        u = u - (M.Tp[a][0] * BxD.x + M.Tp[a][1] * BxD.y + M.Tp[a][2] * BxD.z);
-                        u = u - (M.Tq[a][0] * DxA.x + M.Tq[a][1] * DxA.y + M.Tq[a][2] * DxA.z);
-                        u += M.T0[a] * axbd;
-                        tk = u * (0.25 * scale);
-                    }
-                    out[(NK + a_base + a) * 9 + lane] = tk;
-                }
+        for (int a = 0; a < NT; ++a) {
+            cplx u = cx(0, 0);
+            if (!coinc && !ROT) {
+                const d3 d = gm.fv[j] - gn.fv[i];
+                const d3 BxD = cross3(B, d), DxA = cross3(d, A);
+                u = T[a][7] * d.x + T[a][8] * d.y + T[a][9] * d.z;
+                u = u - (T[a][1] * BxD.x + T[a][2] * BxD.y + T[a][3] * BxD.z);
+                u = u - (T[a][4] * DxA.x + T[a][5] * DxA.y + T[a][6] * DxA.z);
+                u += T[a][0] * dot3(cross3(A, B), d);
+                u = u * (0.25 * scale);
+            } else if (!coinc) {
+                const d3 x = cross3(A, B);
+                u = T[a][4];
+                u = u - (T[a][5] * B.x + T[a][6] * B.y + T[a][7] * B.z);
+                u = u - (T[a][8] * A.x + T[a][9] * A.y + T[a][10] * A.z);
+                u += T[a][0] * x.x + T[a][1] * x.y + T[a][2] * x.z;
+                u = u * (0.25 * scale);
             }
+            tk[a] = u;
         }
-        __syncwarp();
+    }
+};
+
+// Pair blocks: pairs[((m - m0) nf + n) 9 NB + (3 j + i) NB + slot], the NB
+// values of one edge pair adjacent. The regular pass writes its tl to slots
+// s_tl.. and its tk to slots s_tk.. (negative: not kept).
+struct PairOut {
+    cplx* pairs;
+    int NB, s_tl, s_tk;
+};
+template <int NK, int NT>
+__device__ __forceinline__ void put_pair(const PairOut& o, size_t row, int e, const cplx (&tl)[NK],
+                                         const cplx (&tk)[NT ? NT : 1]) {
+    cplx* out = o.pairs + (row * 9 + e) * o.NB;
+    if (o.s_tl >= 0) {
+#pragma unroll
+        for (int a = 0; a < NK; ++a) out[o.s_tl + a] = tl[a];
+    }
+    if (NT > 0 && o.s_tk >= 0) {
+#pragma unroll
+        for (int a = 0; a < NT; ++a) out[o.s_tk + a] = tk[a];
     }
 }
 
-// The same double quadrature with a test point held per lane. Lane l works
-// on test point p (G lanes per point when Q < 32, each taking every G-th
-// source point) and sums over its source points only the moments that do not
-// carry p: per wavenumber S0_p = sum w_q G, Sq_p = sum w_q G q, and for TK
-// T0_p = sum w_q g, Tq_p = sum w_q g q (8 complex for both). The moments
-// with p are folded in once per point,
-//   S0 += w_p S0_p,  Sp += w_p S0_p p,  Sq += w_p Sq_p,  Spq += w_p p.Sq_p,
-//   T0 += w_p T0_p,  Tp += w_p T0_p p,  Tq += w_p Tq_p,  Tpq += w_p p x Tq_p,
-// reduced over the warp and accumulated in shared memory. Per point pair and
-// wavenumber that is 20 FP64 accumulation instructions instead of 40 and no
-// p.q or p x q, and the accumulators fit in half the registers (two CTAs per
-// SM). Each moment is the same sum as in pair_regular_kernel in another
-// order.
-template <int NK, bool TK>
-__global__ void __launch_bounds__(kWarps * 32, 2)
-pair_regular_pq_kernel(const FaceGeom* __restrict__ geom, const d3* __restrict__ qp,
-                       const float* __restrict__ qw_g, int Q, int nf, int m0, double k0, double k1,
-                       float thr, cplx* __restrict__ pairs) {
-    constexpr int NB = TK ? 2 * NK : NK;
-    constexpr int NM = TK ? 18 : 8;  // complex moments per wavenumber
-    __shared__ d3 s_tp[kMaxQ], s_tl[kMaxQ];
-    __shared__ double s_w[kMaxQ];
-    __shared__ d3 s_sp[kWarps][kMaxQ], s_sl[kWarps][kMaxQ];
-    __shared__ cplx s_tot[kWarps][NK * NM];
+struct RuleWeights {
+    double w[kMaxQ], w4[kMaxQ];  // weights, weights / (4 pi)
+};
+static RuleWeights make_rule_weights(const float* w, int Q) {
+    RuleWeights r{};
+    for (int q = 0; q < Q; ++q) {
+        r.w[q] = (double)w[q];
+        r.w4[q] = r.w[q] / (4.0 * kPi);
+    }
+    return r;
+}
+constexpr int kFarWarps = 4;
 
-    const int m = m0 + blockIdx.x;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const FaceGeom& gm = geom[m];
-    const d3 cm = gm.c;
-    for (int t = threadIdx.x; t < Q; t += blockDim.x) {
-        const d3 r = qp[(size_t)m * Q + t];
-        s_tp[t] = r;
-        s_tl[t] = r - cm;
-        s_w[t] = (double)qw_g[t];
+// Far pairs (centroid distance at or above the extraction threshold): one
+// source face per lane group, 2^lg lanes sharing it (each takes every 2^lg-th
+// test point); a warp works on one test face, the CTA's four warps on
+// `chunk` of them against the CTA's 32 >> lg source faces, whose points sit
+// in shared memory about their centroids.
+// Bound: the FP64 pipe. Per Green value with its moments 52 pipe
+// instructions (TL and TK, one wavenumber; 41 each with two wavenumbers and
+// TK summed): 12 for R and 1/R, 15 for the phase factor, 9 for G and g, 16 to
+// accumulate. What keeps it there:
+//  * one lane holds a pair's moments, so no value crosses lanes unless the
+//    mesh is small (lg > 0) and the 3 x 3 expansion runs on all lanes;
+//  * with RWG testing (ROT = false) the blocks of (m, n) and (n, m) are each
+//    other's transposes and both are written from one evaluation (m <= n);
+//  * phase factors and 1/R without library calls (phase.cuh); BIG falls back
+//    to sincos(k R) for meshes whose phases would not fit its step number.
+// Measured: the 2000-face sphere with 61 points and two wavenumbers 54 ms (212 ms
+// for the kernel this replaces: a warp per ordered pair, a test point per lane, sincos
+// and division from the math library); the 2880-face SIE-GSTC sphere with
+// equal wavenumbers 70 ms (435 ms). The FP64 pipe is busy 64 % of the cycles; what is
+// left is the latency of dependent FP64 instructions: 128 registers per thread (16 warps
+// per SM) gave 75 and 54 ms, unrolling by four 70 and 55 ms, so neither more
+// warps nor more independent points fill it.
+template <int NK, int NT, bool ROT, bool BIG>
+__global__ void __launch_bounds__(kFarWarps * 32, 3)
+far_pairs_kernel(const FaceGeom* __restrict__ geom, const d3* __restrict__ qp, const RuleWeights rw, int Q, int nf,
+                 int m0, int m1, const Wave k0, const Wave k1, float thr, int exact, int form_a, int lg, int chunk,
+                 const PairOut out) {
+    extern __shared__ __align__(16) unsigned char far_smem[];
+    double2* tab = reinterpret_cast<double2*>(far_smem);               // [kTurn][kTurnCopies]
+    double* sq = reinterpret_cast<double*>(tab + kTurn * kTurnCopies);  // [Q][3][nt]
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nt = 32 >> lg;
+    const int n0 = blockIdx.y * nt;
+    const int n_last = min(n0 + nt, nf) - 1;
+    // Test faces of this CTA. Tiles inside the slab's own columns stop at the
+    // diagonal with RWG testing.
+    const bool inside = !ROT && n0 >= m0 && n_last < m1;
+    const int m_end = inside ? n_last + 1 : m1;
+    const int mb = m0 + blockIdx.x * chunk;
+    if (mb >= m_end) return;
+    const int me = min(mb + chunk, m_end);
+
+    fill_turn_table(tab);
+    for (int t = threadIdx.x; t < Q * nt; t += blockDim.x) {
+        const int s = t % nt, q = t / nt, f = min(n0 + s, nf - 1);
+        const d3 r = ldg3(&qp[(size_t)f * Q + q]) - ldg3(&geom[f].c);
+        sq[(q * 3 + 0) * nt + s] = r.x;
+        sq[(q * 3 + 1) * nt + s] = r.y;
+        sq[(q * 3 + 2) * nt + s] = r.z;
     }
     __syncthreads();
-    const double kk[2] = {k0, k1};
-    const int G = Q >= 32 ? 1 : 32 / Q;  // lanes per test point
-    const int PL = 32 / G;               // test points per round
-    const int lp = lane / G, lq = lane - (lane / G) * G;
-    cplx* tot = s_tot[warp];
 
-    for (int n = warp; n < nf; n += kWarps) {
-        const FaceGeom& gn = geom[n];
-        const d3 cn = gn.c;
-        for (int t = lane; t < Q; t += 32) {
-            const d3 r = ldg3(&qp[(size_t)n * Q + t]);
-            s_sp[warp][t] = r;
-            s_sl[warp][t] = r - cn;
-        }
-        for (int t = lane; t < NK * NM; t += 32) tot[t] = cx(0, 0);
-        __syncwarp();
-        const bool regular = centroid_distance(gm, gn) < thr;  // warp-uniform
-        const bool coinc = gm.idx[0] == gn.idx[0] && gm.idx[1] == gn.idx[1] &&
-                           gm.idx[2] == gn.idx[2];
+    const int sub = lane & ((1 << lg) - 1), ln = lane >> lg;
+    const int n = min(n0 + ln, nf - 1);
+    const bool have_n = n0 + ln < nf;
+    const d3 cn = ldg3(&geom[n].c);
+    const double2* my_tab = tab + (lane & (kTurnCopies - 1));
+    const double* my_q = sq + ln;
+    const Wave kv[2] = {k0, k1};
+    double kk[NK];
+#pragma unroll
+    for (int a = 0; a < NK; ++a) kk[a] = kv[a].k;
 
-        for (int p0 = 0; p0 < Q; p0 += PL) {
-            const int p = p0 + lp;
-            const bool act = p < Q;
-            cplx S0[NK], Sq[NK][3], T0[TK ? NK : 1], Tq[TK ? NK : 1][3];
+    for (int m = mb + warp; m < me; m += kFarWarps) {
+        const FaceGeom& gm = geom[m];
+        const bool mirror = !ROT && n >= m0 && n < m1;  // (n, m) lies in this slab too
+        const bool mine = have_n && !(mirror && n < m) && !near_pair(gm, geom[n], thr, exact);
+        if (!__any_sync(0xffffffffu, mine)) continue;
+        const d3 cm = ldg3(&gm.c);
+        d3 nm = mk3(0, 0, 0);
+        if (ROT) nm = form_a ? face_normal_div(gm) : face_normal(gm);
+        PairSums<NK, NT, ROT> tot;
+        tot.clear();
+#pragma unroll 1
+        for (int p = sub; p < Q; p += 1 << lg) {
+            const d3 rp = ldg3(&qp[(size_t)m * Q + p]);
+            const d3 P = rp - cn;
+            PointSums<NK, NT> in;
+            in.clear();
+#pragma unroll 2
+            for (int q = 0; q < Q; ++q) {
+                const double qx = my_q[(q * 3 + 0) * nt], qy = my_q[(q * 3 + 1) * nt], qz = my_q[(q * 3 + 2) * nt];
+                const double dx = P.x - qx, dy = P.y - qy, dz = P.z - qz;
+                const double R2 = fma(dz, dz, fma(dy, dy, dx * dx));
+                double inv = rsqrt_refined(R2);
+                if (tiny_square(R2)) inv = 0.0;  // R < 1e-12: no contribution
+                const double R = R2 * inv;
+                const double W = inv * rw.w4[q];
+                const double i2 = inv * inv;
+                cplx G[NK], g[NK];
 #pragma unroll
-            for (int a = 0; a < NK; ++a) {
-                S0[a] = cx(0, 0);
-#pragma unroll
-                for (int c = 0; c < 3; ++c) Sq[a][c] = cx(0, 0);
-                if (TK) {
-                    T0[a] = cx(0, 0);
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) Tq[a][c] = cx(0, 0);
-                }
-            }
-            if (act) {
-                const d3 rp = s_tp[p];
-                for (int q = lq; q < Q; q += G) {
-                    const d3 rq = s_sp[warp][q], ql = s_sl[warp][q];
-                    const double wq = s_w[q];
-                    const d3 Rv = rp - rq;
-                    const double R = sqrt(Rv.x * Rv.x + Rv.y * Rv.y + Rv.z * Rv.z);
-                    cplx Gk[NK], gk[NK];
-                    if (!regular) {
-                        if (R < 1e-12) continue;
-                        const double inv_R = 1.0 / R;
-                        const double i4pR = 1.0 / (4.0 * kPi * R);
-#pragma unroll
-                        for (int a = 0; a < NK; ++a) green_std(R, inv_R, i4pR, kk[a], Gk[a], gk[a]);
+                for (int a = 0; a < NK; ++a) {
+                    double c, s;
+                    if (BIG) {
+                        sincos(kv[a].k * R, &s, &c);
                     } else {
-#pragma unroll
-                        for (int a = 0; a < NK; ++a) green_reg(R, kk[a], Gk[a], gk[a]);
+                        phase_cs(my_tab, kv[a], R, c, s);
                     }
-#pragma unroll
-                    for (int a = 0; a < NK; ++a) {
-                        const cplx Gw = Gk[a] * wq;
-                        S0[a] += Gw;
-                        Sq[a][0] += Gw * ql.x; Sq[a][1] += Gw * ql.y; Sq[a][2] += Gw * ql.z;
-                        if (TK) {
-                            const cplx gw = gk[a] * wq;
-                            T0[a] += gw;
-                            Tq[a][0] += gw * ql.x; Tq[a][1] += gw * ql.y; Tq[a][2] += gw * ql.z;
-                        }
+                    G[a] = cx(c * W, -s * W);
+                    if (NT > 0) {
+                        // g = (1/R) (1/R + j k) G
+                        const double v = kv[a].k * inv;
+                        g[a] = cx(fma(i2, G[a].re, -(v * G[a].im)), fma(i2, G[a].im, v * G[a].re));
                     }
                 }
+                in.add(G, g, qx, qy, qz);
             }
-            // Fold the test point in, reduce over the warp, accumulate.
-            const d3 pl = act ? s_tl[p] : mk3(0, 0, 0);
-            const double wp = act ? s_w[p] : 0.0;
-            auto put = [&](int idx, cplx v) {
-                warp_sum(v);
-                if (lane == 0) tot[idx] += v;
-            };
-#pragma unroll
-            for (int a = 0; a < NK; ++a) {
-                const int b0 = a * NM;
-                const cplx s0 = S0[a] * wp;
-                const cplx sq[3] = {Sq[a][0] * wp, Sq[a][1] * wp, Sq[a][2] * wp};
-                put(b0 + 0, s0);
-                put(b0 + 1, s0 * pl.x); put(b0 + 2, s0 * pl.y); put(b0 + 3, s0 * pl.z);
-                put(b0 + 4, sq[0]); put(b0 + 5, sq[1]); put(b0 + 6, sq[2]);
-                put(b0 + 7, sq[0] * pl.x + sq[1] * pl.y + sq[2] * pl.z);
-                if (TK) {
-                    const cplx t0 = T0[a] * wp;
-                    const cplx tq[3] = {Tq[a][0] * wp, Tq[a][1] * wp, Tq[a][2] * wp};
-                    put(b0 + 8, t0);
-                    put(b0 + 9, t0 * pl.x); put(b0 + 10, t0 * pl.y); put(b0 + 11, t0 * pl.z);
-                    put(b0 + 12, tq[0]); put(b0 + 13, tq[1]); put(b0 + 14, tq[2]);
-                    // p x Tq
-                    put(b0 + 15, tq[2] * pl.y - tq[1] * pl.z);
-                    put(b0 + 16, tq[0] * pl.z - tq[2] * pl.x);
-                    put(b0 + 17, tq[1] * pl.x - tq[0] * pl.y);
-                }
-            }
+            const d3 pl = rp - cm;
+            tot.fold(in, rw.w[p], ROT ? cross3(pl, nm) : pl, P);
         }
-        __syncwarp();
-        if (lane < 9) {
-            const int j = lane / 3, i = lane - 3 * j;
-            const d3 A = gm.A[j], B = gn.A[i];
-            const d3 d = gm.fv[j] - gn.fv[i];
-            const double scale = gm.len[j] * gn.len[i];
-            const double AB = dot3(A, B);
-            cplx* out = pairs + ((size_t)blockIdx.x * nf + n) * (NB * 9);
-#pragma unroll
-            for (int a = 0; a < NK; ++a) {
-                const cplx* M = tot + a * NM;
-                // TL_ji = l_j l_i [ 1/4 (Spq - Sp.B - A.Sq + (A.B) S0) - S0 / k^2 ]
-                cplx t = M[7];
-                t = t - (M[1] * B.x + M[2] * B.y + M[3] * B.z);
-                t = t - (M[4] * A.x + M[5] * A.y + M[6] * A.z);
-                t += M[0] * AB;
-                out[a * 9 + lane] = (t * 0.25 - M[0] * (1.0 / (kk[a] * kk[a]))) * scale;
-                if (TK) {
-                    cplx tk = cx(0, 0);
-                    if (!coinc) {
-                        const d3 BxD = cross3(B, d);
-                        const d3 DxA = cross3(d, A);
-                        const double axbd = dot3(cross3(A, B), d);
-                        cplx u = M[15] * d.x + M[16] * d.y + M[17] * d.z;
-                        u = u - (M[9] * BxD.x + M[10] * BxD.y + M[11] * BxD.z);
-                        u = u - (M[12] * DxA.x + M[13] * DxA.y + M[14] * DxA.z);
-                        u += M[8] * axbd;
-                        tk = u * (0.25 * scale);
-                    }
-                    out[(NK + a) * 9 + lane] = tk;
-                }
-            }
+        tot.reduce(lg);
+        if (!mine) continue;
+        const FaceGeom& gn = geom[n];
+        const bool coinc = gm.idx[0] == gn.idx[0] && gm.idx[1] == gn.idx[1] && gm.idx[2] == gn.idx[2];
+        const size_t row = (size_t)(m - m0) * nf + n, rowT = (size_t)(n - m0) * nf + m;
+        for (int e = sub; e < 9; e += 1 << lg) {
+            const int j = e / 3, i = e - 3 * j;
+            cplx tl[NK], tk[NT ? NT : 1];
+            tot.expand(gm, gn, j, i, nm, coinc, form_a != 0, kk, tl, tk);
+            put_pair<NK, NT>(out, row, e, tl, tk);
+            if (mirror && n != m) put_pair<NK, NT>(out, rowT, i * 3 + j, tl, tk);
         }
-        __syncwarp();
     }
 }
 
-// Lane slots used by pair_regular_pq_kernel for Q points: its lanes do useful
-// work for this share of their iterations (1 for the flat kernel's Q x Q
-// index space up to the last partial round).
-inline double pq_lane_use(int Q) {
+// Near pairs (list): the same sums with the extracted kernel, one warp per
+// pair: lane groups of 32 / Q lanes share a test point (one lane each from 32
+// points on). With RWG testing a pair whose mirror image lies in the slab is
+// evaluated once (m <= n) and written twice.
+template <int NK, int NT, bool ROT>
+__global__ void __launch_bounds__(128)
+near_regular_kernel(const FaceGeom* __restrict__ geom, const d3* __restrict__ qp, const RuleWeights rw, int Q, int nf,
+                    int m0, int m1, const int2* __restrict__ list, int count, double k0, double k1, int form_a,
+                    const PairOut out) {
+    const int id = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (id >= count) return;
+    const int m = list[id].x, n = list[id].y;
+    const bool mirror = !ROT && n >= m0 && n < m1;
+    if (mirror && n < m) return;
+    const FaceGeom &gm = geom[m], &gn = geom[n];
+    const d3 cm = ldg3(&gm.c), cn = ldg3(&gn.c);
+    d3 nm = mk3(0, 0, 0);
+    if (ROT) nm = form_a ? face_normal_div(gm) : face_normal(gm);
+    const double kv[2] = {k0, k1};
+    double kk[NK];
+#pragma unroll
+    for (int a = 0; a < NK; ++a) kk[a] = kv[a];
     const int G = Q >= 32 ? 1 : 32 / Q, PL = 32 / G;
-    const int rounds = (Q + PL - 1) / PL, iters = (Q + G - 1) / G;
-    return (double)Q * Q / (32.0 * rounds * iters);
+    const int lp = lane / G, lq = lane - lp * G;
+    PairSums<NK, NT, ROT> tot;
+    tot.clear();
+#pragma unroll 1
+    for (int p = lp; p < Q && lp < PL; p += PL) {
+        const d3 rp = ldg3(&qp[(size_t)m * Q + p]);
+        PointSums<NK, NT> in;
+        in.clear();
+#pragma unroll 1
+        for (int q = lq; q < Q; q += G) {
+            const d3 rq = ldg3(&qp[(size_t)n * Q + q]);
+            const d3 Rv = rp - rq, ql = rq - cn;
+            const double R = sqrt(Rv.x * Rv.x + Rv.y * Rv.y + Rv.z * Rv.z);
+            cplx Gk[NK], gk[NK];
+#pragma unroll
+            for (int a = 0; a < NK; ++a) {
+                green_reg(R, kk[a], Gk[a], gk[a]);
+                Gk[a] = Gk[a] * rw.w[q];
+                gk[a] = gk[a] * rw.w[q];
+            }
+            in.add(Gk, gk, ql.x, ql.y, ql.z);
+        }
+        const d3 pl = rp - cm;
+        tot.fold(in, rw.w[p], ROT ? cross3(pl, nm) : pl, rp - cn);
+    }
+    tot.reduce(5);
+    const bool coinc = gm.idx[0] == gn.idx[0] && gm.idx[1] == gn.idx[1] && gm.idx[2] == gn.idx[2];
+    if (lane < 9) {
+        const int j = lane / 3, i = lane - 3 * j;
+        cplx tl[NK], tk[NT ? NT : 1];
+        tot.expand(gm, gn, j, i, nm, coinc, form_a != 0, kk, tl, tk);
+        put_pair<NK, NT>(out, (size_t)(m - m0) * nf + n, lane, tl, tk);
+        if (mirror && n != m) put_pair<NK, NT>(out, (size_t)(n - m0) * nf + m, i * 3 + j, tl, tk);
+    }
 }
 
 // ------------------------------------------------------------ Wilton ----
@@ -536,11 +602,6 @@ struct Pots {
     double phi0, phi2, d;
     d3 phi1b, phi3b, r_pi;
 };
-
-__device__ __forceinline__ d3 normalize3(d3 a) {
-    const double inv = 1.0 / sqrt(dot3(a, a));
-    return a * inv;
-}
 
 // semi_analytic_integrals.cuh:35-92 and 563-667 in one pass.
 __device__ Pots wilton(const d3 r, const d3 tri[3]) {
@@ -607,7 +668,7 @@ template <int NK>
 __global__ void pair_singular_kernel(const FaceGeom* __restrict__ geom, const d3* __restrict__ qp,
                                      const float* __restrict__ qw_g, int Q, int nf, int m0,
                                      const int2* __restrict__ list, int count, double k0,
-                                     double k1, bool with_tk, cplx* __restrict__ pairs) {
+                                     double k1, bool with_tk, bool sum_tk, const PairOut dst) {
     const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (warp_global >= count) return;
@@ -652,8 +713,7 @@ __global__ void pair_singular_kernel(const FaceGeom* __restrict__ geom, const d3
         const int j = lane / 3, i = lane - 3 * j;
         const double as = 1.0 / (4.0 * kPi * gn.area);
         const double s = as * gm.len[j] * gn.len[i];
-        const int NB = with_tk ? 2 * NK : NK;
-        cplx* out = pairs + ((size_t)(mn.x - m0) * nf + mn.y) * (NB * 9);
+        cplx* out = dst.pairs + (((size_t)(mn.x - m0) * nf + mn.y) * 9 + lane) * dst.NB;
         double tlv[NK], tkv[NK];
 #pragma unroll
         for (int a = 0; a < NK; ++a) {
@@ -662,44 +722,13 @@ __global__ void pair_singular_kernel(const FaceGeom* __restrict__ geom, const d3
 #pragma unroll
             for (int t = 0; t < 9; ++t)
                 if (t == lane) { tlv[a] = tl[a][t]; tkv[a] = tk[a][t]; }
-            out[a * 9 + lane].re += tlv[a] * s;
-            if (with_tk) out[(NK + a) * 9 + lane].re += tkv[a] * s;
+            out[dst.s_tl + a].re += tlv[a] * s;
+            if (with_tk) out[dst.s_tk + (sum_tk ? 0 : a)].re += tkv[a] * s;
         }
     }
 }
 
 // ---------------------------------------------- rotated (n x RWG) testing --
-// Surface form B of nTL / nTK (dunavant_quadrature.cuh:342-480) with
-// tau_mj = rho_mj x n_m and the TK kernel vector g R (R = r_p - r_q):
-//   nTL = 1/4 (tau . rho_ni) G - 1/(2 k^2) tau . (g R),
-//   nTK = 1/4 (tau x rho_ni) . (g R)   (not on the coincident face).
-// With tau = t_p - t_j (t_p = p_l x n_m, t_j = A_j x n_m) and
-// rho_ni = q_l - B_i, the nine RWG pairs follow from per-warp moments:
-//   sum G tau.rho        = Stq - St.B - t_j.Sq + (t_j.B) S0
-//   sum g tau.R          = TtR - t_j.TR
-//   sum g (tau x rho).R  = U0 - B.V1 - t_j.V2 + (t_j x B).TR
-// St = sum G t_p, Sq = sum G q_l, Stq = sum G t_p.q_l, TR = sum g R,
-// TtR = sum g t_p.R, U0 = sum g (t_p x q_l).R, V1 = sum g R x t_p,
-// V2 = sum g q_l x R.
-template <int NK, bool NTK>
-struct MomentsN {
-    cplx S0[NK], St[NK][3], Sq[NK][3], Stq[NK];
-    cplx TR[NK][3], TtR[NK];
-    cplx U0[NTK ? NK : 1], V1[NTK ? NK : 1][3], V2[NTK ? NK : 1][3];
-};
-
-__device__ __forceinline__ d3 face_normal(const FaceGeom& g) {
-    return normalize3(cross3(g.v[1] - g.v[0], g.v[2] - g.v[0]));
-}
-
-// The line form's unit normal: cross product divided by its length
-// (dunavant_quadrature.cuh:521-525), and twice the area.
-__device__ __forceinline__ d3 face_normal_div(const FaceGeom& g) {
-    const d3 c = cross3(g.v[1] - g.v[0], g.v[2] - g.v[0]);
-    const double l = sqrt(dot3(c, c));
-    return mk3(c.x / l, c.y / l, c.z / l);
-}
-
 // semi_analytic_integrals.cuh:108-171 (calculate_phi_0, on the testing edges
 // of the line form): an edge whose end is within 1e-9 of r is skipped, and on
 // an edge's line (R0 < 1e-8) the end distances are regularised by 1e-8.
@@ -742,147 +771,6 @@ __device__ double phi0_line(const d3 r, const d3 tri[3]) {
     return phi0;
 }
 
-// Regular (or extracted-kernel) double quadrature of the rotated-testing
-// blocks of all face pairs (m, n), m in [m0, m1). Output per pair: nTL for
-// each wavenumber, then (NTK) nTK for each, 3x3 complex each, in the slots
-// pair_regular_kernel gives TL and TK.
-// FORM_A: the area part of the line form A (dunavant_quadrature.cuh:492-567):
-// nTL without the gradient term (pair_line_kernel adds the testing-edge line
-// integral), n_m as the cross product divided by its length.
-template <int NK, bool NTK, bool FORM_A>
-__global__ void __launch_bounds__(kWarps * 32, 1)
-pair_regular_n_kernel(const FaceGeom* __restrict__ geom, const d3* __restrict__ qp,
-                      const float* __restrict__ qw_g, int Q, int nf, int m0, double k0, double k1,
-                      float thr, int exact, cplx* __restrict__ pairs) {
-    constexpr int NB = NTK ? 2 * NK : NK;
-    __shared__ d3 s_tp[kMaxQ], s_tt[kMaxQ];
-    __shared__ double s_w[kMaxQ];
-    __shared__ d3 s_sp[kWarps][kMaxQ], s_sl[kWarps][kMaxQ];
-
-    const int m = m0 + blockIdx.x;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const FaceGeom& gm = geom[m];
-    const d3 nm = FORM_A ? face_normal_div(gm) : face_normal(gm);
-    for (int t = threadIdx.x; t < Q; t += blockDim.x) {
-        const d3 r = qp[(size_t)m * Q + t];
-        s_tp[t] = r;
-        s_tt[t] = cross3(r - gm.c, nm);
-        s_w[t] = (double)qw_g[t];
-    }
-    __syncthreads();
-    const double kk[2] = {k0, k1};
-    const int QQ = Q * Q;
-
-    for (int n = warp; n < nf; n += kWarps) {
-        const FaceGeom& gn = geom[n];
-        const d3 cn = gn.c;
-        for (int t = lane; t < Q; t += 32) {
-            const d3 r = ldg3(&qp[(size_t)n * Q + t]);
-            s_sp[warp][t] = r;
-            s_sl[warp][t] = r - cn;
-        }
-        __syncwarp();
-        const bool regular = near_pair(gm, gn, thr, exact);  // warp-uniform
-        const bool coinc = gm.idx[0] == gn.idx[0] && gm.idx[1] == gn.idx[1] &&
-                           gm.idx[2] == gn.idx[2];
-
-        MomentsN<NK, NTK> M;
-#pragma unroll
-        for (int a = 0; a < NK; ++a) {
-            M.S0[a] = cx(0, 0); M.Stq[a] = cx(0, 0); M.TtR[a] = cx(0, 0);
-#pragma unroll
-            for (int c = 0; c < 3; ++c) { M.St[a][c] = cx(0, 0); M.Sq[a][c] = cx(0, 0); M.TR[a][c] = cx(0, 0); }
-            if (NTK) {
-                M.U0[a] = cx(0, 0);
-#pragma unroll
-                for (int c = 0; c < 3; ++c) { M.V1[a][c] = cx(0, 0); M.V2[a][c] = cx(0, 0); }
-            }
-        }
-
-        for (int idx = lane; idx < QQ; idx += 32) {
-            const int p = idx / Q, q = idx - p * Q;
-            const d3 rp = s_tp[p], rq = s_sp[warp][q];
-            const d3 tp = s_tt[p], ql = s_sl[warp][q];
-            const double ww = s_w[p] * s_w[q];
-            const d3 Rv = rp - rq;
-            const double R = sqrt(Rv.x * Rv.x + Rv.y * Rv.y + Rv.z * Rv.z);
-            if (!regular && R < 1e-12) continue;
-            const double tq = dot3(tp, ql), tR = dot3(tp, Rv);
-            double u0 = 0.0;
-            d3 v1 = mk3(0, 0, 0), v2 = mk3(0, 0, 0);
-            if (NTK) {
-                u0 = dot3(cross3(tp, ql), Rv);
-                v1 = cross3(Rv, tp);
-                v2 = cross3(ql, Rv);
-            }
-            const double inv_R = regular ? 0.0 : 1.0 / R;
-            const double i4pR = regular ? 0.0 : 1.0 / (4.0 * kPi * R);
-#pragma unroll
-            for (int a = 0; a < NK; ++a) {
-                cplx G, g;
-                if (regular) green_reg(R, kk[a], G, g);
-                else green_std(R, inv_R, i4pR, kk[a], G, g);
-                const cplx Gw = G * ww, gw = g * ww;
-                M.S0[a] += Gw;
-                M.St[a][0] += Gw * tp.x; M.St[a][1] += Gw * tp.y; M.St[a][2] += Gw * tp.z;
-                M.Sq[a][0] += Gw * ql.x; M.Sq[a][1] += Gw * ql.y; M.Sq[a][2] += Gw * ql.z;
-                M.Stq[a] += Gw * tq;
-                M.TR[a][0] += gw * Rv.x; M.TR[a][1] += gw * Rv.y; M.TR[a][2] += gw * Rv.z;
-                M.TtR[a] += gw * tR;
-                if (NTK) {
-                    M.U0[a] += gw * u0;
-                    M.V1[a][0] += gw * v1.x; M.V1[a][1] += gw * v1.y; M.V1[a][2] += gw * v1.z;
-                    M.V2[a][0] += gw * v2.x; M.V2[a][1] += gw * v2.y; M.V2[a][2] += gw * v2.z;
-                }
-            }
-        }
-#pragma unroll
-        for (int a = 0; a < NK; ++a) {
-            warp_sum(M.S0[a]); warp_sum(M.Stq[a]); warp_sum(M.TtR[a]);
-#pragma unroll
-            for (int c = 0; c < 3; ++c) { warp_sum(M.St[a][c]); warp_sum(M.Sq[a][c]); warp_sum(M.TR[a][c]); }
-            if (NTK) {
-                warp_sum(M.U0[a]);
-#pragma unroll
-                for (int c = 0; c < 3; ++c) { warp_sum(M.V1[a][c]); warp_sum(M.V2[a][c]); }
-            }
-        }
-        if (lane < 9) {
-            const int j = lane / 3, i = lane - 3 * j;
-            const d3 tj = cross3(gm.A[j], nm), B = gn.A[i];
-            const double scale = gm.len[j] * gn.len[i];
-            const double tjB = dot3(tj, B);
-            const d3 tjxB = cross3(tj, B);
-            cplx* out = pairs + ((size_t)blockIdx.x * nf + n) * (NB * 9);
-#pragma unroll
-            for (int a = 0; a < NK; ++a) {
-                cplx s = M.Stq[a];
-                s = s - (M.St[a][0] * B.x + M.St[a][1] * B.y + M.St[a][2] * B.z);
-                s = s - (M.Sq[a][0] * tj.x + M.Sq[a][1] * tj.y + M.Sq[a][2] * tj.z);
-                s += M.S0[a] * tjB;
-                if (FORM_A) {
-                    out[a * 9 + lane] = s * (0.25 * scale);
-                } else {
-                    const cplx t = M.TtR[a] - (M.TR[a][0] * tj.x + M.TR[a][1] * tj.y + M.TR[a][2] * tj.z);
-                    out[a * 9 + lane] = (s * 0.25 + t * (-0.5 / (kk[a] * kk[a]))) * scale;
-                }
-                if (NTK) {
-                    cplx u = cx(0, 0);
-                    if (!coinc) {
-                        u = M.U0[a];
-                        u = u - (M.V1[a][0] * B.x + M.V1[a][1] * B.y + M.V1[a][2] * B.z);
-                        u = u - (M.V2[a][0] * tj.x + M.V2[a][1] * tj.y + M.V2[a][2] * tj.z);
-                        u += M.TR[a][0] * tjxB.x + M.TR[a][1] * tjxB.y + M.TR[a][2] * tjxB.z;
-                        u = u * (0.25 * scale);
-                    }
-                    out[(NK + a) * 9 + lane] = u;
-                }
-            }
-        }
-        __syncwarp();
-    }
-}
-
 // Singular (extracted) part of the rotated-testing blocks of the near pairs,
 // added to the pair blocks. One warp per pair, lanes over outer points.
 // Surface form B (dunavant_quadrature.cuh:889-1040), per outer point with
@@ -899,7 +787,7 @@ __global__ void pair_singular_n_kernel(const FaceGeom* __restrict__ geom, const 
                                        const float* __restrict__ qw_g, int Q, int nf, int m0,
                                        const int2* __restrict__ list, int count, double k0,
                                        double k1, bool with_ntk, const float* __restrict__ gl_t,
-                                       const float* __restrict__ gl_w, int NG, cplx* __restrict__ pairs) {
+                                       const float* __restrict__ gl_w, int NG, const PairOut dst) {
     const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (warp_global >= count) return;
@@ -975,8 +863,7 @@ __global__ void pair_singular_n_kernel(const FaceGeom* __restrict__ geom, const 
         const int j = lane / 3, i = lane - 3 * j;
         const double as = 1.0 / (4.0 * kPi * gn.area);
         const double s = as * gm.len[j] * gn.len[i];
-        const int NB = with_ntk ? 2 * NK : NK;
-        cplx* out = pairs + ((size_t)(mn.x - m0) * nf + mn.y) * (NB * 9);
+        cplx* out = dst.pairs + (((size_t)(mn.x - m0) * nf + mn.y) * 9 + lane) * dst.NB;
         const double edges = gm.len[j] * gn.len[i];
         const double ls = FORM_A ? 1.0 / (8.0 * kPi * gm.area * gn.area) : 0.0;
         double lj = 0.0;
@@ -990,11 +877,11 @@ __global__ void pair_singular_n_kernel(const FaceGeom* __restrict__ geom, const 
             for (int t = 0; t < 9; ++t)
                 if (t == lane) { tlv = tl[a][t]; tkv = tk[a][t]; }
             if (FORM_A) {
-                out[a * 9 + lane].re += tlv * (edges * as) + edges * ls * lj / (kk[a] * kk[a]);
-                if (with_ntk) out[(NK + a) * 9 + lane].re += tkv * (edges * as);
+                out[dst.s_tl + a].re += tlv * (edges * as) + edges * ls * lj / (kk[a] * kk[a]);
+                if (with_ntk) out[dst.s_tk + a].re += tkv * (edges * as);
             } else {
-                out[a * 9 + lane].re += tlv * s;
-                if (with_ntk) out[(NK + a) * 9 + lane].re += tkv * s;
+                if (dst.s_tl >= 0) out[dst.s_tl + a].re += tlv * s;
+                if (with_ntk) out[dst.s_tk + a].re += tkv * s;
             }
         }
     }
@@ -1013,7 +900,7 @@ __global__ void __launch_bounds__(kWarps * 32)
 pair_line_kernel(const FaceGeom* __restrict__ geom, const d3* __restrict__ qp,
                  const float* __restrict__ qw_g, int Q, int nf, int m0, double k0, double k1,
                  float thr, int exact, const float* __restrict__ gl_t, const float* __restrict__ gl_w,
-                 int NG, int NB, cplx* __restrict__ pairs) {
+                 int NG, const PairOut dst) {
     __shared__ double s_w[kMaxQ];
     __shared__ double s_t[20], s_wl[20];
     const int m = m0 + blockIdx.x;
@@ -1084,9 +971,9 @@ pair_line_kernel(const FaceGeom* __restrict__ geom, const d3* __restrict__ qp,
                 for (int a = 0; a < NK; ++a) acc[a] += (M0[e][a] * c0 + M1[e][a] * c1) * geomf;
             }
             const double scale = gm.len[j] * gn.len[i];
-            cplx* out = pairs + ((size_t)blockIdx.x * nf + n) * (NB * 9);
+            cplx* out = dst.pairs + (((size_t)blockIdx.x * nf + n) * 9 + lane) * dst.NB + dst.s_tl;
 #pragma unroll
-            for (int a = 0; a < NK; ++a) out[a * 9 + lane] += acc[a] * (scale / (kk[a] * kk[a]));
+            for (int a = 0; a < NK; ++a) out[a] += acc[a] * (scale / (kk[a] * kk[a]));
         }
         __syncwarp();
     }
@@ -1335,12 +1222,19 @@ __global__ void tensor_grad_kernel(const FaceGeom* __restrict__ geom, const d3* 
 }
 
 // ------------------------------------------------------------ gather ----
+// Slots of a pair block: TL per wavenumber, then TK per wavenumber (T-EFIE
+// and N-EFIE: TL only); one TL and one TK where both regions have the same
+// wavenumber; TL per wavenumber and TK1 + TK2 (T-PMCHWT, which needs no more);
+// the one nTK of N-MFIE.
+enum { PAIR_FULL = 0, PAIR_SAME_K = 1, PAIR_SUM_TK = 2, PAIR_TK_ONLY = 3 };
+
 struct GatherParams {
     int formulation;
     int variant;  // 0 tangential testing; 1 N-EFIE / N-PMCHWT; 2 N-MFIE / N-Muller
     int nf, ne;
     int m0, m1;
     int NB;
+    int layout;  // the NB slots of an edge pair: PAIR_* below
     cplx c_jj[2], c_mm[2];
     double s_jm, s_mm;
     double me, me2;  // mass scales (float eta0, eta0^2)
@@ -1363,6 +1257,10 @@ __device__ __forceinline__ bool edge_pair_block(const cplx* __restrict__ pairs, 
 #pragma unroll
     for (int a = 0; a < 2; ++a)
         if (it[a] >= 0 && it[a] / 3 >= P.m0 && it[a] / 3 < P.m1) any = true;
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) blk[r][c] = cx(0, 0);
     if (!any) return false;
 
     cplx acc[4] = {cx(0, 0), cx(0, 0), cx(0, 0), cx(0, 0)};
@@ -1380,10 +1278,10 @@ __device__ __forceinline__ bool edge_pair_block(const cplx* __restrict__ pairs, 
         for (int b = 0; b < 2; ++b) {
             if (is[b] < 0) continue;
             const int n = is[b] / 3, i = is[b] - 3 * n;
-            const cplx* pb = pairs + ((size_t)(m - P.m0) * P.nf + n) * (P.NB * 9) + j * 3 + i;
+            const cplx* pb = pairs + (((size_t)(m - P.m0) * P.nf + n) * 9 + j * 3 + i) * P.NB;
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-                if (k < P.NB) acc[k] += pb[k * 9];
+                if (k < P.NB) acc[k] += pb[k];
             if (P.formulation == SIEB200_GSTC && m == n) {
                 has_mass = true;
                 const cplx* mb = mass + (size_t)m * 72 + j * 3 + i;
@@ -1393,10 +1291,12 @@ __device__ __forceinline__ bool edge_pair_block(const cplx* __restrict__ pairs, 
             if (P.variant == 2 && m == n) gram_acc += P.gram[(size_t)m * 9 + j * 3 + i];
         }
     }
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) blk[r][c] = cx(0, 0);
+    if (P.layout == PAIR_SAME_K) {
+        acc[3] = acc[2] = acc[1];
+        acc[1] = acc[0];
+    } else if (P.layout == PAIR_TK_ONLY) {
+        acc[1] = acc[0];
+    }
     if (P.formulation == SIEB200_PEC_EFIE && P.variant == 2) {
         // N-MFIE (pec_solver.cu:171-240): 1/2 Gram on the same face, - nTK2.
         blk[0][0] = cx(0.5 * gram_acc, 0.0) - acc[1];
@@ -1412,7 +1312,7 @@ __device__ __forceinline__ bool edge_pair_block(const cplx* __restrict__ pairs, 
         blk[1][0] = mj * P.s_jm;
         blk[1][1] = jj * (-P.s_mm);
     } else if (P.formulation == SIEB200_PMCHWT) {
-        // acc: TL1, TL2, TK1, TK2
+        // acc: TL1, TL2, TK1, TK2 (or TL1, TL2, TK1 + TK2, 0)
         const cplx tk = acc[2] + acc[3];
         const cplx jm = tk * P.s_jm;
         blk[0][0] = P.c_jj[0] * acc[0] + P.c_jj[1] * acc[1];
@@ -1441,7 +1341,9 @@ __device__ __forceinline__ int region_count(int formulation) {
 
 // One thread per (test edge te, source edge se); te fastest for coalesced
 // column-major stores. Sums the incident face pairs with the test face in
-// [m0, m1) and adds into Z (zeroed before the first slab).
+// [m0, m1). ADD: adds into Z (zeroed before the first of several slabs); else
+// the only slab, and every entry of Z is stored once without being read.
+template <bool ADD>
 __global__ void gather_kernel(const cplx* __restrict__ pairs, const cplx* __restrict__ mass,
                               const int* __restrict__ inc, GatherParams P, cplx* __restrict__ Z,
                               int64_t ldz) {
@@ -1449,14 +1351,17 @@ __global__ void gather_kernel(const cplx* __restrict__ pairs, const cplx* __rest
     const int se = blockIdx.y * blockDim.y + threadIdx.y;
     if (te >= P.ne || se >= P.ne) return;
     cplx blk[4][4];
-    if (!edge_pair_block(pairs, mass, inc, P, te, se, blk)) return;
+    if (!edge_pair_block(pairs, mass, inc, P, te, se, blk) && ADD) return;
     const int64_t E = P.ne;
     const int nr = region_count(P.formulation);
 #pragma unroll
     for (int c = 0; c < 4; ++c)
 #pragma unroll
         for (int r = 0; r < 4; ++r)
-            if (c < nr && r < nr) Z[(te + r * E) + (se + c * E) * ldz] += blk[r][c];
+            if (c < nr && r < nr) {
+                cplx* z = Z + (te + r * E) + (se + c * E) * ldz;
+                *z = ADD ? *z + blk[r][c] : blk[r][c];
+            }
 }
 
 // Matrix-free product: y += (the slab's rows of Z) x without storing Z. One
@@ -1564,6 +1469,59 @@ static int prepare_faces(sieb200_ctx* ctx, const sieb200_mesh& mesh, const float
     return SIEB200_OK;
 }
 
+// The far kernel's phase step number has to fit 32 bits with room for its
+// remainder: k times the mesh's extent below kPhaseMax (about 2e8 steps).
+static bool far_phase_fits(const sieb200_mesh& mesh, double k) {
+    double lo[3], hi[3];
+    for (int c = 0; c < 3; ++c) lo[c] = hi[c] = mesh.vertices[c];
+    for (int64_t v = 1; v < mesh.num_vertices; ++v)
+        for (int c = 0; c < 3; ++c) {
+            lo[c] = std::min(lo[c], mesh.vertices[3 * v + c]);
+            hi[c] = std::max(hi[c], mesh.vertices[3 * v + c]);
+        }
+    const double d = (hi[0] - lo[0]) + (hi[1] - lo[1]) + (hi[2] - lo[2]);
+    return k * d < kPhaseMax;
+}
+
+struct FarLaunch {
+    const FaceGeom* geom;
+    const d3* qp;
+    const RuleWeights* rw;
+    int Q, nf, m0, m1;
+    double k0, k1;
+    float thr;
+    int exact;
+    bool form_a;
+    PairOut out;
+    cudaStream_t st;
+};
+
+template <int NK, int NT, bool ROT>
+static int launch_far(const FarLaunch& f, bool big) {
+    // Lanes per pair: one where the mesh gives every SM several rounds of
+    // warps (a warp takes 32 pairs then), else up to the test point count.
+    const int rows = f.m1 - f.m0;
+    const double pairs = (double)rows * f.nf * (ROT ? 1.0 : 0.5);
+    int lg = 0;
+    while ((2 << lg) <= std::min(32, std::max(1, f.Q)) && pairs * (1 << lg) / 32.0 < 8192.0) ++lg;
+    const int nt = 32 >> lg;
+    // Test faces per CTA: enough point pairs to pay for the table and the
+    // staged points, few enough that the last wave stays short.
+    const double warp_pairs = pairs * (1 << lg) / 32.0;
+    int per_warp = std::max(1, std::min(16, 2048 / std::max(1, f.Q * f.Q >> lg)));
+    per_warp = (int)std::max(1.0, std::min((double)per_warp, warp_pairs / 8192.0));
+    const int chunk = kFarWarps * per_warp;
+    const int smem = (int)(sizeof(double2) * kTurn * kTurnCopies + sizeof(double) * 3 * (size_t)f.Q * nt);
+    const dim3 grid((unsigned)((rows + chunk - 1) / chunk), (unsigned)((f.nf + nt - 1) / nt));
+    auto* kernel = big ? far_pairs_kernel<NK, NT, ROT, true> : far_pairs_kernel<NK, NT, ROT, false>;
+    SIEB_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    kernel<<<grid, kFarWarps * 32, smem, f.st>>>(f.geom, f.qp, *f.rw, f.Q, f.nf, f.m0, f.m1, make_wave(f.k0),
+                                                 make_wave(f.k1), f.thr, f.exact, f.form_a ? 1 : 0, lg, chunk, f.out);
+    SIEB_NOTE_LAUNCH();
+    SIEB_TRY_CUDA(cudaGetLastError());
+    return SIEB200_OK;
+}
+
 // Assembly of Z (dx == nullptr) or, matrix-free, y = Z x with the same face
 // pair blocks contracted against x slab by slab instead of written to Z.
 static int assemble_or_apply(sieb200_ctx* ctx, const sieb200_mesh& mesh, const sieb200_options& opt,
@@ -1611,13 +1569,23 @@ static int assemble_or_apply(sieb200_ctx* ctx, const sieb200_mesh& mesh, const s
         SIEB_TRY_CUDA(cudaGetLastError());
     }
 
-    // Slabs of test faces bounded by the pair-block workspace. Blocks per
-    // pair: TL (or nTL) per wavenumber, then TK (or nTK) where the
-    // formulation uses it (all but T-EFIE and N-EFIE).
-    const bool tk = !(opt.formulation == SIEB200_PEC_EFIE && variant != 2);
-    const int NK = ap.nk;
-    const int NB = tk ? 2 * NK : NK;
-    const int exact = (opt.formulation == SIEB200_PEC_EFIE && variant != 0) ? 1 : 0;
+    // Slabs of test faces bounded by the pair-block workspace. Values per
+    // edge pair (PAIR_*): TL (or nTL) per distinct wavenumber, then TK (or
+    // nTK) where the formulation uses it (all but T-EFIE and N-EFIE).
+    const bool pec = opt.formulation == SIEB200_PEC_EFIE;
+    const bool rot = variant != 0;
+    const bool tk = !(pec && variant != 2);
+    const bool same_k = ap.nk == 2 && ap.k[0] == ap.k[1];
+    const int NK = same_k ? 1 : ap.nk;  // distinct wavenumbers
+    int layout = PAIR_FULL;
+    if (pec && variant == 2) layout = PAIR_TK_ONLY;
+    else if (same_k) layout = PAIR_SAME_K;
+    else if (opt.formulation == SIEB200_PMCHWT && !rot) layout = PAIR_SUM_TK;
+    PairOut po;
+    po.NB = layout == PAIR_SUM_TK ? 3 : (layout == PAIR_TK_ONLY ? 1 : (tk ? 2 * NK : NK));
+    po.s_tl = layout == PAIR_TK_ONLY ? -1 : 0;
+    po.s_tk = !tk ? -1 : (layout == PAIR_TK_ONLY ? 0 : NK);
+    const int exact = (pec && rot) ? 1 : 0;
     // Line form A of nTL (N-EFIE, N-PMCHWT, N-Muller): Gauss-Legendre rule on
     // [0, 1] after the Dunavant rule in the rule buffer.
     const int NG = ap.line_points;
@@ -1629,26 +1597,28 @@ static int assemble_or_apply(sieb200_ctx* ctx, const sieb200_mesh& mesh, const s
                    "Gauss-Legendre point count must be in [1, 20]");
         SIEB_TRY_CUDA(cudaMemcpyAsync(dgl, glt, sizeof(glt), cudaMemcpyHostToDevice, st));
     }
-    const size_t pair_bytes = sizeof(cplx) * 9 * NB;
+    const size_t pair_bytes = sizeof(cplx) * 9 * po.NB;
     size_t budget = (size_t)8 << 30;
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) budget = std::min(budget, free_b / 3);
-    int slab = (int)std::max<size_t>(1, std::min<size_t>(nf, budget / (pair_bytes * nf)));
+    const int slab = (int)std::max<size_t>(1, std::min<size_t>(nf, budget / (pair_bytes * nf)));
     SIEB_RETURN_IF(ctx->pairs.reserve(pair_bytes * (size_t)slab * nf));
-    cplx* pairs = ctx->pairs.as<cplx>();
+    po.pairs = ctx->pairs.as<cplx>();
     SIEB_RETURN_IF(ctx->counter.reserve(sizeof(unsigned long long)));
     unsigned long long* counter = ctx->counter.as<unsigned long long>();
 
+    const bool one_slab = slab >= nf;
     if (dx)
         SIEB_TRY_CUDA(cudaMemsetAsync(dy, 0, sizeof(cplx) * N, st));
-    else
+    else if (!one_slab)
         SIEB_TRY_CUDA(cudaMemset2DAsync(dZ, sizeof(cplx) * ldz, 0, sizeof(cplx) * N, N, st));
 
     GatherParams gp;
     gp.formulation = opt.formulation;
     gp.nf = nf;
     gp.ne = ne;
-    gp.NB = NB;
+    gp.NB = po.NB;
+    gp.layout = layout;
     gp.c_jj[0] = ap.c_jj[0]; gp.c_jj[1] = ap.c_jj[1];
     gp.c_mm[0] = ap.c_mm[0]; gp.c_mm[1] = ap.c_mm[1];
     gp.s_jm = ap.s_jm; gp.s_mm = ap.s_mm;
@@ -1658,119 +1628,109 @@ static int assemble_or_apply(sieb200_ctx* ctx, const sieb200_mesh& mesh, const s
     gp.eps_f = ap.eps_f; gp.mu_f = ap.mu_f;
     gp.gram = dgram;
 
-    // SIEB200_ASM_SPLIT=1: the two-wavenumber regular pass as one CTA per
-    // (face, wavenumber), two CTAs per SM. It raises the FP64 pipe's busy
-    // share (51 % against 47 %) but issues 37 % more instructions (the pair
-    // geometry twice), so the default is one CTA per face over both.
-    const char* split_env = getenv("SIEB200_ASM_SPLIT");
-    const bool split_wavenumbers = split_env && split_env[0] == '1';
-    // Test point per lane (pair_regular_pq_kernel) where its lanes stay busy
-    // (>= 75 % of their iterations); SIEB200_ASM_PER_POINT=0 keeps the flat
-    // point-pair kernel everywhere.
-    const char* pp_env = getenv("SIEB200_ASM_PER_POINT");
-    const bool per_point = !(pp_env && pp_env[0] == '0') && pq_lane_use(Q) >= 0.75;
+    // The regular pass: T-PMCHWT with two wavenumbers in one launch (R and
+    // the TK sums are shared); otherwise one launch per distinct wavenumber,
+    // which keeps a pair's moments in registers.
+    const RuleWeights rw = make_rule_weights(wts, Q);
+    const int passes = layout == PAIR_SUM_TK ? 1 : NK;
+    const bool big = !far_phase_fits(mesh, std::max(ap.k[0], ap.k[1]));
+    // The near list of a slab, filled in one pass where the buffer kept from
+    // earlier slabs and calls holds it.
+    SIEB_RETURN_IF(ctx->near_list.reserve(sizeof(int2) * 32 * (size_t)slab));
     for (int m0 = 0; m0 < nf; m0 += slab) {
         const int m1 = std::min(nf, m0 + slab);
         const int rows = m1 - m0;
-        if (variant != 0 && opt.formulation == SIEB200_PEC_EFIE && !tk && form_a)
-            pair_regular_n_kernel<1, false, true><<<rows, kWarps * 32, 0, st>>>(
-                geom, qp, dw, Q, nf, m0, ap.k[1], ap.k[1], ap.threshold, exact, pairs);
-        else if (variant != 0 && opt.formulation == SIEB200_PEC_EFIE && !tk)
-            pair_regular_n_kernel<1, false, false><<<rows, kWarps * 32, 0, st>>>(
-                geom, qp, dw, Q, nf, m0, ap.k[1], ap.k[1], ap.threshold, exact, pairs);
-        else if (variant != 0 && opt.formulation == SIEB200_PEC_EFIE)
-            pair_regular_n_kernel<1, true, false><<<rows, kWarps * 32, 0, st>>>(
-                geom, qp, dw, Q, nf, m0, ap.k[1], ap.k[1], ap.threshold, exact, pairs);
-        else if (variant != 0 && form_a)
-            pair_regular_n_kernel<2, true, true><<<rows, kWarps * 32, 0, st>>>(
-                geom, qp, dw, Q, nf, m0, ap.k[0], ap.k[1], ap.threshold, exact, pairs);
-        else if (variant != 0)
-            pair_regular_n_kernel<2, true, false><<<rows, kWarps * 32, 0, st>>>(
-                geom, qp, dw, Q, nf, m0, ap.k[0], ap.k[1], ap.threshold, exact, pairs);
-        else if (opt.formulation == SIEB200_PEC_EFIE && per_point)
-            pair_regular_pq_kernel<1, false><<<rows, kWarps * 32, 0, st>>>(
-                geom, qp, dw, Q, nf, m0, ap.k[1], ap.k[1], ap.threshold, pairs);
-        else if (opt.formulation == SIEB200_PEC_EFIE)
-            pair_regular_kernel<1, false><<<rows, kWarps * 32, 0, st>>>(
-                geom, qp, dw, Q, nf, m0, ap.k[1], ap.k[1], ap.threshold, pairs);
-        else if (split_wavenumbers)
-            pair_regular_kernel<2, true, true><<<dim3(rows, 2), kWarps * 32, 0, st>>>(
-                geom, qp, dw, Q, nf, m0, ap.k[0], ap.k[1], ap.threshold, pairs);
-        else if (per_point)
-            pair_regular_pq_kernel<2, true><<<rows, kWarps * 32, 0, st>>>(
-                geom, qp, dw, Q, nf, m0, ap.k[0], ap.k[1], ap.threshold, pairs);
-        else
-            pair_regular_kernel<2, true><<<rows, kWarps * 32, 0, st>>>(
-                geom, qp, dw, Q, nf, m0, ap.k[0], ap.k[1], ap.threshold, pairs);
-        SIEB_NOTE_LAUNCH();
-        SIEB_TRY_CUDA(cudaGetLastError());
+        const long long span = (long long)rows * nf;
+        const int nb = (int)((span + 255) / 256);
+        unsigned long long count = 0;
+        for (int attempt = 0; attempt < 2; ++attempt) {
+            const unsigned long long capacity = ctx->near_list.bytes / sizeof(int2);
+            SIEB_TRY_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st));
+            near_pairs_kernel<<<nb, 256, 0, st>>>(geom, nf, ap.threshold, exact, m0, m1, counter,
+                                                  ctx->near_list.as<int2>(), capacity);
+            SIEB_NOTE_LAUNCH();
+            SIEB_TRY_CUDA(cudaGetLastError());
+            SIEB_TRY_CUDA(cudaMemcpyAsync(&count, counter, sizeof(count), cudaMemcpyDeviceToHost, st));
+            SIEB_TRY_CUDA(cudaStreamSynchronize(st));
+            if (count <= capacity) break;
+            SIEB_RETURN_IF(ctx->near_list.reserve(sizeof(int2) * count));
+        }
+        const int2* list = ctx->near_list.as<int2>();
+        const int near_threads = 128;
+        const unsigned near_blocks = (unsigned)((count * 32 + near_threads - 1) / near_threads);
+        for (int a = 0; a < passes; ++a) {
+            PairOut pa = po;
+            if (passes == 2) {
+                pa.s_tl = a;
+                pa.s_tk = 2 + a;
+            }
+            // PEC and equal wavenumbers: the second entry
+            const double ka = passes == 2 ? ap.k[a] : (layout == PAIR_SUM_TK ? ap.k[0] : ap.k[1]);
+            const FarLaunch f{geom, qp, &rw, Q, nf, m0, m1, ka, ap.k[1], ap.threshold, exact, form_a, pa, st};
+            if (rot) SIEB_RETURN_IF((launch_far<1, 1, true>(f, big)));
+            else if (pec) SIEB_RETURN_IF((launch_far<1, 0, false>(f, big)));
+            else if (layout == PAIR_SUM_TK) SIEB_RETURN_IF((launch_far<2, 1, false>(f, big)));
+            else SIEB_RETURN_IF((launch_far<1, 1, false>(f, big)));
+            if (count > 0) {
+                if (rot)
+                    near_regular_kernel<1, 1, true><<<near_blocks, near_threads, 0, st>>>(
+                        geom, qp, rw, Q, nf, m0, m1, list, (int)count, ka, ap.k[1], form_a, pa);
+                else if (pec)
+                    near_regular_kernel<1, 0, false><<<near_blocks, near_threads, 0, st>>>(
+                        geom, qp, rw, Q, nf, m0, m1, list, (int)count, ka, ap.k[1], 0, pa);
+                else if (layout == PAIR_SUM_TK)
+                    near_regular_kernel<2, 1, false><<<near_blocks, near_threads, 0, st>>>(
+                        geom, qp, rw, Q, nf, m0, m1, list, (int)count, ka, ap.k[1], 0, pa);
+                else
+                    near_regular_kernel<1, 1, false><<<near_blocks, near_threads, 0, st>>>(
+                        geom, qp, rw, Q, nf, m0, m1, list, (int)count, ka, ap.k[1], 0, pa);
+                SIEB_NOTE_LAUNCH();
+                SIEB_TRY_CUDA(cudaGetLastError());
+            }
+        }
         if (form_a) {
             if (NK == 1)
                 pair_line_kernel<1><<<rows, kWarps * 32, 0, st>>>(geom, qp, dw, Q, nf, m0, ap.k[1], ap.k[1],
-                                                                  ap.threshold, exact, dgl, dgl + kMaxLine, NG,
-                                                                  NB, pairs);
+                                                                  ap.threshold, exact, dgl, dgl + kMaxLine, NG, po);
             else
                 pair_line_kernel<2><<<rows, kWarps * 32, 0, st>>>(geom, qp, dw, Q, nf, m0, ap.k[0], ap.k[1],
-                                                                  ap.threshold, exact, dgl, dgl + kMaxLine, NG,
-                                                                  NB, pairs);
+                                                                  ap.threshold, exact, dgl, dgl + kMaxLine, NG, po);
             SIEB_NOTE_LAUNCH();
             SIEB_TRY_CUDA(cudaGetLastError());
         }
-
-        // Near-pair list of this slab: count, size, fill.
-        const long long span = (long long)rows * nf;
-        const int nb = (int)((span + 255) / 256);
-        SIEB_TRY_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st));
-        near_pairs_kernel<<<nb, 256, 0, st>>>(geom, nf, ap.threshold, exact, m0, m1, counter, nullptr, 0);
-        SIEB_NOTE_LAUNCH();
-        SIEB_TRY_CUDA(cudaGetLastError());
-        unsigned long long count = 0;
-        SIEB_TRY_CUDA(cudaMemcpyAsync(&count, counter, sizeof(count), cudaMemcpyDeviceToHost, st));
-        SIEB_TRY_CUDA(cudaStreamSynchronize(st));
         if (count > 0) {
-            SIEB_RETURN_IF(ctx->near_list.reserve(sizeof(int2) * count));
-            SIEB_TRY_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st));
-            near_pairs_kernel<<<nb, 256, 0, st>>>(geom, nf, ap.threshold, exact, m0, m1, counter,
-                                                  ctx->near_list.as<int2>(), count);
-            SIEB_NOTE_LAUNCH();
-            SIEB_TRY_CUDA(cudaGetLastError());
-            const int threads = 128;
-            const int blocks = (int)((count * 32 + threads - 1) / threads);
-            if (variant != 0 && opt.formulation == SIEB200_PEC_EFIE && form_a)
-                pair_singular_n_kernel<1, true><<<blocks, threads, 0, st>>>(
-                    geom, qp, dw, Q, nf, m0, ctx->near_list.as<int2>(), (int)count, ap.k[1],
-                    ap.k[1], tk, dgl, dgl + kMaxLine, NG, pairs);
-            else if (variant != 0 && opt.formulation == SIEB200_PEC_EFIE)
-                pair_singular_n_kernel<1, false><<<blocks, threads, 0, st>>>(
-                    geom, qp, dw, Q, nf, m0, ctx->near_list.as<int2>(), (int)count, ap.k[1],
-                    ap.k[1], tk, dgl, dgl + kMaxLine, 0, pairs);
-            else if (variant != 0 && form_a)
-                pair_singular_n_kernel<2, true><<<blocks, threads, 0, st>>>(
-                    geom, qp, dw, Q, nf, m0, ctx->near_list.as<int2>(), (int)count, ap.k[0],
-                    ap.k[1], true, dgl, dgl + kMaxLine, NG, pairs);
-            else if (variant != 0)
-                pair_singular_n_kernel<2, false><<<blocks, threads, 0, st>>>(
-                    geom, qp, dw, Q, nf, m0, ctx->near_list.as<int2>(), (int)count, ap.k[0],
-                    ap.k[1], true, dgl, dgl + kMaxLine, 0, pairs);
-            else if (opt.formulation == SIEB200_PEC_EFIE)
-                pair_singular_kernel<1><<<blocks, threads, 0, st>>>(
-                    geom, qp, dw, Q, nf, m0, ctx->near_list.as<int2>(), (int)count, ap.k[1],
-                    ap.k[1], false, pairs);
+            const double ks = NK == 1 ? ap.k[1] : ap.k[0];
+            if (rot && form_a && NK == 1)
+                pair_singular_n_kernel<1, true><<<near_blocks, near_threads, 0, st>>>(
+                    geom, qp, dw, Q, nf, m0, list, (int)count, ks, ap.k[1], tk, dgl, dgl + kMaxLine, NG, po);
+            else if (rot && form_a)
+                pair_singular_n_kernel<2, true><<<near_blocks, near_threads, 0, st>>>(
+                    geom, qp, dw, Q, nf, m0, list, (int)count, ks, ap.k[1], tk, dgl, dgl + kMaxLine, NG, po);
+            else if (rot && NK == 1)
+                pair_singular_n_kernel<1, false><<<near_blocks, near_threads, 0, st>>>(
+                    geom, qp, dw, Q, nf, m0, list, (int)count, ks, ap.k[1], tk, dgl, dgl + kMaxLine, 0, po);
+            else if (rot)
+                pair_singular_n_kernel<2, false><<<near_blocks, near_threads, 0, st>>>(
+                    geom, qp, dw, Q, nf, m0, list, (int)count, ks, ap.k[1], tk, dgl, dgl + kMaxLine, 0, po);
+            else if (NK == 1)
+                pair_singular_kernel<1><<<near_blocks, near_threads, 0, st>>>(geom, qp, dw, Q, nf, m0, list, (int)count,
+                                                                              ks, ap.k[1], tk, false, po);
             else
-                pair_singular_kernel<2><<<blocks, threads, 0, st>>>(
-                    geom, qp, dw, Q, nf, m0, ctx->near_list.as<int2>(), (int)count, ap.k[0],
-                    ap.k[1], true, pairs);
+                pair_singular_kernel<2><<<near_blocks, near_threads, 0, st>>>(geom, qp, dw, Q, nf, m0, list, (int)count,
+                                                                              ks, ap.k[1], tk, layout == PAIR_SUM_TK,
+                                                                              po);
             SIEB_NOTE_LAUNCH();
             SIEB_TRY_CUDA(cudaGetLastError());
         }
         gp.m0 = m0;
         gp.m1 = m1;
-        if (dx) {
-            gather_matvec_kernel<<<(ne + 7) / 8, 256, 0, st>>>(pairs, dmass, ctx->inc.as<int>(), gp, dx, dy);
-        } else {
-            const dim3 gb(32, 8), gg((ne + 31) / 32, (ne + 7) / 8);
-            gather_kernel<<<gg, gb, 0, st>>>(pairs, dmass, ctx->inc.as<int>(), gp, dZ, ldz);
-        }
+        const dim3 gb(32, 8), gg((ne + 31) / 32, (ne + 7) / 8);
+        if (dx)
+            gather_matvec_kernel<<<(ne + 7) / 8, 256, 0, st>>>(po.pairs, dmass, ctx->inc.as<int>(), gp, dx, dy);
+        else if (one_slab)
+            gather_kernel<false><<<gg, gb, 0, st>>>(po.pairs, dmass, ctx->inc.as<int>(), gp, dZ, ldz);
+        else
+            gather_kernel<true><<<gg, gb, 0, st>>>(po.pairs, dmass, ctx->inc.as<int>(), gp, dZ, ldz);
         SIEB_NOTE_LAUNCH();
         SIEB_TRY_CUDA(cudaGetLastError());
     }
@@ -1815,46 +1775,6 @@ int tensor_gradient_device(sieb200_ctx* ctx, const sieb200_mesh& mesh, const sie
 //   Q_E = j w mu L[J] + K[M],   Q_H = -K[J] + j w eps L[M]
 // (surface_current_fields.hpp:12-44, kernel sie_kernels_utils.cuh:21-140).
 
-// G and grad G of the field evaluation (green_functions_utils.cuh:142-221):
-// standard, or with the static and k^2/2 terms extracted.
-__device__ __forceinline__ void field_green(d3 r1, d3 r2, double k, bool regular, cplx& G, cplx g[3]) {
-    const d3 Rv = r1 - r2;
-    const double R = sqrt(Rv.x * Rv.x + Rv.y * Rv.y + Rv.z * Rv.z);
-    if (!regular) {
-        if (R < 1e-12) {
-            G = cx(0.0, 0.0);
-            g[0] = g[1] = g[2] = cx(0.0, 0.0);
-            return;
-        }
-        const double inv_R = 1.0 / R;
-        const double i4pR = 1.0 / (4.0 * kPi * R);
-        double s, c;
-        sincos(k * R, &s, &c);
-        G = cx(c * i4pR, -s * i4pR);
-        const cplx wg = cx(inv_R, k) * G;
-        g[0] = wg * (Rv.x * inv_R);
-        g[1] = wg * (Rv.y * inv_R);
-        g[2] = wg * (Rv.z * inv_R);
-    } else {
-        if (R < 1e-6) {
-            G = cx(0.0, -k / (4.0 * kPi));
-            g[0] = g[1] = g[2] = cx(0.0, 0.0);
-            return;
-        }
-        const double i4p = 1.0 / (4.0 * kPi);
-        const double inv_R = 1.0 / R, inv_R2 = inv_R * inv_R, inv_R3 = inv_R2 * inv_R;
-        double s, c;
-        sincos(k * R, &s, &c);
-        G = cx((c - 1.0) * (i4p * inv_R), -s * (i4p * inv_R));
-        cplx Kr = cx(inv_R3, k * inv_R2) * cx(c, -s);
-        Kr.re += -(inv_R3 + k * k * 0.5 * inv_R);
-        const cplx sc = Kr * i4p;
-        g[0] = sc * Rv.x;
-        g[1] = sc * Rv.y;
-        g[2] = sc * Rv.z;
-    }
-}
-
 struct FieldConsts {
     cplx cJ, cM, cJh, cMh;   // j w mu, 1, -1, j w eps
     float k;                 // the wavenumber as the quadrature helpers receive it
@@ -1862,104 +1782,229 @@ struct FieldConsts {
     float threshold;         // 0.1 lambda in float
 };
 
-// One CTA of 256 threads per observation point; threads take faces
-// f = t, t + 256, ...; per face the three half-RWG integrals
-// (dunavant_quadrature.cuh:1634-1705, plus the Wilton part of :1719-1770
-// when the face centroid is within 0.1 lambda), folded into E and H; a warp
-// butterfly and one pass over the warps in a fixed order sum them.
-__global__ void __launch_bounds__(256) surface_fields_kernel(const FaceGeom* __restrict__ geom,
-                                                            const d3* __restrict__ qp,
-                                                            const float* __restrict__ qw, int Q, int nf,
-                                                            const d3* __restrict__ obs,
-                                                            const cplx* __restrict__ J,
-                                                            const cplx* __restrict__ M, FieldConsts fc,
-                                                            cplx* __restrict__ E, cplx* __restrict__ H) {
-    const d3 r = obs[blockIdx.x];
-    const double kd = (double)fc.k;
-    cplx e[3] = {cx(0, 0), cx(0, 0), cx(0, 0)}, h[3] = {cx(0, 0), cx(0, 0), cx(0, 0)};
-    for (int f = threadIdx.x; f < nf; f += blockDim.x) {
-        const FaceGeom g = geom[f];
-        // float distance from the centroid, formed without contraction
-        const double dx = __dsub_rn(r.x, g.c.x), dy = __dsub_rn(r.y, g.c.y), dz = __dsub_rn(r.z, g.c.z);
-        const float dist = (float)__dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)),
-                                                       __dmul_rn(dz, dz)));
-        const bool near = dist < fc.threshold;
-        cplx L[3][3], K[3][3];
+// Per face, for the field sums: the currents' coefficients a = sum_i l_i c_i
+// and aA = sum_i l_i c_i A_i (A_i = v_i - centroid, l_i the float edge length)
+// for J and M, and the quadrature points about the centroid. Structure of
+// arrays over `ld` >= nf faces, so that one thread per face reads coalesced:
+// rows 0-2 centroid, 3-4 a_J, 5-10 aA_J, 11-12 a_M, 13-18 aA_M, then q x 3.
+constexpr int kFieldRows = 19;
+__global__ void field_faces_kernel(const FaceGeom* __restrict__ geom, const d3* __restrict__ qp, int Q, int nf,
+                                   const cplx* __restrict__ J, const cplx* __restrict__ M, int ld,
+                                   double* __restrict__ fs) {
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= nf) return;
+    const d3 c = geom[f].c;
+    const int q = blockIdx.y;
+    if (q < Q) {
+        const d3 r = qp[(size_t)f * Q + q] - c;
+        double* o = fs + (size_t)(kFieldRows + 3 * q) * ld + f;
+        o[0] = r.x; o[ld] = r.y; o[2 * (size_t)ld] = r.z;
+        return;
+    }
+    double v[kFieldRows];
+    v[0] = c.x; v[1] = c.y; v[2] = c.z;
 #pragma unroll
-        for (int i = 0; i < 3; ++i)
+    for (int e = 3; e < kFieldRows; ++e) v[e] = 0.0;
 #pragma unroll
-            for (int c = 0; c < 3; ++c) { L[i][c] = cx(0, 0); K[i][c] = cx(0, 0); }
-        for (int q = 0; q < Q; ++q) {
-            const d3 rq = qp[(size_t)f * Q + q];
-            const double w = (double)qw[q];
-            cplx G, gg[3];
-            field_green(r, rq, kd, near, G, gg);
+    for (int i = 0; i < 3; ++i) {
+        const double el = (double)(float)geom[f].len[i];
+        const d3 A = geom[f].A[i];
+        const int ed = geom[f].edge[i];
+        const cplx a[2] = {J[ed] * el, M ? M[ed] * el : cx(0, 0)};
 #pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                const d3 rho = rq - g.fv[i];
-                const double rc[3] = {rho.x, rho.y, rho.z};
-#pragma unroll
-                for (int c = 0; c < 3; ++c)
-                    L[i][c] += ((G * rc[c]) * 0.5 + gg[c] * (double)(-fc.k_sq_inv)) * w;
-                const cplx cr[3] = {gg[2] * rho.y - gg[1] * rho.z, gg[0] * rho.z - gg[2] * rho.x,
-                                    gg[1] * rho.x - gg[0] * rho.y};
-#pragma unroll
-                for (int c = 0; c < 3; ++c) K[i][c] += (cr[c] * 0.5) * w;
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const double el = (double)(float)g.len[i];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) { L[i][c] = L[i][c] * el; K[i][c] = K[i][c] * el; }
-        }
-        if (near) {
-            const float A = (float)g.area;
-            const float base = __fdiv_rn(1.0f, __fmul_rn(__fmul_rn(8.0f, (float)kPi), A));
-            const Pots P = wilton(r, g.v);
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                const d3 fv = g.fv[i];
-                const d3 Rf = r - fv;
-                const d3 phi3 = P.phi3b + (P.r_pi - fv) * P.phi2;
-                const d3 Lin = (psi1(P, fv) - (Rf * 0.5) * P.phi0) + (phi3 - Rf * P.phi2) * (double)fc.k_sq_inv;
-                const d3 Kv = upsilon(P, fv, r, fc.k);
-                const double ls = (double)__fmul_rn((float)g.len[i], base);
-                const d3 Lv = Lin * 2.0;
-                L[i][0] += cx(Lv.x * ls, 0.0); L[i][1] += cx(Lv.y * ls, 0.0); L[i][2] += cx(Lv.z * ls, 0.0);
-                K[i][0] += cx(Kv.x * ls, 0.0); K[i][1] += cx(Kv.y * ls, 0.0); K[i][2] += cx(Kv.z * ls, 0.0);
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const int ed = g.edge[i];
-            const cplx je = J[ed], me = M ? M[ed] : cx(0, 0);
-            const cplx wEJ = fc.cJ * je, wEM = fc.cM * me, wHJ = fc.cJh * je, wHM = fc.cMh * me;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                e[c] += wEJ * L[i][c];
-                e[c] += wEM * K[i][c];
-                h[c] += wHJ * K[i][c];
-                h[c] += wHM * L[i][c];
-            }
+        for (int t = 0; t < 2; ++t) {
+            double* o = v + 3 + 8 * t;
+            o[0] += a[t].re; o[1] += a[t].im;
+            o[2] += a[t].re * A.x; o[3] += a[t].im * A.x;
+            o[4] += a[t].re * A.y; o[5] += a[t].im * A.y;
+            o[6] += a[t].re * A.z; o[7] += a[t].im * A.z;
         }
     }
-    __shared__ double part[8][12];
+#pragma unroll
+    for (int e = 0; e < kFieldRows; ++e) fs[(size_t)e * ld + f] = v[e];
+}
+
+// E and H of one face's quadrature sums S0 = sum w G, Sq = sum w G q,
+// T0 = sum w g, Tq = sum w g q (grad G = g R, R = r - r_q, P = r - centroid).
+// With TR = T0 P - Tq and KP = Tq x P, both linear in the edge currents:
+//   L = 1/2 (a Sq - S0 aA) - a TR / k^2,  K = 1/2 (a KP - aA x TR).
+__device__ __forceinline__ void add_face_fields(const PointSums<1, 1>& I, d3 P, const double (&v)[kFieldRows],
+                                                const FieldConsts& fc, cplx (&e)[3], cplx (&h)[3]) {
+    const cplx TR[3] = {I.T0[0] * P.x - I.Tq[0][0], I.T0[0] * P.y - I.Tq[0][1], I.T0[0] * P.z - I.Tq[0][2]};
+    const cplx KP[3] = {I.Tq[0][1] * P.z - I.Tq[0][2] * P.y, I.Tq[0][2] * P.x - I.Tq[0][0] * P.z,
+                        I.Tq[0][0] * P.y - I.Tq[0][1] * P.x};
+    const double ik2 = (double)fc.k_sq_inv;
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        const double* u = v + 3 + 8 * t;
+        const cplx a = cx(u[0], u[1]);
+        const cplx aA[3] = {cx(u[2], u[3]), cx(u[4], u[5]), cx(u[6], u[7])};
+        cplx L[3], K[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            L[c] = a * (I.Sq[0][c] * 0.5 - TR[c] * ik2) - (I.S0[0] * aA[c]) * 0.5;
+            const int c1 = c == 2 ? 0 : c + 1, c2 = c == 0 ? 2 : c - 1;
+            K[c] = (a * KP[c] - (aA[c1] * TR[c2] - aA[c2] * TR[c1])) * 0.5;
+        }
+        const cplx cE_L = fc.cJ, cH_K = fc.cJh, cE_K = fc.cM, cH_L = fc.cMh;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            e[c] += t == 0 ? cE_L * L[c] : cE_K * K[c];
+            h[c] += t == 0 ? cH_K * K[c] : cH_L * L[c];
+        }
+    }
+}
+
+// Analytic (Wilton) part of a near face (dunavant_quadrature.cuh:1719-1770).
+__device__ void add_near_fields(const FaceGeom& g, d3 r, const cplx* __restrict__ J, const cplx* __restrict__ M,
+                                const FieldConsts& fc, cplx (&e)[3], cplx (&h)[3]) {
+    const float A = (float)g.area;
+    const float base = __fdiv_rn(1.0f, __fmul_rn(__fmul_rn(8.0f, (float)kPi), A));
+    const Pots P = wilton(r, g.v);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const d3 fv = g.fv[i];
+        const d3 Rf = r - fv;
+        const d3 phi3 = P.phi3b + (P.r_pi - fv) * P.phi2;
+        const d3 Lin = (psi1(P, fv) - (Rf * 0.5) * P.phi0) + (phi3 - Rf * P.phi2) * (double)fc.k_sq_inv;
+        const d3 Kv = upsilon(P, fv, r, fc.k);
+        const double ls = (double)__fmul_rn((float)g.len[i], base);
+        const d3 Lv = Lin * (2.0 * ls), Kl = Kv * ls;
+        const double lc[3] = {Lv.x, Lv.y, Lv.z}, kc[3] = {Kl.x, Kl.y, Kl.z};
+        const int ed = g.edge[i];
+        const cplx je = J[ed], me = M ? M[ed] : cx(0, 0);
+        const cplx wEJ = fc.cJ * je, wEM = fc.cM * me, wHJ = fc.cJh * je, wHM = fc.cMh * me;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            e[c] += wEJ * lc[c] + wEM * kc[c];
+            h[c] += wHJ * kc[c] + wHM * lc[c];
+        }
+    }
+}
+
+// One CTA per observation point and face chunk (blockIdx.y), one thread per
+// face; the chunk's E and H go to part[point][chunk][12]. Bound: the FP64
+// pipe, 52 instructions per kernel value (the sums are those of the assembly,
+// so the three half-RWG integrals cost nothing per value). A face whose
+// centroid is within 0.1 lambda of the point takes the extracted kernel
+// (green_functions_utils.cuh:142-221) and the analytic part instead.
+constexpr int kFieldThreads = 128;
+template <bool BIG>
+__global__ void __launch_bounds__(kFieldThreads, 4)
+surface_fields_kernel(const FaceGeom* __restrict__ geom, const d3* __restrict__ qp, const RuleWeights rw, int Q, int nf,
+                      const double* __restrict__ fs, int ld, int faces_per_chunk, const d3* __restrict__ obs,
+                      const cplx* __restrict__ J, const cplx* __restrict__ M, const FieldConsts fc, const Wave wave,
+                      double* __restrict__ part) {
+    __shared__ __align__(16) double2 tab[kTurn * kTurnCopies];
+    __shared__ double red[kFieldThreads / 32][12];
+    fill_turn_table(tab);
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const double2* my_tab = tab + (lane & (kTurnCopies - 1));
+    const d3 r = obs[blockIdx.x];
+    cplx e[3] = {cx(0, 0), cx(0, 0), cx(0, 0)}, h[3] = {cx(0, 0), cx(0, 0), cx(0, 0)};
+    const int f0 = blockIdx.y * faces_per_chunk, f1 = min(nf, f0 + faces_per_chunk);
+    for (int fb = f0 + 32 * warp; fb < f1; fb += kFieldThreads) {  // warp-uniform
+        const int f = fb + lane;
+        const bool have = f < f1;
+        const double* col = fs + (have ? f : f1 - 1);
+        const d3 c = mk3(col[0], col[ld], col[2 * (size_t)ld]);
+        // float distance from the centroid, formed without contraction
+        const double dx = __dsub_rn(r.x, c.x), dy = __dsub_rn(r.y, c.y), dz = __dsub_rn(r.z, c.z);
+        const float dist = (float)__dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)),
+                                                       __dmul_rn(dz, dz)));
+        const bool near = have && dist < fc.threshold;
+        const d3 P = mk3(dx, dy, dz);
+        PointSums<1, 1> in;
+        in.clear();
+        if (have && !near) {
+            const double* qc = col + (size_t)kFieldRows * ld;
+#pragma unroll 2
+            for (int q = 0; q < Q; ++q, qc += 3 * (size_t)ld) {
+                const double qx = qc[0], qy = qc[ld], qz = qc[2 * (size_t)ld];
+                const double ax = P.x - qx, ay = P.y - qy, az = P.z - qz;
+                const double R2 = fma(az, az, fma(ay, ay, ax * ax));
+                double inv = rsqrt_refined(R2);
+                if (tiny_square(R2)) inv = 0.0;  // R < 1e-12: no contribution
+                const double R = R2 * inv;
+                const double W = inv * rw.w4[q], v = wave.k * inv, i2 = inv * inv;
+                double cs, sn;
+                if (BIG) sincos(wave.k * R, &sn, &cs);
+                else phase_cs(my_tab, wave, R, cs, sn);
+                const cplx G[1] = {cx(cs * W, -sn * W)};
+                const cplx g[1] = {cx(fma(i2, G[0].re, -(v * G[0].im)), fma(i2, G[0].im, v * G[0].re))};
+                in.add(G, g, qx, qy, qz);
+            }
+        }
+        // Near faces: few against the rule's points, the warp takes them one after
+        // the other, lanes over the points; many, every lane its own.
+        unsigned todo = __ballot_sync(0xffffffffu, near);
+        auto near_point = [&](int fn, int q, PointSums<1, 1>& s) {
+            const double* qc = fs + fn + (size_t)(kFieldRows + 3 * q) * ld;
+            const d3 Rv = r - qp[(size_t)fn * Q + q];
+            const double R = sqrt(Rv.x * Rv.x + Rv.y * Rv.y + Rv.z * Rv.z);
+            cplx G[1], g[1];
+            if (R < 1e-6) {
+                G[0] = cx(0.0, -wave.k / (4.0 * kPi));
+                g[0] = cx(0.0, 0.0);
+            } else {
+                green_reg(R, wave.k, G[0], g[0]);
+            }
+            G[0] = G[0] * rw.w[q];
+            g[0] = g[0] * rw.w[q];
+            s.add(G, g, qc[0], qc[ld], qc[2 * (size_t)ld]);
+        };
+        if (__popc(todo) * ((Q + 31) / 32) >= Q) {
+            todo = 0;
+            if (near)
+#pragma unroll 1
+                for (int q = 0; q < Q; ++q) near_point(f, q, in);
+        }
+        while (todo) {
+            const int b = __ffs(todo) - 1;
+            todo &= todo - 1;
+            PointSums<1, 1> s;
+            s.clear();
+#pragma unroll 1
+            for (int q = lane; q < Q; q += 32) near_point(fb + b, q, s);
+            warp_sum(s.S0[0]); warp_sum(s.T0[0]);
+#pragma unroll
+            for (int t = 0; t < 3; ++t) { warp_sum(s.Sq[0][t]); warp_sum(s.Tq[0][t]); }
+            if (lane == b) in = s;
+        }
+        if (have) {
+            double v[kFieldRows];
+#pragma unroll
+            for (int t = 3; t < kFieldRows; ++t) v[t] = col[(size_t)t * ld];
+            add_face_fields(in, P, v, fc, e, h);
+        }
+        if (near) add_near_fields(geom[f], r, J, M, fc, e, h);
+    }
     double v[12] = {e[0].re, e[0].im, e[1].re, e[1].im, e[2].re, e[2].im,
                     h[0].re, h[0].im, h[1].re, h[1].im, h[2].re, h[2].im};
 #pragma unroll
     for (int j = 0; j < 12; ++j) warp_sum(v[j]);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (lane == 0)
 #pragma unroll
-        for (int j = 0; j < 12; ++j) part[warp][j] = v[j];
+        for (int j = 0; j < 12; ++j) red[warp][j] = v[j];
     __syncthreads();
     if (threadIdx.x < 12) {
         double t = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += part[w][threadIdx.x];
-        double* out = reinterpret_cast<double*>(threadIdx.x < 6 ? E : H) + 6 * (size_t)blockIdx.x;
-        out[threadIdx.x % 6] = t;
+        for (int w = 0; w < kFieldThreads / 32; ++w) t += red[w][threadIdx.x];
+        part[((size_t)blockIdx.x * gridDim.y + blockIdx.y) * 12 + threadIdx.x] = t;
     }
+}
+
+// Sums the chunks of each point in order: E (6 values), then H.
+__global__ void surface_fields_finish_kernel(const double* __restrict__ part, int64_t nobs, int chunks,
+                                             cplx* __restrict__ E, cplx* __restrict__ H) {
+    const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (id >= nobs * 12) return;
+    const int64_t p = id / 12;
+    const int j = (int)(id - 12 * p);
+    double t = 0.0;
+    for (int c = 0; c < chunks; ++c) t += part[(p * chunks + c) * 12 + j];
+    reinterpret_cast<double*>(j < 6 ? E : H)[6 * p + j % 6] = t;
 }
 
 int surface_fields_device(sieb200_ctx* ctx, const sieb200_mesh& mesh, const double* j_cur, const double* m_cur,
@@ -2007,20 +2052,45 @@ int surface_fields_device(sieb200_ctx* ctx, const sieb200_mesh& mesh, const doub
     volatile float lambda = (float)((double)(2.0f * (float)M_PI) / k);
     fc.threshold = 0.1f * lambda;
 
+    // Chunks of faces per point: some 16 CTAs per SM in all, so that few
+    // points still fill the GPU and the last wave is short; at least one face
+    // per thread.
+    const int most = (nf + kFieldThreads - 1) / kFieldThreads;
+    const int64_t want = ((int64_t)ctx->sm_count * 16 + nobs - 1) / nobs;
+    const int per_chunk = kFieldThreads * (int)((most + std::min<int64_t>(most, want) - 1) / std::min<int64_t>(most, want));
+    const int chunks = (nf + per_chunk - 1) / per_chunk;
+    const int ld = ((nf + 31) / 32) * 32;
     DeviceBuffer buf;
     const size_t b_obs = sizeof(d3) * (size_t)nobs, b_cur = sizeof(cplx) * (size_t)ne;
     const size_t b_out = sizeof(cplx) * 3 * (size_t)nobs;
-    SIEB_RETURN_IF(buf.reserve(b_obs + 2 * b_cur + 2 * b_out));
+    const size_t b_fs = sizeof(double) * (size_t)(kFieldRows + 3 * Q) * ld;
+    const size_t b_part = sizeof(double) * 12 * (size_t)nobs * chunks;
+    SIEB_RETURN_IF(buf.reserve(2 * b_cur + 2 * b_out + b_fs + b_part + b_obs));
     char* b = buf.as<char>();
-    d3* dobs = reinterpret_cast<d3*>(b);
-    cplx* dJ = reinterpret_cast<cplx*>(b + b_obs);
+    cplx* dJ = reinterpret_cast<cplx*>(b);
     cplx* dM = m_cur ? dJ + ne : nullptr;
-    cplx* dE = reinterpret_cast<cplx*>(b + b_obs + 2 * b_cur);
+    cplx* dE = reinterpret_cast<cplx*>(b + 2 * b_cur);
     cplx* dH = dE + 3 * (size_t)nobs;
+    double* fs = reinterpret_cast<double*>(b + 2 * b_cur + 2 * b_out);
+    double* part = reinterpret_cast<double*>(b + 2 * b_cur + 2 * b_out + b_fs);
+    d3* dobs = reinterpret_cast<d3*>(b + 2 * b_cur + 2 * b_out + b_fs + b_part);
     SIEB_TRY_CUDA(cudaMemcpyAsync(dobs, points, b_obs, cudaMemcpyHostToDevice, st));
     SIEB_TRY_CUDA(cudaMemcpyAsync(dJ, j_cur, b_cur, cudaMemcpyHostToDevice, st));
     if (m_cur) SIEB_TRY_CUDA(cudaMemcpyAsync(dM, m_cur, b_cur, cudaMemcpyHostToDevice, st));
-    surface_fields_kernel<<<(unsigned)nobs, 256, 0, st>>>(geom, qp, dw, Q, nf, dobs, dJ, dM, fc, dE, dH);
+    field_faces_kernel<<<dim3((unsigned)most, (unsigned)(Q + 1)), kFieldThreads, 0, st>>>(geom, qp, Q, nf, dJ, dM, ld,
+                                                                                         fs);
+    SIEB_NOTE_LAUNCH();
+    SIEB_TRY_CUDA(cudaGetLastError());
+    double far = 0.0;  // no farther than this from any point to any face
+    for (int64_t i = 0; i < 3 * nobs; ++i) far = std::max(far, std::fabs(points[i]));
+    for (int64_t i = 0; i < 3 * mesh.num_vertices; ++i) far = std::max(far, std::fabs(mesh.vertices[i]));
+    const bool big = !((double)fc.k * 4.0 * far < kPhaseMax);
+    auto* kernel = big ? surface_fields_kernel<true> : surface_fields_kernel<false>;
+    kernel<<<dim3((unsigned)nobs, (unsigned)chunks), kFieldThreads, 0, st>>>(
+        geom, qp, make_rule_weights(wts, Q), Q, nf, fs, ld, per_chunk, dobs, dJ, dM, fc, make_wave((double)fc.k), part);
+    SIEB_NOTE_LAUNCH();
+    SIEB_TRY_CUDA(cudaGetLastError());
+    surface_fields_finish_kernel<<<(unsigned)((nobs * 12 + 255) / 256), 256, 0, st>>>(part, nobs, chunks, dE, dH);
     SIEB_NOTE_LAUNCH();
     SIEB_TRY_CUDA(cudaGetLastError());
     SIEB_TRY_CUDA(cudaMemcpyAsync(E_out, dE, b_out, cudaMemcpyDeviceToHost, st));

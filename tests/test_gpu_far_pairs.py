@@ -1,0 +1,130 @@
+"""The regular quadrature pass: lane splits, pair layouts, slabs and phases at
+the edges of its dispatch, and the far-field and surface-field sums that share
+its phase factors, against the oracle."""
+
+import math
+
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+C0 = 299792458.0
+
+
+def _mesh(name):
+    import sieb200
+    return {"ico20": lambda: sieb200.icosphere(0.5, 0), "geo180": lambda: sieb200.geodesic_sphere(0.5, 3),
+            "spindle90": lambda: sieb200.revolved_spindle(0.6, 60.0, n_axial=6, n_azimuth=9)}[name]()
+
+
+def _options(form, rule, freq, eps_in, eps_out=1.0):
+    import sieb200
+    medium = sieb200.IsotropicMedium
+    if form == "pec":
+        return sieb200.PecOptions(frequency_hz=freq, quadrature_rule=rule), 0, 0
+    if form == "gstc":
+        return sieb200.GstcSieOptions(frequency_hz=freq, quadrature_rule=rule, interior=medium(eps_in, 1.0),
+                                      exterior=medium(eps_out, 1.0)), 2, 0
+    name, variant = {"pmchwt": ("T_PMCHWT", 0), "n_pmchwt": ("N_PMCHWT", 1), "muller": ("N_Muller", 2)}[form]
+    return sieb200.DielectricOptions(frequency_hz=freq, quadrature_rule=rule, formulation=name,
+                                     interior=medium(eps_in, 1.0), exterior=medium(eps_out, 1.0)), 1, variant
+
+
+def _oracle(mesh, kind, variant, rule, opts, eps_in, eps_out=1.0, tensors=None):
+    eps = (eps_in, eps_out) if kind else (1.0, 1.0)
+    s = O.kernel_scalars(kind, opts.frequency_hz, eps_r=eps)
+    return O.assemble(O.oracle(), kind, mesh, rule, s, tensors=tensors, variant=variant)
+
+
+def _tensors(nf):
+    rng = np.random.default_rng(nf)
+    t = rng.standard_normal((nf, 32)) + 1j * rng.standard_normal((nf, 32))
+    return np.ascontiguousarray(t)
+
+
+@pytest.mark.parametrize("form", ["pec", "pmchwt", "gstc", "n_pmchwt", "muller"])
+@pytest.mark.parametrize("rule", [1, 2, 5, 8, 20])
+@pytest.mark.parametrize("name", ["ico20", "geo180", "spindle90"])
+@pytest.mark.parametrize("same", [False, True])
+def test_assembly_layouts(form, rule, name, same, gpu_ctx):
+    """Every pair layout (one wavenumber, two, two equal, TK summed) with 1 to
+    79 rule points, and so with 1 to 32 lanes per pair."""
+    import sieb200
+    mesh = _mesh(name)
+    eps_in = 1.0 if same else 2.56
+    opts, kind, variant = _options(form, rule, 0.6 * C0, eps_in)
+    t = _tensors(mesh.num_faces) if kind == 2 else None
+    Z = sieb200.assemble_matrix(mesh, opts, tensors=t, ctx=gpu_ctx)
+    Zo = _oracle(mesh, kind, variant, rule, opts, eps_in, tensors=t)
+    assert np.abs(Z - Zo).max() <= 1e-12 * np.abs(Zo).max()
+
+
+@pytest.mark.parametrize("k_extent", [9.0e6, 4.0e7])
+def test_assembly_large_phase(k_extent, gpu_ctx):
+    """Phases up to the step number's limit, and past it (sincos). The bound
+    is the rounding of k R itself, 1e7 x 1e-16 and some."""
+    import sieb200
+    mesh = _mesh("ico20")
+    v = np.asarray(mesh.vertices)
+    freq = k_extent / (v.max(0) - v.min(0)).sum() * C0 / (2 * math.pi)
+    opts, kind, variant = _options("pec", 5, freq, 1.0)
+    Z = sieb200.assemble_matrix(mesh, opts, ctx=gpu_ctx)
+    Zo = _oracle(mesh, kind, variant, 5, opts, 1.0)
+    assert np.abs(Z - Zo).max() <= 1e-6 * np.abs(Zo).max()
+
+
+def test_assembly_two_slabs(gpu_ctx):
+    """4500 faces in two slabs of test faces (pairs inside a slab are evaluated
+    once and mirrored, pairs across slabs twice): rows of faces around the
+    slab boundary and elsewhere."""
+    import torch
+    import sieb200
+    mesh = sieb200.geodesic_sphere(1.0, 15)
+    opts, kind, variant = _options("pmchwt", 1, 1.5 * C0, 4.0)
+    n = 2 * mesh.num_edges
+    Z = torch.empty((n, n), dtype=torch.complex128, device="cuda")  # Z[c] is column c
+    torch.cuda.synchronize()
+    sieb200.assemble_matrix_device(mesh, opts, Z.data_ptr(), ctx=gpu_ctx)
+    edge = np.unique(mesh.faces_edges[[0, 2000, 4410, 4418, 4419, 4430, 4499]])
+    rows = np.concatenate([edge, edge + mesh.num_edges])
+    s = O.kernel_scalars(kind, opts.frequency_hz, eps_r=(4.0, 1.0))
+    Zo = O.assemble_rows(O.oracle(), kind, mesh, 1, s, rows)
+    Zg = Z[:, torch.from_numpy(rows).cuda()].cpu().numpy().T
+    assert np.abs(Zg - Zo).max() <= 1e-12 * np.abs(Zo).max()
+
+
+@pytest.mark.parametrize("rule", [1, 5, 17])
+@pytest.mark.parametrize("name", ["ico20", "geo180"])
+@pytest.mark.parametrize("points", [1, 130])
+def test_surface_fields_near_and_far(rule, name, points, gpu_ctx):
+    """Few and many near faces per warp, with and without magnetic currents."""
+    import sieb200
+    mesh = _mesh(name)
+    rng = np.random.default_rng(rule)
+    p = rng.standard_normal((points, 3))
+    p *= (np.where(np.arange(points) % 3, 0.52, 1.7) / np.linalg.norm(p, axis=1))[:, None]
+    j, m = (rng.standard_normal(mesh.num_edges) + 1j * rng.standard_normal(mesh.num_edges) for _ in range(2))
+    for mc in (m, None):
+        E, H = sieb200.evaluate_surface_integral_fields(mesh, j, mc, p, 0.4 * C0, quadrature_rule=rule, ctx=gpu_ctx)
+        Eo, Ho = O.surface_fields(O.oracle(), mesh, j, mc, p, 0.4 * C0, rule=rule)
+        assert np.abs(E - Eo).max() <= 1e-12 * np.abs(Eo).max()
+        assert np.abs(H - Ho).max() <= 1e-12 * np.abs(Ho).max()
+
+
+@pytest.mark.parametrize("name", ["ico20", "geo180", "spindle90"])
+@pytest.mark.parametrize("ndir", [1, 127, 129, 1000])
+@pytest.mark.parametrize("k0", [3.0, 4.0e7])
+def test_far_field_chunks(name, ndir, k0, gpu_ctx):
+    import sieb200
+    mesh = _mesh(name)
+    rng = np.random.default_rng(ndir)
+    j, m = (rng.standard_normal(mesh.num_edges) + 1j * rng.standard_normal(mesh.num_edges) for _ in range(2))
+    frames = sieb200.spherical_frames(np.arccos(rng.uniform(-1, 1, ndir)), rng.uniform(0, 2 * math.pi, ndir))
+    got = sieb200.far_field(mesh, j, m, k0, 376.73, *frames, ctx=gpu_ctx)
+    want = O.far_field(O.oracle(), mesh, j, m, k0, 376.73, *frames)
+    bound = 1e-12 if k0 < 10 else 1e-6  # the rounding of k0 r.r' at phases of 2e7
+    for a, b in zip(got, want):
+        assert np.abs(a - b).max() <= bound * np.abs(b).max()
