@@ -14,15 +14,17 @@
 // them, so every column is produced without atomics.
 //
 // Far field: applications/anisotropic_gstc_sphere/plot_far_field.py:88-220.
-// One CTA per direction reduces exp(+j k0 r_hat . r_q) c(q) over the F*7
-// weighted basis samples.
+// One thread per direction sums exp(+j k0 r_hat . r_q) over the faces of a
+// chunk into per-face moments, which the face's currents turn into N and L.
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
 #include "common.cuh"
+#include "phase.cuh"
 
 namespace sieb200 {
 
@@ -186,56 +188,66 @@ __global__ void rhs_gather_kernel(const cplx* __restrict__ face_vals, const int*
 }
 
 // ------------------------------------------------------------ far field --
-__global__ void ff_samples_kernel(const double* __restrict__ V, const int* __restrict__ F,
-                                  const int* __restrict__ FE, int nf, const cplx* __restrict__ jc,
-                                  const cplx* __restrict__ mc, d3* __restrict__ rq,
-                                  cplx* __restrict__ cj, cplx* __restrict__ cm) {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= nf) return;
-    // plot_far_field.py:88-115 rule (double): centroid, then two 3-orbits.
-    const double s15 = sqrt(15.0);
+// The 7-point rule of plot_far_field.py:88-115 (double): centroid, then two
+// 3-orbits.
+struct FarRule {
+    double xi[7], eta[7], w[7];
+};
+FarRule far_rule() {
+    const double s15 = std::sqrt(15.0);
     const double a1 = (6.0 - s15) / 21.0, w1 = (155.0 - s15) / 1200.0;
     const double a2 = (6.0 + s15) / 21.0, w2 = (155.0 + s15) / 1200.0;
-    const double nodes[7][2] = {{1.0 / 3.0, 1.0 / 3.0}, {a1, a1}, {1.0 - 2.0 * a1, a1},
-                                {a1, 1.0 - 2.0 * a1}, {a2, a2}, {1.0 - 2.0 * a2, a2},
-                                {a2, 1.0 - 2.0 * a2}};
-    const double wq[7] = {0.225, w1, w1, w1, w2, w2, w2};
+    return FarRule{{1.0 / 3.0, a1, 1.0 - 2.0 * a1, a1, a2, 1.0 - 2.0 * a2, a2},
+                   {1.0 / 3.0, a1, a1, 1.0 - 2.0 * a1, a2, a2, 1.0 - 2.0 * a2},
+                   {0.225, w1, w1, w1, w2, w2, w2}};
+}
+
+// Face record of the far-field sums (kFarRow doubles): centroid c; for J and
+// for M a = 1/2 sum_i l_i c_i and aA = 1/2 sum_i l_i c_i A_i (A_i = v_i - c);
+// the 7 points about c. With S0 = sum w e and Sq = sum w e q over the points
+// (e = exp(j k0 r_hat . r_q)) the face adds a Sq - aA S0 to N (J) and L (M).
+constexpr int kFarRow = 40;
+__global__ void ff_faces_kernel(const double* __restrict__ V, const int* __restrict__ F, const int* __restrict__ FE,
+                                int nf, const FarRule rule, const cplx* __restrict__ jc, const cplx* __restrict__ mc,
+                                double* __restrict__ rec) {
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= nf) return;
     int idx[3];
     d3 v[3];
     for (int a = 0; a < 3; ++a) {
         idx[a] = F[3 * f + a];
         v[a] = mk3(V[3 * idx[a]], V[3 * idx[a] + 1], V[3 * idx[a] + 2]);
     }
-    d3 r[7];
-    for (int q = 0; q < 7; ++q) {
-        const double xi = nodes[q][0], eta = nodes[q][1], zeta = 1.0 - xi - eta;
-        r[q] = v[0] * zeta + v[1] * xi + v[2] * eta;
-        rq[f * 7 + q] = r[q];
-    }
+    const d3 c = (v[0] + v[1] + v[2]) * (1.0 / 3.0);
+    double* o = rec + (size_t)f * kFarRow;
+    o[0] = c.x; o[1] = c.y; o[2] = c.z;
     const int EA[3] = {0, 1, 2}, EB[3] = {1, 2, 0}, EF[3] = {2, 0, 1};
-    cplx accj[7][3], accm[7][3];
-    for (int q = 0; q < 7; ++q)
-        for (int c = 0; c < 3; ++c) { accj[q][c] = cx(0, 0); accm[q][c] = cx(0, 0); }
+    cplx a[2] = {cx(0, 0), cx(0, 0)}, aA[2][3];
+    for (int t = 0; t < 2; ++t)
+        for (int k = 0; k < 3; ++k) aA[t][k] = cx(0, 0);
     for (int le = 0; le < 3; ++le) {
         const d3 ev = v[EB[le]] - v[EA[le]];
         const double len = (idx[EA[le]] > idx[EB[le]] ? 1.0 : -1.0) * sqrt(dot3(ev, ev));
         const int e = FE[3 * f + le];
-        const cplx coj = jc[e] * (0.5 * len);
-        const cplx com = mc ? mc[e] * (0.5 * len) : cx(0, 0);
-        for (int q = 0; q < 7; ++q) {
-            const d3 rho = r[q] - v[EF[le]];
-            const double rr[3] = {rho.x, rho.y, rho.z};
-            for (int c = 0; c < 3; ++c) {
-                accj[q][c] += coj * (wq[q] * rr[c]);
-                accm[q][c] += com * (wq[q] * rr[c]);
-            }
+        const d3 A = v[EF[le]] - c;
+        const cplx co[2] = {jc[e] * (0.5 * len), mc ? mc[e] * (0.5 * len) : cx(0, 0)};
+        for (int t = 0; t < 2; ++t) {
+            a[t] += co[t];
+            aA[t][0] += co[t] * A.x;
+            aA[t][1] += co[t] * A.y;
+            aA[t][2] += co[t] * A.z;
         }
     }
-    for (int q = 0; q < 7; ++q)
-        for (int c = 0; c < 3; ++c) {
-            cj[(f * 7 + q) * 3 + c] = accj[q][c];
-            cm[(f * 7 + q) * 3 + c] = accm[q][c];
-        }
+    for (int t = 0; t < 2; ++t) {
+        double* u = o + 3 + 8 * t;
+        u[0] = a[t].re; u[1] = a[t].im;
+        for (int k = 0; k < 3; ++k) { u[2 + 2 * k] = aA[t][k].re; u[3 + 2 * k] = aA[t][k].im; }
+    }
+    for (int q = 0; q < 7; ++q) {
+        const double xi = rule.xi[q], eta = rule.eta[q], zeta = 1.0 - xi - eta;
+        const d3 r = v[0] * zeta + v[1] * xi + v[2] * eta - c;
+        o[19 + 3 * q] = r.x; o[20 + 3 * q] = r.y; o[21 + 3 * q] = r.z;
+    }
 }
 
 // Far-field operator as a matrix: rows (F_theta of direction d, then F_phi),
@@ -298,60 +310,94 @@ __global__ void ff_matrix_kernel(const double* __restrict__ V, const int* __rest
     A[(ndir + d) * cols + ne + e] = cx(0, 0) - coeff * nt;
 }
 
-__global__ void ff_directions_kernel(const d3* __restrict__ rq, const cplx* __restrict__ cj,
-                                     const cplx* __restrict__ cm, int64_t M, double k0, double eta0,
-                                     const double* __restrict__ rh, const double* __restrict__ th,
-                                     const double* __restrict__ ph, cplx* __restrict__ ft,
-                                     cplx* __restrict__ fp, double* __restrict__ U) {
-    const int d = blockIdx.x;
-    const d3 r = mk3(rh[3 * d], rh[3 * d + 1], rh[3 * d + 2]);
+// One thread per direction, blockIdx.y a chunk of faces whose records are
+// staged in shared memory (all lanes read the same word). Bound: the FP64 pipe,
+// 28 instructions per sample (3 for the path, 15 for the phase factor, 10 for
+// the moments) and 51 per face. part: [chunk][direction][N, L: 12].
+constexpr int kFarThreads = 128, kFarStage = 32;
+template <bool BIG>
+__global__ void __launch_bounds__(kFarThreads)
+ff_directions_kernel(const double* __restrict__ rec, int nf, int faces_per_chunk, const FarRule rule, const Wave wave,
+                     int64_t ndir, const double* __restrict__ rh, double* __restrict__ part) {
+    __shared__ __align__(16) double2 tab[kTurn * kTurnCopies];
+    __shared__ double sr[kFarStage * kFarRow];
+    fill_turn_table(tab);
+    const double2* my_tab = tab + (threadIdx.x & (kTurnCopies - 1));
+    const int64_t d = (int64_t)blockIdx.x * kFarThreads + threadIdx.x;
+    const int64_t dd = d < ndir ? d : ndir - 1;
+    const d3 r = mk3(rh[3 * dd], rh[3 * dd + 1], rh[3 * dd + 2]);
     cplx acc[6];
+#pragma unroll
     for (int c = 0; c < 6; ++c) acc[c] = cx(0, 0);
-    for (int64_t i = threadIdx.x; i < M; i += blockDim.x) {
-        const double phase = k0 * dot3(r, rq[i]);
-        double sn, cs;
-        sincos(phase, &sn, &cs);
-        const cplx e = cx(cs, sn);
-        for (int c = 0; c < 3; ++c) {
-            acc[c] += e * cj[i * 3 + c];
-            acc[3 + c] += e * cm[i * 3 + c];
-        }
-    }
-    __shared__ cplx red[6][32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int c = 0; c < 6; ++c) {
-        double re = acc[c].re, im = acc[c].im;
-        for (int o = 16; o > 0; o >>= 1) {
-            re += __shfl_xor_sync(0xffffffffu, re, o);
-            im += __shfl_xor_sync(0xffffffffu, im, o);
-        }
-        if (lane == 0) red[c][warp] = cx(re, im);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const int nw = blockDim.x >> 5;
-        cplx Nv[3], Lv[3];
-        for (int c = 0; c < 3; ++c) {
-            Nv[c] = cx(0, 0);
-            Lv[c] = cx(0, 0);
-            for (int w = 0; w < nw; ++w) {
-                Nv[c] += red[c][w];
-                Lv[c] += red[3 + c][w];
+    const int f1 = min(nf, (int)(blockIdx.y + 1) * faces_per_chunk);
+    for (int f0 = blockIdx.y * faces_per_chunk; f0 < f1; f0 += kFarStage) {
+        const int n = min(kFarStage, f1 - f0);
+        __syncthreads();
+        for (int t = threadIdx.x; t < n * kFarRow; t += kFarThreads) sr[t] = rec[(size_t)f0 * kFarRow + t];
+        __syncthreads();
+        for (int f = 0; f < n; ++f) {
+            const double* o = sr + f * kFarRow;
+            const double x0 = r.x * o[0] + r.y * o[1] + r.z * o[2];
+            cplx S0 = cx(0, 0), Sq[3] = {cx(0, 0), cx(0, 0), cx(0, 0)};
+#pragma unroll
+            for (int q = 0; q < 7; ++q) {
+                const double qx = o[19 + 3 * q], qy = o[20 + 3 * q], qz = o[21 + 3 * q];
+                const double x = fma(r.x, qx, fma(r.y, qy, fma(r.z, qz, x0)));
+                double c, s;
+                if (BIG) sincos(wave.k * x, &s, &c);
+                else phase_cs(my_tab, wave, x, c, s);
+                const cplx e = cx(c * rule.w[q], s * rule.w[q]);
+                S0 += e;
+                Sq[0].re = fma(e.re, qx, Sq[0].re); Sq[0].im = fma(e.im, qx, Sq[0].im);
+                Sq[1].re = fma(e.re, qy, Sq[1].re); Sq[1].im = fma(e.im, qy, Sq[1].im);
+                Sq[2].re = fma(e.re, qz, Sq[2].re); Sq[2].im = fma(e.im, qz, Sq[2].im);
+            }
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                const double* u = o + 3 + 8 * t;
+                const cplx a = cx(u[0], u[1]);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) acc[3 * t + c] += a * Sq[c] - cx(u[2 + 2 * c], u[3 + 2 * c]) * S0;
             }
         }
-        const double* t = th + 3 * d;
-        const double* p = ph + 3 * d;
-        const cplx nt = Nv[0] * t[0] + Nv[1] * t[1] + Nv[2] * t[2];
-        const cplx np = Nv[0] * p[0] + Nv[1] * p[1] + Nv[2] * p[2];
-        const cplx lt = Lv[0] * t[0] + Lv[1] * t[1] + Lv[2] * t[2];
-        const cplx lp = Lv[0] * p[0] + Lv[1] * p[1] + Lv[2] * p[2];
-        const cplx coeff = cx(0.0, -k0 / (4.0 * 3.14159265358979323846));
-        const cplx a = coeff * (nt * eta0 + lp);
-        const cplx b = coeff * (np * eta0 - lt);
-        ft[d] = a;
-        fp[d] = b;
-        U[d] = (a.re * a.re + a.im * a.im + b.re * b.re + b.im * b.im) / (2.0 * eta0);
     }
+    if (d >= ndir) return;
+    double* o = part + ((size_t)blockIdx.y * ndir + d) * 12;
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+        o[2 * c] = acc[c].re;
+        o[2 * c + 1] = acc[c].im;
+    }
+}
+
+// Sums the chunks of each direction in order and projects N and L.
+__global__ void ff_finish_kernel(const double* __restrict__ part, int chunks, int64_t ndir, double k0, double eta0,
+                                 const double* __restrict__ th, const double* __restrict__ ph, cplx* __restrict__ ft,
+                                 cplx* __restrict__ fp, double* __restrict__ U) {
+    const int64_t d = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (d >= ndir) return;
+    double v[12];
+#pragma unroll
+    for (int c = 0; c < 12; ++c) v[c] = 0.0;
+    for (int k = 0; k < chunks; ++k) {
+        const double* o = part + ((size_t)k * ndir + d) * 12;
+#pragma unroll
+        for (int c = 0; c < 12; ++c) v[c] += o[c];
+    }
+    const cplx Nv[3] = {cx(v[0], v[1]), cx(v[2], v[3]), cx(v[4], v[5])};
+    const cplx Lv[3] = {cx(v[6], v[7]), cx(v[8], v[9]), cx(v[10], v[11])};
+    const double* t = th + 3 * d;
+    const double* p = ph + 3 * d;
+    const cplx nt = Nv[0] * t[0] + Nv[1] * t[1] + Nv[2] * t[2];
+    const cplx np = Nv[0] * p[0] + Nv[1] * p[1] + Nv[2] * p[2];
+    const cplx lt = Lv[0] * t[0] + Lv[1] * t[1] + Lv[2] * t[2];
+    const cplx lp = Lv[0] * p[0] + Lv[1] * p[1] + Lv[2] * p[2];
+    const cplx coeff = cx(0.0, -k0 / (4.0 * 3.14159265358979323846));
+    const cplx a = coeff * (nt * eta0 + lp);
+    const cplx b = coeff * (np * eta0 - lt);
+    ft[d] = a;
+    fp[d] = b;
+    U[d] = (a.re * a.re + a.im * a.im + b.re * b.re + b.im * b.im) / (2.0 * eta0);
 }
 
 }  // namespace
@@ -519,18 +565,26 @@ int far_field_device(sieb200_ctx* ctx, const sieb200_mesh& mesh, const double* j
                      double* intensity) {
     const int nf = (int)mesh.num_faces, ne = (int)mesh.num_edges, nv = (int)mesh.num_vertices;
     cudaStream_t st = ctx->stream;
-    const int64_t M = (int64_t)nf * 7;
+    // Chunks of faces: some 16 CTAs per SM in all, whole staging rounds each.
+    const int64_t dir_blocks = std::max<int64_t>(1, (ndir + kFarThreads - 1) / kFarThreads);
+    const int64_t want = ((int64_t)ctx->sm_count * 16 + dir_blocks - 1) / dir_blocks;
+    const int rounds = (nf + kFarStage - 1) / kFarStage;
+    const int64_t split = std::min<int64_t>(rounds, want);
+    const int per_chunk = kFarStage * (int)((rounds + split - 1) / split);
+    const int chunks = (nf + per_chunk - 1) / per_chunk;
     size_t off = 0;
     auto take = [&](size_t bytes) { size_t o = off; off += ((bytes + 255) / 256) * 256; return o; };
     const size_t oV = take(sizeof(double) * 3 * nv), oF = take(sizeof(int) * 3 * nf),
                  oFE = take(sizeof(int) * 3 * nf), oJ = take(sizeof(cplx) * ne),
-                 oM = take(sizeof(cplx) * ne), oRq = take(sizeof(d3) * M),
-                 oCj = take(sizeof(cplx) * 3 * M), oCm = take(sizeof(cplx) * 3 * M),
+                 oM = take(sizeof(cplx) * ne), oRec = take(sizeof(double) * kFarRow * nf),
+                 oPart = take(sizeof(double) * 12 * (size_t)chunks * ndir),
                  oDir = take(sizeof(double) * 9 * ndir), oOut = take(sizeof(cplx) * 2 * ndir),
                  oU = take(sizeof(double) * ndir);
     DeviceBuffer buf;
     SIEB_RETURN_IF(buf.reserve(off));
     char* b = buf.as<char>();
+    double* rec = reinterpret_cast<double*>(b + oRec);
+    double* part = reinterpret_cast<double*>(b + oPart);
     SIEB_TRY_CUDA(cudaMemcpyAsync(b + oV, mesh.vertices, sizeof(double) * 3 * nv, cudaMemcpyHostToDevice, st));
     SIEB_TRY_CUDA(cudaMemcpyAsync(b + oF, mesh.faces, sizeof(int) * 3 * nf, cudaMemcpyHostToDevice, st));
     SIEB_TRY_CUDA(cudaMemcpyAsync(b + oFE, mesh.faces_edges, sizeof(int) * 3 * nf, cudaMemcpyHostToDevice, st));
@@ -539,20 +593,27 @@ int far_field_device(sieb200_ctx* ctx, const sieb200_mesh& mesh, const double* j
     SIEB_TRY_CUDA(cudaMemcpyAsync(b + oDir, rh, sizeof(double) * 3 * ndir, cudaMemcpyHostToDevice, st));
     SIEB_TRY_CUDA(cudaMemcpyAsync(b + oDir + sizeof(double) * 3 * ndir, th, sizeof(double) * 3 * ndir, cudaMemcpyHostToDevice, st));
     SIEB_TRY_CUDA(cudaMemcpyAsync(b + oDir + sizeof(double) * 6 * ndir, ph, sizeof(double) * 3 * ndir, cudaMemcpyHostToDevice, st));
-    ff_samples_kernel<<<(nf + 127) / 128, 128, 0, st>>>(
-        reinterpret_cast<double*>(b + oV), reinterpret_cast<int*>(b + oF),
-        reinterpret_cast<int*>(b + oFE), nf, reinterpret_cast<cplx*>(b + oJ),
-        m_cur ? reinterpret_cast<cplx*>(b + oM) : nullptr, reinterpret_cast<d3*>(b + oRq),
-        reinterpret_cast<cplx*>(b + oCj), reinterpret_cast<cplx*>(b + oCm));
+    const FarRule rule = far_rule();
+    ff_faces_kernel<<<(nf + 127) / 128, 128, 0, st>>>(
+        reinterpret_cast<double*>(b + oV), reinterpret_cast<int*>(b + oF), reinterpret_cast<int*>(b + oFE), nf, rule,
+        reinterpret_cast<cplx*>(b + oJ), m_cur ? reinterpret_cast<cplx*>(b + oM) : nullptr, rec);
     SIEB_NOTE_LAUNCH();
     SIEB_TRY_CUDA(cudaGetLastError());
     if (ndir > 0) {
         double* dd = reinterpret_cast<double*>(b + oDir);
-        ff_directions_kernel<<<(unsigned)ndir, 256, 0, st>>>(
-            reinterpret_cast<d3*>(b + oRq), reinterpret_cast<cplx*>(b + oCj),
-            reinterpret_cast<cplx*>(b + oCm), M, k0, eta0, dd, dd + 3 * ndir, dd + 6 * ndir,
-            reinterpret_cast<cplx*>(b + oOut), reinterpret_cast<cplx*>(b + oOut) + ndir,
-            reinterpret_cast<double*>(b + oU));
+        // |r_hat . r_q| is at most |r_hat| times the sum of the largest coordinates
+        double ext = 0.0, rmax = 0.0;
+        for (int64_t i = 0; i < 3 * (int64_t)nv; ++i) ext = std::max(ext, std::fabs(mesh.vertices[i]));
+        for (int64_t i = 0; i < 3 * ndir; ++i) rmax = std::max(rmax, std::fabs(rh[i]));
+        const bool big = !(k0 * 3.0 * ext * rmax < kPhaseMax);
+        auto* kernel = big ? ff_directions_kernel<true> : ff_directions_kernel<false>;
+        kernel<<<dim3((unsigned)dir_blocks, (unsigned)chunks), kFarThreads, 0, st>>>(rec, nf, per_chunk, rule,
+                                                                                     make_wave(k0), ndir, dd, part);
+        SIEB_NOTE_LAUNCH();
+        SIEB_TRY_CUDA(cudaGetLastError());
+        ff_finish_kernel<<<(unsigned)((ndir + 127) / 128), 128, 0, st>>>(
+            part, chunks, ndir, k0, eta0, dd + 3 * ndir, dd + 6 * ndir, reinterpret_cast<cplx*>(b + oOut),
+            reinterpret_cast<cplx*>(b + oOut) + ndir, reinterpret_cast<double*>(b + oU));
         SIEB_NOTE_LAUNCH();
         SIEB_TRY_CUDA(cudaGetLastError());
         SIEB_TRY_CUDA(cudaMemcpyAsync(f_theta, b + oOut, sizeof(cplx) * ndir, cudaMemcpyDeviceToHost, st));
