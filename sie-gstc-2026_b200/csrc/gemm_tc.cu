@@ -482,6 +482,233 @@ gemm_tf32_sub_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const _
     }
 }
 
+// ------------------------------------------------ scaled FP16 split operands
+// The trailing updates of the blocked schedule (mixed.cu):
+//   C -= (A_hi B_hi^T + 2^-11 (A_hi B_lo^T + A_lo B_hi^T)) / s
+// with sA A = A_hi + 2^-11 A_lo and sB B = B_hi + 2^-11 B_lo in FP16 (s = sA sB,
+// powers of two): 11 + 11 significant bits, as many as the TF32 split, at twice
+// the tensor rate and half the operand bytes. lo is kept 2^11 up, so that it has
+// hi's exponent range; the two mixed products share one accumulator, hi.hi has
+// the other, and the epilogue joins them.
+// The tensor core's own accumulation truncates, so a sum over all of K = 512
+// loses more than the single-step schedule's sums over 128 did. The epilogue
+// warps therefore take the accumulator over after every 128 columns of K
+// (H_CHUNK stages) and add it up in registers, rounding to nearest, while the
+// next chunk's MMAs fill the other accumulator: 600 of a chunk's 1500 cycles.
+// One preconditioned step's residual against the TF32 single-step schedule's:
+// 1.0-1.4 times without this, 0.7-1.0 with it (systems of 1000 to 17280).
+// Persistent, one CTA per SM, 128 x 128 tiles; 192 threads in the roles of
+// gemm_tf32_sub_persistent_kernel<REDUCE, HILO>. A stage holds 64 columns
+// (128 bytes) of [A_hi | A_lo] and [B_hi | B_lo], 64 KB; three stages fit beside
+// two 32-column C slots (the TF32 kernel had two stages and four slots): with
+// K = 512 the operand stream, 1 KB per tile and column of K, is what bounds the
+// kernel, and a third stage covers its latency.
+// Tiles (HalfTiles): region 1 is all row tiles against the first w columns,
+// region 2 the first r2 row tiles against the rest: w = N is a whole trailing
+// update, w < N the L-shaped border a block step updates at once. The first
+// row tile starts shift0 columns in (the next diagonal block is updated
+// elsewhere). Columns are written in 32-column slots up to the region's end.
+constexpr int H_BK = 64;                 // FP16 columns per stage: one 128-byte swizzle row
+constexpr int H_OPB = BM * H_BK * 2;     // bytes of a 128-row hi or lo operand block
+constexpr int H_STAGE = 4 * H_OPB;
+constexpr int H_NS = 3;
+constexpr int H_CHUNK = 2;               // stages per accumulator pass
+constexpr int H_CC = 32;                 // columns per C slot
+constexpr int H_CSLOT = BM * H_CC * 4;
+constexpr int H_SMEM_BYTES = H_NS * H_STAGE + 2 * H_CSLOT + 1024 /*align*/ + 256 /*barriers*/;
+static_assert(H_SMEM_BYTES <= 227 * 1024, "shared memory of the FP16 split GEMM");
+
+struct HalfTiles {
+    int mt, r2, w, N, shift0, tiles1, tiles;
+};
+
+// D f32, A and B f16, both K-major.
+constexpr uint32_t idesc_f16(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BM >> 4) << 24); }
+
+__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate,
+                                         uint32_t idesc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
+}
+
+__global__ void __launch_bounds__(P_THREADS, 1)
+gemm_f16_sub_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                    const __grid_constant__ CUtensorMap tmC, const HalfTiles tl, int k0, int klo, int kblocks,
+                    const unsigned* __restrict__ scale_bits, unsigned* err) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    const uint32_t raw = smem_u32(smem_raw);
+    const uint32_t base = (raw + 1023u) & ~1023u;
+    unsigned char* gbase = smem_raw + (base - raw);
+    const uint32_t sC = base + H_NS * H_STAGE;
+    float* cs = reinterpret_cast<float*>(gbase + H_NS * H_STAGE);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(gbase + H_NS * H_STAGE + 2 * H_CSLOT);
+    const uint32_t full0 = smem_u32(&bars[0]);
+    const uint32_t empty0 = smem_u32(&bars[H_NS]);
+    const uint32_t accf0 = smem_u32(&bars[2 * H_NS]);      // accumulator b ready (MMA -> epilogue)
+    const uint32_t acce0 = smem_u32(&bars[2 * H_NS + 2]);  // accumulator b drained (epilogue -> MMA)
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(&bars[2 * H_NS + 4]);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    // Tile t: row tile, first column, end of its region; empty tiles are
+    // skipped alike by the three roles.
+    auto locate = [&](int t, int& rt, int& col, int& lim) {
+        if (t < tl.tiles1) {
+            rt = t % tl.mt;
+            col = (t / tl.mt) * BN + (rt == 0 ? tl.shift0 : 0);
+            lim = tl.w;
+        } else {
+            const int u = t - tl.tiles1;
+            rt = u % tl.r2;
+            col = tl.w + (u / tl.r2) * BN;
+            lim = tl.N;
+        }
+        return col < lim;
+    };
+    auto from = [&](int t, int& rt, int& col, int& lim) {
+        while (t < tl.tiles && !locate(t, rt, col, lim)) t += gridDim.x;
+        return t;
+    };
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < H_NS; ++s) {
+            mbar_init(full0 + 8 * s, 1);
+            mbar_init(empty0 + 8 * s, 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(accf0 + 8 * b, 1);
+            mbar_init(acce0 + 8 * b, 4);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                     "r"(4 * BN));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
+
+    int rt = 0, col = 0, lim = 0;
+    if (warp == 0) {
+        if (lane == 0) {
+            int g = 0;
+            bool ok = true;
+            for (int t = from(blockIdx.x, rt, col, lim); t < tl.tiles && ok; t = from(t + gridDim.x, rt, col, lim)) {
+                for (int kb = 0; kb < kblocks; ++kb, ++g) {
+                    const int s = g % H_NS;
+                    const uint32_t ph = (uint32_t)(g / H_NS) & 1u;
+                    if (!mbar_wait(empty0 + 8 * s, ph ^ 1u, err)) { ok = false; break; }
+                    const uint32_t dst = base + s * H_STAGE, bar = full0 + 8 * s;
+                    mbar_expect_tx(bar, H_STAGE);
+                    tma_load_2d(dst, &tmA, bar, k0 + kb * H_BK, rt * BM);
+                    tma_load_2d(dst + 2 * H_OPB, &tmB, bar, k0 + kb * H_BK, col);
+                    tma_load_2d(dst + 3 * H_OPB, &tmB, bar, klo + kb * H_BK, col);
+                    tma_load_2d(dst + H_OPB, &tmA, bar, klo + kb * H_BK, rt * BM);
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            int g = 0, li = 0;
+            bool ok = true;
+            for (int t = from(blockIdx.x, rt, col, lim); t < tl.tiles && ok; t = from(t + gridDim.x, rt, col, lim)) {
+                for (int kb = 0; kb < kblocks; ++kb, ++g) {
+                    const int s = g % H_NS, kc = kb % H_CHUNK;
+                    const int b = li & 1;  // li counts chunks
+                    if (kc == 0) {
+                        if (!mbar_wait(acce0 + 8 * b, ((uint32_t)(li >> 1) & 1u) ^ 1u, err)) { ok = false; break; }
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    }
+                    const uint32_t acc = tmem + (uint32_t)(b * 2 * BN);
+                    if (!mbar_wait(full0 + 8 * s, (uint32_t)(g / H_NS) & 1u, err)) { ok = false; break; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint64_t ah = smem_desc_sw128(base + s * H_STAGE);
+                    const uint64_t al = smem_desc_sw128(base + s * H_STAGE + H_OPB);
+                    const uint64_t bd = smem_desc_sw128(base + s * H_STAGE + 2 * H_OPB);  // [B_hi; B_lo]
+#pragma unroll
+                    for (int k = 0; k < H_BK / 16; ++k) {  // 16 FP16 = 32 bytes per instruction
+                        umma_f16(acc, ah + 2 * k, bd + 2 * k, (kc | k) != 0 ? 1u : 0u, idesc_f16(2 * BN));
+                        umma_f16(acc + BN, al + 2 * k, bd + 2 * k, 1u, idesc_f16(BN));
+                    }
+                    umma_commit(empty0 + 8 * s);
+                    if (kc == H_CHUNK - 1 || kb == kblocks - 1) {
+                        umma_commit(accf0 + 8 * b);
+                        ++li;
+                    }
+                }
+            }
+        }
+    } else {
+        const int q = warp & 3;            // TMEM lane quarter of this warp
+        const int row = q * 32 + lane;     // row of the tile
+        const bool e0 = threadIdx.x == 64;
+        const float inv = 1.0f / (kHalfScaleA * half_scale(*scale_bits));
+        const int chunks = (kblocks + H_CHUNK - 1) / H_CHUNK;
+        int li = 0;
+        for (int t = from(blockIdx.x, rt, col, lim); t < tl.tiles; t = from(t + gridDim.x, rt, col, lim)) {
+            float sum[BN];
+#pragma unroll
+            for (int j = 0; j < BN; ++j) sum[j] = 0.f;
+            int got = 1;
+#pragma unroll 1
+            for (int ch = 0; ch < chunks && got; ++ch, ++li) {
+                const int b = li & 1;
+                if (lane == 0) got = mbar_wait(accf0 + 8 * b, (uint32_t)(li >> 1) & 1u, err) ? 1 : 0;
+                got = __shfl_sync(0xffffffffu, got, 0);
+                __syncwarp();
+                if (!got) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * 2 * BN);
+#pragma unroll
+                for (int c = 0; c < BN / 32; ++c) {
+                    float v[32], w[32];
+                    tmem_ld32(ta + c * 32, v);
+                    tmem_ld32(ta + BN + c * 32, w);
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) sum[c * 32 + j] += fmaf(w[j], 0x1p-11f, v[j]);
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(acce0 + 8 * b);
+            }
+            const int slots = min(BN / H_CC, (lim - col + H_CC - 1) / H_CC);
+#pragma unroll
+            for (int c = 0; c < BN / H_CC; ++c) {
+                if (c >= slots) break;
+                float* cc = cs + (c & 1) * (BM * H_CC);
+#pragma unroll
+                for (int j = 0; j < H_CC; ++j) cc[j * BM + row] = -sum[c * H_CC + j] * inv;
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                epilogue_bar();
+                if (e0) {
+                    if (got) tma_reduce_add_2d(&tmC, sC + (c & 1) * H_CSLOT, rt * BM, col + c * H_CC);
+                    bulk_commit();
+                    // the other slot is written next: its reduction has to be read
+                    bulk_wait_read<1>();
+                }
+                epilogue_bar();
+            }
+            // slot 0 starts the next tile: after an odd number of slots it was the last one reduced
+            if (slots & 1) {
+                if (e0) bulk_wait_read_all();
+                epilogue_bar();
+            }
+        }
+        if (e0) bulk_wait_all();
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 1) {
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(4 * BN));
+    }
+}
+
 // SIMT reference on the same packed operands (checking path).
 // hilo: A = [A_hi | A_lo], B = [B_hi | B_lo] along K; the sum is
 // a_hi (b_hi + b_lo) + a_lo b_hi per k of the first half.
@@ -566,6 +793,7 @@ struct GemmTC {
     int lolo = 0;     // split operands: also the product A_lo B_lo^T
     bool attr_set = false;
     bool attr_set_p[8] = {};
+    bool attr_set_h = false;
     int sms = 148;
 };
 
@@ -633,6 +861,8 @@ void gemm_tc_destroy(GemmTC* g) {
 
 void gemm_tc_set_mode(GemmTC* g, int mode) { g->mode = mode; }
 
+bool gemm_tc_default(const GemmTC* g) { return g->mode == 3 && g->c_slots == 4 && g->lolo == 0; }
+
 int gemm_tc_sub(GemmTC* g, cudaStream_t stream, float* C, int64_t ldc, const float* A, const float* B,
                 int64_t M2, int64_t N, int K, int max_ctas, int layout, int64_t shift0) {
     SIEB_CHECK(K % BK == 0 && K > 0, SIEB200_INVALID_ARG, "GEMM K must be a positive multiple of 32");
@@ -680,6 +910,45 @@ int gemm_tc_sub(GemmTC* g, cudaStream_t stream, float* C, int64_t ldc, const flo
     }
     const dim3 grid((unsigned)((M2 + BM - 1) / BM), (unsigned)((N + BN - 1) / BN));
     gemm_tf32_sub_kernel<<<grid, 128, SMEM_BYTES, stream>>>(ma, mb, C, ldc, (int)M2, (int)N, K, (int)shift0, g->err);
+    SIEB_NOTE_LAUNCH();
+    SIEB_TRY_CUDA(cudaGetLastError());
+    return SIEB200_OK;
+}
+
+int gemm_half_sub(GemmTC* g, cudaStream_t stream, float* C, int64_t ldc, const __half* A, const __half* B, int64_t ld,
+                  int64_t M2, int64_t N, int64_t w, int k0, int klo, int K, const unsigned* scale_bits, int max_ctas,
+                  int64_t shift0) {
+    SIEB_CHECK(K > 0 && K % H_BK == 0 && k0 >= 0 && k0 % H_BK == 0 && klo % H_BK == 0 && klo + K <= ld && ld % 8 == 0,
+               SIEB200_INVALID_ARG, "FP16 split GEMM: K offsets must be multiples of 64 inside the packs");
+    SIEB_CHECK(M2 > 0 && N > 0 && M2 < (1ll << 31) && N < (1ll << 31) && w > 0 && w <= N && (w == N || w % 64 == 0),
+               SIEB200_INVALID_ARG, "GEMM size out of range");
+    SIEB_CHECK(shift0 >= 0 && shift0 < N, SIEB200_INVALID_ARG, "GEMM first-row-tile column shift out of range");
+    SIEB_CHECK(((uintptr_t)A % 16) == 0 && ((uintptr_t)B % 16) == 0 && ((uintptr_t)C % 16) == 0 && (ldc * 4) % 16 == 0,
+               SIEB200_INVALID_ARG, "GEMM operands must be 16-byte aligned");
+    CUtensorMap ma, mb, mc;
+    for (int i = 0; i < 2; ++i)
+        SIEB_RETURN_IF(encode_tensor_map_2d(i ? &mb : &ma, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, i ? B : A, (uint64_t)ld,
+                                            (uint64_t)(i ? N : M2), (uint64_t)ld * 2, H_BK, BM,
+                                            CU_TENSOR_MAP_SWIZZLE_128B));
+    SIEB_RETURN_IF(encode_tensor_map_2d(&mc, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, C, (uint64_t)M2, (uint64_t)N,
+                                        (uint64_t)ldc * sizeof(float), BM, H_CC, CU_TENSOR_MAP_SWIZZLE_NONE));
+    HalfTiles tl;
+    tl.mt = (int)((M2 + BM - 1) / BM);
+    tl.w = (int)w;
+    tl.N = (int)N;
+    tl.shift0 = (int)shift0;
+    tl.r2 = (int)(w < N ? std::min<int64_t>(tl.mt, 2 * w / BM) : 0);
+    tl.tiles1 = tl.mt * (int)((w + BN - 1) / BN);
+    tl.tiles = tl.tiles1 + tl.r2 * (int)((N - w + BN - 1) / BN);
+    const int cap = max_ctas > 0 ? std::min(max_ctas, g->sms) : g->sms;
+    const unsigned grid = (unsigned)std::min(tl.tiles, std::max(1, cap));
+    if (!g->attr_set_h) {
+        SIEB_TRY_CUDA(cudaFuncSetAttribute(gemm_f16_sub_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           H_SMEM_BYTES));
+        g->attr_set_h = true;
+    }
+    gemm_f16_sub_kernel<<<grid, P_THREADS, H_SMEM_BYTES, stream>>>(ma, mb, mc, tl, k0, klo, K / H_BK, scale_bits,
+                                                                   g->err);
     SIEB_NOTE_LAUNCH();
     SIEB_TRY_CUDA(cudaGetLastError());
     return SIEB200_OK;

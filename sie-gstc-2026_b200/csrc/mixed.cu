@@ -104,11 +104,12 @@ __global__ void rbt_init_kernel(double* diag, int64_t np, uint64_t seed) {
     diag[i] = rbt_value(seed, i);
 }
 
-// W = U^T A_pad V, read A (c128, n x n, lda) once, write W (c64).
+// W = U^T A_pad V, read A (c128, n x n, lda) once, write W (c64); wmax (optional)
+// receives the bits of W's largest component.
 template <class T>
 __global__ void rbt_matrix_kernel(const cplx* __restrict__ A, int64_t lda, int64_t n, int64_t np,
                                   const double* __restrict__ du, const double* __restrict__ dv,
-                                  T* __restrict__ W, int64_t ldw) {
+                                  T* __restrict__ W, int64_t ldw, unsigned* __restrict__ wmax) {
     const int64_t q = np / 4;
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t j = blockIdx.y;
@@ -147,6 +148,16 @@ __global__ void rbt_matrix_kernel(const cplx* __restrict__ A, int64_t lda, int64
 #pragma unroll
         for (int s = 0; s < 4; ++s)
             W[(i + s * q) + (j + t * q) * ldw] = T{(decltype(T::x))blk[s][t].re, (decltype(T::x))blk[s][t].im};
+    if (wmax) {  // largest component of W, as float bits (ordered like the values)
+        float mx = 0.f;
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+#pragma unroll
+            for (int s = 0; s < 4; ++s)
+                mx = fmaxf(mx, fmaxf(fabsf((float)blk[s][t].re), fabsf((float)blk[s][t].im)));
+        const unsigned m = __reduce_max_sync(__activemask(), __float_as_uint(mx));
+        if (m > *reinterpret_cast<volatile unsigned*>(wmax)) atomicMax(wmax, m);
+    }
 }
 
 // y = U^T x_pad (vector); x has n entries (rest treated as 0).
@@ -805,10 +816,25 @@ struct PanelArgs {
     int64_t b_ld = 0, b_c0 = 0;
     int64_t a_lo = 0, b_lo = 0;
     int lo_rn = 0;  // lo parts rounded to the nearest TF32
+    // pack 2: scaled FP16 split instead, strides and offsets in FP16 values
+    // (lo kept 2^11 up, L21 times kHalfScaleA, U12 times half_scale(*wmax); a
+    // value outside FP16's range sets the error word to 4)
+    __half* Ah = nullptr;
+    __half* Bh = nullptr;
+    const unsigned* wmax = nullptr;
+    unsigned* err = nullptr;
     // CTA range of one launch: L21 row blocks and U12 column blocks
     // [b_first, b_first + nl_run) of 32 each (nl_run 0: all nL from 0)
     int b_first = 0, nl_run = 0;
 };
+
+// v = h + 2^-11 l in FP16, both rounded to nearest.
+__device__ __forceinline__ void split_half(float2 v, __half2& h, __half2& l, unsigned* err) {
+    if (!(fmaxf(fabsf(v.x), fabsf(v.y)) <= 65504.f)) atomicCAS(err, 0u, 4u);
+    h = __floats2half2_rn(v.x, v.y);
+    const float2 r = __half22float2(h);
+    l = __floats2half2_rn((v.x - r.x) * 2048.f, (v.y - r.y) * 2048.f);
+}
 
 // L21 = A21 * inv(U11) for rows [s0, np) of the panel columns [k0, k0+kb);
 // writes L21 back into W and the split realified rows into Apack.
@@ -949,6 +975,26 @@ __device__ __forceinline__ void panel_L_body(T* __restrict__ W, int64_t ldw, con
     }
     if constexpr (!std::is_same<T, float2>::value) return;
     if (!pa.pack) return;
+    if constexpr (std::is_same<T, float2>::value) {
+        if (pa.pack == 2) {
+            for (int e = tid; e < 32 * NB; e += blockDim.x) {
+                const int rr = e / NB, c = e % NB;
+                const int64_t gr = rb + rr;
+                if (gr >= np) continue;
+                const float2 v = Ar[rr][c];
+                __half2 h, l;
+                split_half(make_float2(v.x * kHalfScaleA, v.y * kHalfScaleA), h, l, pa.err);
+                __half2* row0 = reinterpret_cast<__half2*>(pa.Ah + 2 * (gr - pa.a_r0) * pa.a_ld) + c;
+                __half2* row1 = reinterpret_cast<__half2*>(pa.Ah + (2 * (gr - pa.a_r0) + 1) * pa.a_ld) + c;
+                const int64_t lo = pa.a_lo / 2;
+                row0[0] = __halves2half2(__low2half(h), __hneg(__high2half(h)));
+                row1[0] = __lowhigh2highlow(h);
+                row0[lo] = __halves2half2(__low2half(l), __hneg(__high2half(l)));
+                row1[lo] = __lowhigh2highlow(l);
+            }
+            return;
+        }
+    }
     // ... and to the split realified rows (K fastest: coalesced rows).
     // row 2i: [Re, -Im] per column, row 2i+1: [Im, Re]; layout [hi | hi | lo].
     for (int e = tid; e < 32 * 2 * NB; e += blockDim.x) {
@@ -1095,12 +1141,23 @@ __device__ __forceinline__ void panel_U_body(T* __restrict__ W, int64_t ldw, con
 #pragma unroll
         for (int j = 0; j < 2; ++j) Ac[2 * tx + j][row[i]] = acc[i][j];
     __syncthreads();
+    const float bscale = pa.pack == 2 ? half_scale(*pa.wmax) : 1.f;
     for (int e = tid; e < 32 * NB; e += blockDim.x) {
         const int r = e % NB, c = e / NB;
         const int64_t gc = cb + c;
         if (gc >= np) continue;
         const T v = Ac[c][r];
         if (r < kb) W[(k0 + r) + gc * ldw] = v;
+        if constexpr (std::is_same<T, float2>::value) {
+            if (pa.pack == 2) {
+                __half2 h, l;
+                split_half(make_float2(v.x * bscale, v.y * bscale), h, l, pa.err);
+                __half2* col = reinterpret_cast<__half2*>(pa.Bh + (gc - pa.b_c0) * pa.b_ld) + r;
+                col[0] = h;
+                col[pa.b_lo / 2] = l;
+                continue;
+            }
+        }
         if (std::is_same<T, float2>::value && pa.pack && gc >= pa.b_c0) {
             float* col = pa.Bpack + (gc - pa.b_c0) * pa.b_ld;
             const float h0 = tf32_hi(v.x), h1 = tf32_hi(v.y);
@@ -2068,11 +2125,17 @@ void mixed_release(DenseSolver* s) {
     s->krylov.release(); s->vec.release(); s->flags.release(); s->gemv_scratch.release(); s->couple.release();
 }
 
-static int check_err(DenseSolver* s, const char* what) {
+// *overflow (optional) receives whether the FP16 packs overflowed, which is
+// then not an error.
+static int check_err(DenseSolver* s, const char* what, bool* overflow = nullptr) {
     MixedState* st = state_of(s);
     unsigned e = 0;
     SIEB_TRY_CUDA(cudaMemcpyAsync(&e, st->err, sizeof(unsigned), cudaMemcpyDeviceToHost, s->ctx->stream));
     SIEB_TRY_CUDA(cudaStreamSynchronize(s->ctx->stream));
+    if (overflow) {
+        *overflow = e == 4u;
+        if (e == 4u) return SIEB200_OK;
+    }
     if (e == 1u) {
         set_error(std::string(what) + ": zero or non-finite pivot in the unpivoted LU of the randomized matrix");
         return SIEB200_SINGULAR;
@@ -2110,6 +2173,10 @@ constexpr double kGmresEstFactorDefault = 0.9;
 constexpr int kOverlapSmsDefault = 20;
 // Split panels (SIEB200_PANEL_HEAD_MAX): 0 = off.
 constexpr int kPanelHeadMaxDefault = 0;
+// Block steps per group of the blocked schedule.
+constexpr int kGroup = 4;
+static_assert(kGroup >= 2 && kGroup * 8 * NB <= 2 * 6 * NB * (int)sizeof(float),
+              "a group's packs fit the buffers of the step packs");
 
 static int fp64_factorize(DenseSolver* s);
 
@@ -2137,6 +2204,7 @@ int mixed_factorize(DenseSolver* s) {
     st->pair = (pair_env && pair_env[0] == '1') ? 1 : 0;
     const char* pmin_env = getenv("SIEB200_PAIR_MIN");
     st->pair_min = pmin_env ? std::max(0, atoi(pmin_env)) : kPairMinDefault;
+    const bool pmin_env_on = pmin_env && st->pair_min > 0;
     const char* hilo_env = getenv("SIEB200_GEMM_HILO");
     st->hilo = (hilo_env && hilo_env[0] == '0') ? 0 : 1;
     const char* ovl_env = getenv("SIEB200_OVERLAP_MIN");
@@ -2211,24 +2279,40 @@ int mixed_factorize(DenseSolver* s) {
         attrs_set = true;
     }
 
+    // The blocked schedule (see mixed_enqueue) unless a switch asks for one of
+    // the single-step or pair schedules.
+    st->blocked = st->use_tc && gemm_tc_default(st->gemm) && st->hilo && st->lcol == 1 && !st->pair && !pmin_env_on &&
+                  st->ovl_min == 0 && !st->lo_rn;
+
     // Replay, capture or run eagerly (see MixedState::graphs).
     MixedState::GraphKey key;
     key.A = s->A; key.lda = s->lda; key.n = n; key.W = st->W; key.pack = st->Apack[0];
     const int gemm_sms = s->sm_cap > 0 ? std::min(s->sm_cap, ctx->sm_count - 1) : ctx->sm_count - 1;
     key.use_tc = st->use_tc + 2 * st->pair + 4 * st->hilo + 8 * st->lcol + 16 * st->lo_rn + 32 * st->diag_split +
-                 64 * st->diag_panels + 128 * st->diag_rec + 256 * st->diag_compact;
+                 64 * st->diag_panels + 128 * st->diag_rec + 256 * st->diag_compact + 512 * st->blocked;
     key.sms = gemm_sms;
     key.ovl = ((int64_t)st->pair_min << 32) | (int64_t)(st->ovl_min * 1000 + st->ovl_sms);
     key.head = ((int64_t)st->head_max << 20) | (int64_t)st->head_smem;
     const char* no_graphs = getenv("SIEB200_NO_GRAPHS");
     const bool graphs = !ctx->prof.enabled && !(no_graphs && no_graphs[0] == '1');
+    // A value of L21 or U12 outside FP16's range (element growth far beyond
+    // what the butterfly transform leaves in practice): factor again with the
+    // FP32 operands of the single-step schedule.
+    auto finish = [&]() -> int {
+        bool overflow = false;
+        SIEB_RETURN_IF(check_err(s, "mixed LU factorization", &overflow));
+        if (!overflow) return SIEB200_OK;
+        st->blocked = 0;
+        SIEB_RETURN_IF(mixed_enqueue(s, st, bFlags, K3));
+        return check_err(s, "mixed LU factorization");
+    };
     if (graphs) {
         for (auto& g : st->graphs) {
             if (g.exec && g.key == key) {
                 g.used = ++st->tick;
                 SIEB_TRY_CUDA(cudaGraphLaunch(g.exec, stream));
                 note_launches(g.launches);
-                return check_err(s, "mixed LU factorization");
+                return finish();
             }
         }
     }
@@ -2263,7 +2347,7 @@ int mixed_factorize(DenseSolver* s) {
     } else {
         SIEB_RETURN_IF(mixed_enqueue(s, st, bFlags, K3));
     }
-    return check_err(s, "mixed LU factorization");
+    return finish();
 }
 
 // Enqueues one mixed factorization on the context stream and the lookahead
@@ -2280,7 +2364,7 @@ static int mixed_enqueue(DenseSolver* s, MixedState* st, size_t bFlags, int K3) 
     SIEB_TRY_CUDA(cudaGetLastError());
     const int64_t q = np / 4;
     rbt_matrix_kernel<float2><<<dim3(blocks_for(q, 128), (unsigned)q), 128, 0, stream>>>(
-        reinterpret_cast<const cplx*>(s->A), s->lda, n, np, st->diag, st->diag + 4 * np, st->W, ldw);
+        reinterpret_cast<const cplx*>(s->A), s->lda, n, np, st->diag, st->diag + 4 * np, st->W, ldw, st->err + 1);
     SIEB_NOTE_LAUNCH();
     SIEB_TRY_CUDA(cudaGetLastError());
 
@@ -2405,6 +2489,91 @@ static int mixed_enqueue(DenseSolver* s, MixedState* st, size_t bFlags, int K3) 
         return SIEB200_OK;
     };
     const int gemm_ctas = s->sm_cap > 0 ? std::min(s->sm_cap, ctx->sm_count - 1) : ctx->sm_count - 1;
+
+    // Blocked schedule (default). Block steps in groups of kGroup: within a
+    // group a step's trailing update covers only the group's own rows and
+    // columns (an L-shaped border of the trailing matrix), and the rest takes
+    // all of the group's updates in one GEMM after its last step, K = kGroup x
+    // 128 of each operand half. The trailing matrix so moves through HBM once
+    // per group instead of once per step: with single steps that traffic, 16
+    // bytes per entry and step, was 66 of the 113 ms of an N = 17280
+    // factorization. A step's chain is as in the single-step schedule: panels,
+    // then the next diagonal block on the side stream beside the update.
+    if (st->blocked) {
+        __half* Ah = reinterpret_cast<__half*>(st->Apack[0]);
+        __half* Bh = reinterpret_cast<__half*>(st->Bpack);
+        const int LO = kGroup * 2 * NB;  // lo half of a pack row
+        const int64_t LD = 2 * LO;       // FP16 values per pack row
+        const unsigned* wmax = st->err + 1;
+        auto group_panels = [&](int64_t bk) -> int {
+            const int64_t k0 = bk * NB;
+            const int kb = (int)std::min<int64_t>(NB, np - k0);
+            const int64_t s0 = k0 + kb;
+            if (s0 >= np) return SIEB200_OK;
+            const int64_t m = np - s0, g0 = (bk / kGroup) * kGroup * NB;
+            PanelArgs pa;
+            pa.k0 = k0; pa.kb = kb; pa.s0 = s0; pa.np = np;
+            pa.nL = (int)blocks_for(m, 32);
+            pa.pack = 2;
+            pa.Ah = Ah + (bk % kGroup) * 2 * NB; pa.a_ld = LD; pa.a_r0 = g0; pa.a_lo = LO;
+            pa.Bh = Bh + (bk % kGroup) * 2 * NB; pa.b_ld = LD; pa.b_c0 = g0; pa.b_lo = LO;
+            pa.wmax = wmax;
+            pa.err = st->err;
+            cudaEvent_t ev;
+            ctx->prof.begin(stream, 4, 16.0 * NB * NB * (double)m, 32.0 * NB * (double)m, &ev);
+            panels_kernel<float2><<<(unsigned)(2 * pa.nL), 256, kSmemPanel, stream>>>(
+                st->W, ldw, st->Uinv + (size_t)bk * NB * NB, st->Linv + (size_t)bk * NB * NB, pa);
+            SIEB_NOTE_LAUNCH();
+            ctx->prof.end(stream, ev);
+            SIEB_TRY_CUDA(cudaGetLastError());
+            return SIEB200_OK;
+        };
+        SIEB_RETURN_IF(diag_blk(0, -1, -1, stream));
+        SIEB_RETURN_IF(group_panels(0));
+        bool forked = false;
+        for (int64_t bk = 0; bk < nbl; ++bk) {
+            const int64_t k0 = bk * NB;
+            const int64_t s0 = k0 + NB;
+            if (s0 >= np) break;
+            const int64_t m = np - s0, n1 = std::min<int64_t>(NB, m);
+            const int i = (int)(bk % kGroup);
+            const int64_t g0 = k0 - (int64_t)i * NB;
+            const bool last = i == kGroup - 1;
+            SIEB_TRY_CUDA(cudaEventRecord(st->ev_cols, stream));
+            SIEB_TRY_CUDA(cudaStreamWaitEvent(st->side, st->ev_cols, 0));
+            forked = true;
+            SIEB_RETURN_IF(diag_blk(bk + 1, k0, -1, st->side));
+            SIEB_TRY_CUDA(cudaEventRecord(st->ev_diag, st->side));
+            // The next group's first diagonal block takes this step's update
+            // here, off the chain (the group's GEMM leaves that block out).
+            const int64_t gn = g0 + kGroup * NB;
+            if (!last && gn < np) {
+                diag_update_kernel<float2><<<dim3(NB / 16, NB / 16), 256, 0, st->side>>>(
+                    st->W, ldw, gn, (int)std::min<int64_t>(NB, np - gn), k0, -1);
+                SIEB_NOTE_LAUNCH();
+                SIEB_TRY_CUDA(cudaGetLastError());
+            }
+            if (m > n1) {
+                const int64_t w = last ? m : std::min<int64_t>(m, (int64_t)(kGroup - 1 - i) * NB);
+                const int kx = last ? 0 : i * 2 * NB, K = last ? LO : 2 * NB;
+                const double elems = 2.0 * ((double)m * w + (double)w * (m - w)) - 128.0 * n1;
+                cudaEvent_t ev;
+                ctx->prof.begin(stream, 0, 2.0 * elems * 3.0 * K, 8.0 * elems + 4.0 * (3.0 * m) * K, &ev);
+                SIEB_RETURN_IF(gemm_half_sub(st->gemm, stream, reinterpret_cast<float*>(st->W + s0 + s0 * ldw),
+                                             2 * ldw, Ah + 2 * (s0 - g0) * LD, Bh + (s0 - g0) * LD, LD, 2 * m, m, w,
+                                             kx, LO + kx, K, wmax, gemm_ctas, n1));
+                ctx->prof.end(stream, ev);
+            }
+            SIEB_TRY_CUDA(cudaStreamWaitEvent(stream, st->ev_diag, 0));
+            SIEB_RETURN_IF(group_panels(bk + 1));
+        }
+        if (forked) {
+            SIEB_TRY_CUDA(cudaEventRecord(st->ev_pan, st->side));
+            SIEB_TRY_CUDA(cudaStreamWaitEvent(stream, st->ev_pan, 0));
+        }
+        ctx->prof.end(stream, ev_fact);
+        return SIEB200_OK;
+    }
 
     // Right-looking block LU with a lookahead of one block. Step bk: the
     // panels of block bk are formed on the context stream; the next
@@ -3015,7 +3184,7 @@ static int fp64_factorize(DenseSolver* s) {
     SIEB_NOTE_LAUNCH();
     const int64_t q = np / 4;
     rbt_matrix_kernel<double2><<<dim3(blocks_for(q, 128), (unsigned)q), 128, 0, stream>>>(
-        reinterpret_cast<const cplx*>(s->A), s->lda, n, np, st->diag, st->diag + 4 * np, st->W64, ldw);
+        reinterpret_cast<const cplx*>(s->A), s->lda, n, np, st->diag, st->diag + 4 * np, st->W64, ldw, nullptr);
     SIEB_NOTE_LAUNCH();
     SIEB_TRY_CUDA(cudaGetLastError());
     auto diag_blk = [&](int64_t bk, int64_t kp, cudaStream_t sm) -> int {

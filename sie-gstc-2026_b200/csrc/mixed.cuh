@@ -29,6 +29,7 @@ struct MixedState {
     unsigned* tri_flags = nullptr;   // per block progress flags (2 * nbl) + 2 tickets
     cplx* vecs = nullptr;       // FP64 work vectors
     int use_tc = 1;
+    int blocked = 0;            // grouped block steps with FP16 split packs (the default schedule)
     int hilo = 1;               // split [hi | lo] packs, three products per GEMM k-block
     int pair = 0;               // trailing update every second block step (K = 2 x 384)
     int pair_min = 0;           // pair schedule for steps whose paired GEMM is at least this wide
