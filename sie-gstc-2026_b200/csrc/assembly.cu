@@ -412,6 +412,7 @@ static RuleWeights make_rule_weights(const float* w, int Q) {
     return r;
 }
 constexpr int kFarWarps = 4;
+constexpr int kFarSmemMax = kTurnBytes + (int)sizeof(double) * 3 * kMaxQ * 32;
 
 // Far pairs (centroid distance at or above the extraction threshold): one
 // source face per lane group, 2^lg lanes sharing it (each takes every 2^lg-th
@@ -1514,7 +1515,9 @@ static int launch_far(const FarLaunch& f, bool big) {
     const int smem = (int)(sizeof(double2) * kTurn * kTurnCopies + sizeof(double) * 3 * (size_t)f.Q * nt);
     const dim3 grid((unsigned)((rows + chunk - 1) / chunk), (unsigned)((f.nf + nt - 1) / nt));
     auto* kernel = big ? far_pairs_kernel<NK, NT, ROT, true> : far_pairs_kernel<NK, NT, ROT, false>;
-    SIEB_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    // (the largest size any rule asks for: another thread may launch the same
+    // kernel with another one)
+    SIEB_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFarSmemMax));
     kernel<<<grid, kFarWarps * 32, smem, f.st>>>(f.geom, f.qp, *f.rw, f.Q, f.nf, f.m0, f.m1, make_wave(f.k0),
                                                  make_wave(f.k1), f.thr, f.exact, f.form_a ? 1 : 0, lg, chunk, f.out);
     SIEB_NOTE_LAUNCH();
