@@ -484,12 +484,16 @@ gemm_tf32_sub_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const _
 
 // ------------------------------------------------ scaled FP16 split operands
 // The trailing updates of the blocked schedule (mixed.cu):
-//   C -= (A_hi B_hi^T + 2^-11 (A_hi B_lo^T + A_lo B_hi^T)) / s
-// with sA A = A_hi + 2^-11 A_lo and sB B = B_hi + 2^-11 B_lo in FP16 (s = sA sB,
-// powers of two): 11 + 11 significant bits, as many as the TF32 split, at twice
-// the tensor rate and half the operand bytes. lo is kept 2^11 up, so that it has
-// hi's exponent range; the two mixed products share one accumulator, hi.hi has
-// the other, and the epilogue joins them.
+//   C -= sum over the steps of fa (A_hi B_hi^T + 2^-11 (A_hi B_lo^T + A_lo B_hi^T)) fb
+// with A / fa = A_hi + 2^-11 A_lo and B / fb = B_hi + 2^-11 B_lo in FP16: 11 + 11
+// significant bits, as many as the TF32 split, at twice the tensor rate and half
+// the operand bytes. fa and fb are powers of two per row, column and block
+// step (128 columns of K) that bring the row's or column's largest entry up to
+// FP16's range, and lo is kept 2^11 up, so that it has hi's exponent range: entries down
+// to 2^-28 of the largest keep all 22 bits. (One scale for a whole operand did not
+// do: on the 20,880-unknown omega spindle entries of L21 beyond 1023 stand beside rows
+// whose lo parts were lost, 17 refinement iterations instead of 15.) The two mixed
+// products share one accumulator, hi.hi has the other, and the epilogue joins them.
 // The tensor core's own accumulation truncates, so a sum over all of K = 512
 // loses more than the single-step schedule's sums over 128 did. The epilogue
 // warps therefore take the accumulator over after every 128 columns of K
@@ -520,7 +524,31 @@ static_assert(H_SMEM_BYTES <= 227 * 1024, "shared memory of the FP16 split GEMM"
 
 struct HalfTiles {
     int mt, r2, w, N, shift0, tiles1, tiles;
+    int rows;  // complex rows (M2 / 2)
 };
+
+// 16 accumulator columns of this warp's rows; the values are defined once
+// tmem_wait16 on the same registers has returned.
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_wait16(uint32_t (&r)[16], uint32_t (&s)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]),
+                   "+r"(r[15])
+                 :
+                 : "memory");
+    asm volatile(""
+                 : "+r"(s[0]), "+r"(s[1]), "+r"(s[2]), "+r"(s[3]), "+r"(s[4]), "+r"(s[5]), "+r"(s[6]), "+r"(s[7]),
+                   "+r"(s[8]), "+r"(s[9]), "+r"(s[10]), "+r"(s[11]), "+r"(s[12]), "+r"(s[13]), "+r"(s[14]),
+                   "+r"(s[15]));
+}
 
 // D f32, A and B f16, both K-major.
 constexpr uint32_t idesc_f16(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BM >> 4) << 24); }
@@ -537,7 +565,7 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64
 __global__ void __launch_bounds__(P_THREADS, 1)
 gemm_f16_sub_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ CUtensorMap tmC, const HalfTiles tl, int k0, int klo, int kblocks,
-                    const unsigned* __restrict__ scale_bits, unsigned* err) {
+                    const float* __restrict__ fa, const float* __restrict__ fb, int64_t fstride, unsigned* err) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
@@ -648,7 +676,6 @@ gemm_f16_sub_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         const int q = warp & 3;            // TMEM lane quarter of this warp
         const int row = q * 32 + lane;     // row of the tile
         const bool e0 = threadIdx.x == 64;
-        const float inv = 1.0f / (kHalfScaleA * half_scale(*scale_bits));
         const int chunks = (kblocks + H_CHUNK - 1) / H_CHUNK;
         int li = 0;
         for (int t = from(blockIdx.x, rt, col, lim); t < tl.tiles; t = from(t + gridDim.x, rt, col, lim)) {
@@ -659,19 +686,38 @@ gemm_f16_sub_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 #pragma unroll 1
             for (int ch = 0; ch < chunks && got; ++ch, ++li) {
                 const int b = li & 1;
+                // (rows past the last are not stored)
+                const float rowf = fa[ch * fstride + min((rt * BM + row) >> 1, tl.rows - 1)];
+                const float* colf = fb + ch * fstride + col;
                 if (lane == 0) got = mbar_wait(accf0 + 8 * b, (uint32_t)(li >> 1) & 1u, err) ? 1 : 0;
                 got = __shfl_sync(0xffffffffu, got, 0);
                 __syncwarp();
                 if (!got) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * 2 * BN);
+                // 16 columns at a time, the next ones' loads in flight meanwhile
+                uint32_t v[2][16], w[2][16];
+                tmem_ld16(ta, v[0]);
+                tmem_ld16(ta + BN, w[0]);
 #pragma unroll
-                for (int c = 0; c < BN / 32; ++c) {
-                    float v[32], w[32];
-                    tmem_ld32(ta + c * 32, v);
-                    tmem_ld32(ta + BN + c * 32, w);
+                for (int c = 0; c < BN / 16; ++c) {
+                    uint32_t(&vc)[16] = v[c & 1];
+                    uint32_t(&wc)[16] = w[c & 1];
+                    tmem_wait16(vc, wc);
+                    if (c + 1 < BN / 16) {
+                        tmem_ld16(ta + (c + 1) * 16, v[(c + 1) & 1]);
+                        tmem_ld16(ta + BN + (c + 1) * 16, w[(c + 1) & 1]);
+                    }
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) sum[c * 32 + j] += fmaf(w[j], 0x1p-11f, v[j]);
+                    for (int j = 0; j < 16; j += 4) {
+                        const float4 f = __ldg(reinterpret_cast<const float4*>(colf + c * 16 + j));
+                        const float fj[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            sum[c * 16 + j + i] =
+                                fmaf(fmaf(__uint_as_float(wc[j + i]), 0x1p-11f, __uint_as_float(vc[j + i])),
+                                     rowf * fj[i], sum[c * 16 + j + i]);
+                    }
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
@@ -683,7 +729,7 @@ gemm_f16_sub_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 if (c >= slots) break;
                 float* cc = cs + (c & 1) * (BM * H_CC);
 #pragma unroll
-                for (int j = 0; j < H_CC; ++j) cc[j * BM + row] = -sum[c * H_CC + j] * inv;
+                for (int j = 0; j < H_CC; ++j) cc[j * BM + row] = -sum[c * H_CC + j];
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 epilogue_bar();
                 if (e0) {
@@ -916,14 +962,15 @@ int gemm_tc_sub(GemmTC* g, cudaStream_t stream, float* C, int64_t ldc, const flo
 }
 
 int gemm_half_sub(GemmTC* g, cudaStream_t stream, float* C, int64_t ldc, const __half* A, const __half* B, int64_t ld,
-                  int64_t M2, int64_t N, int64_t w, int k0, int klo, int K, const unsigned* scale_bits, int max_ctas,
-                  int64_t shift0) {
+                  int64_t M2, int64_t N, int64_t w, int k0, int klo, int K, const float* fa, const float* fb,
+                  int64_t fstride, int max_ctas, int64_t shift0) {
     SIEB_CHECK(K > 0 && K % H_BK == 0 && k0 >= 0 && k0 % H_BK == 0 && klo % H_BK == 0 && klo + K <= ld && ld % 8 == 0,
                SIEB200_INVALID_ARG, "FP16 split GEMM: K offsets must be multiples of 64 inside the packs");
     SIEB_CHECK(M2 > 0 && N > 0 && M2 < (1ll << 31) && N < (1ll << 31) && w > 0 && w <= N && (w == N || w % 64 == 0),
                SIEB200_INVALID_ARG, "GEMM size out of range");
     SIEB_CHECK(shift0 >= 0 && shift0 < N, SIEB200_INVALID_ARG, "GEMM first-row-tile column shift out of range");
-    SIEB_CHECK(((uintptr_t)A % 16) == 0 && ((uintptr_t)B % 16) == 0 && ((uintptr_t)C % 16) == 0 && (ldc * 4) % 16 == 0,
+    SIEB_CHECK(((uintptr_t)A % 16) == 0 && ((uintptr_t)B % 16) == 0 && ((uintptr_t)C % 16) == 0 && (ldc * 4) % 16 == 0 &&
+                   ((uintptr_t)fb % 16) == 0 && fstride % 4 == 0 && w % 4 == 0 && shift0 % 4 == 0,
                SIEB200_INVALID_ARG, "GEMM operands must be 16-byte aligned");
     CUtensorMap ma, mb, mc;
     for (int i = 0; i < 2; ++i)
@@ -934,6 +981,7 @@ int gemm_half_sub(GemmTC* g, cudaStream_t stream, float* C, int64_t ldc, const _
                                         (uint64_t)ldc * sizeof(float), BM, H_CC, CU_TENSOR_MAP_SWIZZLE_NONE));
     HalfTiles tl;
     tl.mt = (int)((M2 + BM - 1) / BM);
+    tl.rows = (int)(M2 / 2);
     tl.w = (int)w;
     tl.N = (int)N;
     tl.shift0 = (int)shift0;
@@ -947,8 +995,8 @@ int gemm_half_sub(GemmTC* g, cudaStream_t stream, float* C, int64_t ldc, const _
                                            H_SMEM_BYTES));
         g->attr_set_h = true;
     }
-    gemm_f16_sub_kernel<<<grid, P_THREADS, H_SMEM_BYTES, stream>>>(ma, mb, mc, tl, k0, klo, K / H_BK, scale_bits,
-                                                                   g->err);
+    gemm_f16_sub_kernel<<<grid, P_THREADS, H_SMEM_BYTES, stream>>>(ma, mb, mc, tl, k0, klo, K / H_BK, fa, fb,
+                                                                   fstride, g->err);
     SIEB_NOTE_LAUNCH();
     SIEB_TRY_CUDA(cudaGetLastError());
     return SIEB200_OK;

@@ -31,33 +31,24 @@ int gemm_tc_check(GemmTC* g, cudaStream_t stream);
 // Whether the default kernel configuration is selected (no switch).
 bool gemm_tc_default(const GemmTC* g);
 
-// Scales of the FP16 split operands. B: the power of two that brings a largest
-// magnitude (its float bits) into [2^8, 2^9), the largest entry of the matrix
-// before the factorization (U12 may grow 128-fold before it leaves FP16's
-// range); A = L21, whose entries are relative to the pivots, 2^6 (up to 1023). Both
-// as high as the growth allows: entries below 2^-14 of a scaled value lose bits
-// of lo (with scales of 1 the 20,880-unknown omega spindle took 17 refinement
-// iterations instead of 15).
-constexpr float kHalfScaleA = 64.f;
-__host__ __device__ inline float half_scale(unsigned max_bits) {
-    const unsigned e = max_bits >> 23;
-    const unsigned b = (e >= 16 && e <= 253 ? 262u - e : 127u) << 23;
-#ifdef __CUDA_ARCH__
-    return __uint_as_float(b);
-#else
-    union { unsigned u; float f; } v;
-    v.u = b;
-    return v.f;
-#endif
+// Scale of a row of L21 or a column of U12 in the FP16 split operands: the power of
+// two that brings its largest magnitude (float bits) into [2^14, 2^15), one per
+// block step. Returns its exponent; 0 for a row of zeros or of non-finite values.
+__host__ __device__ inline int half_exponent(unsigned max_bits) {
+    const int e = (int)(max_bits >> 23) - 127;
+    return max_bits == 0u || e > 127 ? 0 : (14 - e > 120 ? 120 : 14 - e);
 }
 // The same update from scaled FP16 split packs (rows of ld FP16 values, hi
-// columns from k0, lo columns from klo, K of each; lo kept 2^11 up, A times
-// kHalfScaleA, B times half_scale(*scale_bits)): all rows of the first w columns and the first 2 w rows of the
-// others (w = N: all of C; w a multiple of 64 otherwise), the first 128 rows from
-// column shift0 on.
+// columns from k0, lo columns from klo, K of each; lo kept 2^11 up; per 128 columns of
+// K, one block step, a row of A is 1 / fa and a column of B 1 / fb times its value:
+// fa and fb hold a float per complex row and column and step, fstride apart, the first
+// step of this call first): all rows of the first w columns and the first 2 w rows of
+// the others (w = N: all of C; w a multiple of 64 otherwise), the first 128 rows from
+// column shift0 on. fb may be read up to 128 entries past N.
 int gemm_half_sub(GemmTC* g, cudaStream_t stream, float* C, int64_t ldc, const __half* A, const __half* B, int64_t ld,
-                  int64_t M2, int64_t N, int64_t w, int k0, int klo, int K, const unsigned* scale_bits, int max_ctas,
-                  int64_t shift0);
+                  int64_t M2, int64_t N, int64_t w, int k0, int klo, int K, const float* fa, const float* fb,
+                  int64_t fstride, int max_ctas, int64_t shift0);
+
 // Selects the implementation: 3 = persistent tcgen05 kernel whose epilogue
 // adds -acc to C by TMA reduction (default), 2 = persistent kernel that
 // loads, subtracts and stores the C tile by TMA, 1 = one CTA per tile

@@ -104,12 +104,11 @@ __global__ void rbt_init_kernel(double* diag, int64_t np, uint64_t seed) {
     diag[i] = rbt_value(seed, i);
 }
 
-// W = U^T A_pad V, read A (c128, n x n, lda) once, write W (c64); wmax (optional)
-// receives the bits of W's largest component.
+// W = U^T A_pad V, read A (c128, n x n, lda) once, write W (c64).
 template <class T>
 __global__ void rbt_matrix_kernel(const cplx* __restrict__ A, int64_t lda, int64_t n, int64_t np,
                                   const double* __restrict__ du, const double* __restrict__ dv,
-                                  T* __restrict__ W, int64_t ldw, unsigned* __restrict__ wmax) {
+                                  T* __restrict__ W, int64_t ldw) {
     const int64_t q = np / 4;
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t j = blockIdx.y;
@@ -148,16 +147,6 @@ __global__ void rbt_matrix_kernel(const cplx* __restrict__ A, int64_t lda, int64
 #pragma unroll
         for (int s = 0; s < 4; ++s)
             W[(i + s * q) + (j + t * q) * ldw] = T{(decltype(T::x))blk[s][t].re, (decltype(T::x))blk[s][t].im};
-    if (wmax) {  // largest component of W, as float bits (ordered like the values)
-        float mx = 0.f;
-#pragma unroll
-        for (int t = 0; t < 4; ++t)
-#pragma unroll
-            for (int s = 0; s < 4; ++s)
-                mx = fmaxf(mx, fmaxf(fabsf((float)blk[s][t].re), fabsf((float)blk[s][t].im)));
-        const unsigned m = __reduce_max_sync(__activemask(), __float_as_uint(mx));
-        if (m > *reinterpret_cast<volatile unsigned*>(wmax)) atomicMax(wmax, m);
-    }
 }
 
 // y = U^T x_pad (vector); x has n entries (rest treated as 0).
@@ -816,24 +805,47 @@ struct PanelArgs {
     int64_t b_ld = 0, b_c0 = 0;
     int64_t a_lo = 0, b_lo = 0;
     int lo_rn = 0;  // lo parts rounded to the nearest TF32
-    // pack 2: scaled FP16 split instead, strides and offsets in FP16 values
-    // (lo kept 2^11 up, L21 times kHalfScaleA, U12 times half_scale(*wmax); a
-    // value outside FP16's range sets the error word to 4)
+    // pack 2: scaled FP16 split instead, strides and offsets in FP16 values (lo
+    // kept 2^11 up); the scale of each row of L21 and column of U12 goes to fa and fb
+    // as its reciprocal
     __half* Ah = nullptr;
     __half* Bh = nullptr;
-    const unsigned* wmax = nullptr;
-    unsigned* err = nullptr;
+    float* fa = nullptr;
+    float* fb = nullptr;
     // CTA range of one launch: L21 row blocks and U12 column blocks
     // [b_first, b_first + nl_run) of 32 each (nl_run 0: all nL from 0)
     int b_first = 0, nl_run = 0;
 };
 
+__device__ __forceinline__ float pow2f(int e) { return __int_as_float((e + 127) << 23); }  // |e| <= 126
+
 // v = h + 2^-11 l in FP16, both rounded to nearest.
-__device__ __forceinline__ void split_half(float2 v, __half2& h, __half2& l, unsigned* err) {
-    if (!(fmaxf(fabsf(v.x), fabsf(v.y)) <= 65504.f)) atomicCAS(err, 0u, 4u);
+__device__ __forceinline__ void split_half(float2 v, __half2& h, __half2& l) {
     h = __floats2half2_rn(v.x, v.y);
     const float2 r = __half22float2(h);
     l = __floats2half2_rn((v.x - r.x) * 2048.f, (v.y - r.y) * 2048.f);
+}
+
+// FP16 scale exponents of the 32 lines (rows of L21, columns of U12) a panels CTA holds in
+// shared memory, line i at lines[i][0 .. NB): eight lanes per line, result in ex[32]; f
+// receives the reciprocals of the `count` first.
+template <class L>
+__device__ __forceinline__ void line_exponents(const L& lines, int* ex, float* f, int64_t count) {
+    const int line = threadIdx.x >> 3, part = threadIdx.x & 7;
+    float mx = 0.f;
+#pragma unroll
+    for (int c = 0; c < NB / 8; ++c) {
+        const float2 v = lines[line][part + 8 * c];
+        mx = fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.y)));
+    }
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if (part == 0) {
+        const int e = half_exponent(__float_as_uint(mx));
+        ex[line] = e;
+        if (line < count) f[line] = pow2f(-e);
+    }
+    __syncthreads();
 }
 
 // L21 = A21 * inv(U11) for rows [s0, np) of the panel columns [k0, k0+kb);
@@ -977,13 +989,16 @@ __device__ __forceinline__ void panel_L_body(T* __restrict__ W, int64_t ldw, con
     if (!pa.pack) return;
     if constexpr (std::is_same<T, float2>::value) {
         if (pa.pack == 2) {
+            __shared__ int ex[32];
+            line_exponents(Ar, ex, pa.fa + (rb - pa.a_r0), np - rb);
             for (int e = tid; e < 32 * NB; e += blockDim.x) {
                 const int rr = e / NB, c = e % NB;
                 const int64_t gr = rb + rr;
                 if (gr >= np) continue;
                 const float2 v = Ar[rr][c];
+                const float sc = pow2f(ex[rr]);
                 __half2 h, l;
-                split_half(make_float2(v.x * kHalfScaleA, v.y * kHalfScaleA), h, l, pa.err);
+                split_half(make_float2(v.x * sc, v.y * sc), h, l);
                 __half2* row0 = reinterpret_cast<__half2*>(pa.Ah + 2 * (gr - pa.a_r0) * pa.a_ld) + c;
                 __half2* row1 = reinterpret_cast<__half2*>(pa.Ah + (2 * (gr - pa.a_r0) + 1) * pa.a_ld) + c;
                 const int64_t lo = pa.a_lo / 2;
@@ -1141,7 +1156,10 @@ __device__ __forceinline__ void panel_U_body(T* __restrict__ W, int64_t ldw, con
 #pragma unroll
         for (int j = 0; j < 2; ++j) Ac[2 * tx + j][row[i]] = acc[i][j];
     __syncthreads();
-    const float bscale = pa.pack == 2 ? half_scale(*pa.wmax) : 1.f;
+    __shared__ int ex[32];
+    if constexpr (std::is_same<T, float2>::value) {
+        if (pa.pack == 2) line_exponents(Ac, ex, pa.fb + (cb - pa.b_c0), np - cb);
+    }
     for (int e = tid; e < 32 * NB; e += blockDim.x) {
         const int r = e % NB, c = e / NB;
         const int64_t gc = cb + c;
@@ -1150,8 +1168,9 @@ __device__ __forceinline__ void panel_U_body(T* __restrict__ W, int64_t ldw, con
         if (r < kb) W[(k0 + r) + gc * ldw] = v;
         if constexpr (std::is_same<T, float2>::value) {
             if (pa.pack == 2) {
+                const float sc = pow2f(ex[c]);
                 __half2 h, l;
-                split_half(make_float2(v.x * bscale, v.y * bscale), h, l, pa.err);
+                split_half(make_float2(v.x * sc, v.y * sc), h, l);
                 __half2* col = reinterpret_cast<__half2*>(pa.Bh + (gc - pa.b_c0) * pa.b_ld) + r;
                 col[0] = h;
                 col[pa.b_lo / 2] = l;
@@ -2125,17 +2144,11 @@ void mixed_release(DenseSolver* s) {
     s->krylov.release(); s->vec.release(); s->flags.release(); s->gemv_scratch.release(); s->couple.release();
 }
 
-// *overflow (optional) receives whether the FP16 packs overflowed, which is
-// then not an error.
-static int check_err(DenseSolver* s, const char* what, bool* overflow = nullptr) {
+static int check_err(DenseSolver* s, const char* what) {
     MixedState* st = state_of(s);
     unsigned e = 0;
     SIEB_TRY_CUDA(cudaMemcpyAsync(&e, st->err, sizeof(unsigned), cudaMemcpyDeviceToHost, s->ctx->stream));
     SIEB_TRY_CUDA(cudaStreamSynchronize(s->ctx->stream));
-    if (overflow) {
-        *overflow = e == 4u;
-        if (e == 4u) return SIEB200_OK;
-    }
     if (e == 1u) {
         set_error(std::string(what) + ": zero or non-finite pivot in the unpivoted LU of the randomized matrix");
         return SIEB200_SINGULAR;
@@ -2243,7 +2256,9 @@ int mixed_factorize(DenseSolver* s) {
     const size_t bApack = ((sizeof(float) * 2 * np * K3 + 255) / 256) * 256;
     SIEB_RETURN_IF(s->gemm_a.reserve(2 * bApack));
     // two step buffers (single-step schedule) or the pair schedule's K = 2 x 384
-    SIEB_RETURN_IF(s->gemm_b.reserve(sizeof(float) * np * 2 * K3));
+    // (or a group's B pack and the scales of its rows and columns)
+    SIEB_RETURN_IF(s->gemm_b.reserve(std::max(sizeof(float) * np * 2 * K3,
+                                              (size_t)np * 8 * kGroup * NB + sizeof(float) * 2 * kGroup * (np + 128))));
     st->Apack[0] = s->gemm_a.as<float>();
     st->Apack[1] = reinterpret_cast<float*>(s->gemm_a.as<char>() + bApack);
     st->Bpack = s->gemm_b.as<float>();
@@ -2295,24 +2310,13 @@ int mixed_factorize(DenseSolver* s) {
     key.head = ((int64_t)st->head_max << 20) | (int64_t)st->head_smem;
     const char* no_graphs = getenv("SIEB200_NO_GRAPHS");
     const bool graphs = !ctx->prof.enabled && !(no_graphs && no_graphs[0] == '1');
-    // A value of L21 or U12 outside FP16's range (element growth far beyond
-    // what the butterfly transform leaves in practice): factor again with the
-    // FP32 operands of the single-step schedule.
-    auto finish = [&]() -> int {
-        bool overflow = false;
-        SIEB_RETURN_IF(check_err(s, "mixed LU factorization", &overflow));
-        if (!overflow) return SIEB200_OK;
-        st->blocked = 0;
-        SIEB_RETURN_IF(mixed_enqueue(s, st, bFlags, K3));
-        return check_err(s, "mixed LU factorization");
-    };
     if (graphs) {
         for (auto& g : st->graphs) {
             if (g.exec && g.key == key) {
                 g.used = ++st->tick;
                 SIEB_TRY_CUDA(cudaGraphLaunch(g.exec, stream));
                 note_launches(g.launches);
-                return finish();
+                return check_err(s, "mixed LU factorization");
             }
         }
     }
@@ -2347,7 +2351,7 @@ int mixed_factorize(DenseSolver* s) {
     } else {
         SIEB_RETURN_IF(mixed_enqueue(s, st, bFlags, K3));
     }
-    return finish();
+    return check_err(s, "mixed LU factorization");
 }
 
 // Enqueues one mixed factorization on the context stream and the lookahead
@@ -2364,7 +2368,7 @@ static int mixed_enqueue(DenseSolver* s, MixedState* st, size_t bFlags, int K3) 
     SIEB_TRY_CUDA(cudaGetLastError());
     const int64_t q = np / 4;
     rbt_matrix_kernel<float2><<<dim3(blocks_for(q, 128), (unsigned)q), 128, 0, stream>>>(
-        reinterpret_cast<const cplx*>(s->A), s->lda, n, np, st->diag, st->diag + 4 * np, st->W, ldw, st->err + 1);
+        reinterpret_cast<const cplx*>(s->A), s->lda, n, np, st->diag, st->diag + 4 * np, st->W, ldw);
     SIEB_NOTE_LAUNCH();
     SIEB_TRY_CUDA(cudaGetLastError());
 
@@ -2504,7 +2508,11 @@ static int mixed_enqueue(DenseSolver* s, MixedState* st, size_t bFlags, int K3) 
         __half* Bh = reinterpret_cast<__half*>(st->Bpack);
         const int LO = kGroup * 2 * NB;  // lo half of a pack row
         const int64_t LD = 2 * LO;       // FP16 values per pack row
-        const unsigned* wmax = st->err + 1;
+        // Per step of the group and row (column) from the group's first: the
+        // reciprocal scales, behind the B pack.
+        float* fa = st->Bpack + np * (LD / 2);
+        const int64_t fs = np + 128;
+        float* fb = fa + kGroup * fs;
         auto group_panels = [&](int64_t bk) -> int {
             const int64_t k0 = bk * NB;
             const int kb = (int)std::min<int64_t>(NB, np - k0);
@@ -2517,8 +2525,8 @@ static int mixed_enqueue(DenseSolver* s, MixedState* st, size_t bFlags, int K3) 
             pa.pack = 2;
             pa.Ah = Ah + (bk % kGroup) * 2 * NB; pa.a_ld = LD; pa.a_r0 = g0; pa.a_lo = LO;
             pa.Bh = Bh + (bk % kGroup) * 2 * NB; pa.b_ld = LD; pa.b_c0 = g0; pa.b_lo = LO;
-            pa.wmax = wmax;
-            pa.err = st->err;
+            pa.fa = fa + (bk % kGroup) * fs;
+            pa.fb = fb + (bk % kGroup) * fs;
             cudaEvent_t ev;
             ctx->prof.begin(stream, 4, 16.0 * NB * NB * (double)m, 32.0 * NB * (double)m, &ev);
             panels_kernel<float2><<<(unsigned)(2 * pa.nL), 256, kSmemPanel, stream>>>(
@@ -2561,7 +2569,8 @@ static int mixed_enqueue(DenseSolver* s, MixedState* st, size_t bFlags, int K3) 
                 ctx->prof.begin(stream, 0, 2.0 * elems * 3.0 * K, 8.0 * elems + 4.0 * (3.0 * m) * K, &ev);
                 SIEB_RETURN_IF(gemm_half_sub(st->gemm, stream, reinterpret_cast<float*>(st->W + s0 + s0 * ldw),
                                              2 * ldw, Ah + 2 * (s0 - g0) * LD, Bh + (s0 - g0) * LD, LD, 2 * m, m, w,
-                                             kx, LO + kx, K, wmax, gemm_ctas, n1));
+                                             kx, LO + kx, K, fa + (last ? 0 : i) * fs + (s0 - g0),
+                                             fb + (last ? 0 : i) * fs + (s0 - g0), fs, gemm_ctas, n1));
                 ctx->prof.end(stream, ev);
             }
             SIEB_TRY_CUDA(cudaStreamWaitEvent(stream, st->ev_diag, 0));
@@ -3184,7 +3193,7 @@ static int fp64_factorize(DenseSolver* s) {
     SIEB_NOTE_LAUNCH();
     const int64_t q = np / 4;
     rbt_matrix_kernel<double2><<<dim3(blocks_for(q, 128), (unsigned)q), 128, 0, stream>>>(
-        reinterpret_cast<const cplx*>(s->A), s->lda, n, np, st->diag, st->diag + 4 * np, st->W64, ldw, nullptr);
+        reinterpret_cast<const cplx*>(s->A), s->lda, n, np, st->diag, st->diag + 4 * np, st->W64, ldw);
     SIEB_NOTE_LAUNCH();
     SIEB_TRY_CUDA(cudaGetLastError());
     auto diag_blk = [&](int64_t bk, int64_t kp, cudaStream_t sm) -> int {

@@ -1,5 +1,5 @@
 """The blocked schedule of the mixed LU (groups of four block steps, FP16
-split packs) at the edges of its groups, and its return to FP32 operands."""
+split packs) at the edges of its groups, and entries far apart in size."""
 
 import math
 
@@ -65,9 +65,8 @@ def _butterfly(n, offset):
 
 @pytest.mark.parametrize("entry", [500.0, 2000.0])
 def test_packs_out_of_fp16_range(entry, gpu_ctx):
-    """A transformed matrix whose L21 holds one large entry, inside the FP16
-    packs' range (1023) and past it, where the factorization repeats with FP32
-    operands: refined to 1e-10 alike."""
+    """A transformed matrix whose L21 holds one entry far above its neighbours in
+    the row: refined to 1e-10 alike."""
     n = 192
     rng = np.random.default_rng(5)
     W = np.eye(n) + 0.01 * (rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)))
