@@ -115,11 +115,56 @@ void Profiler::collect() {
     cudaGetLastError();
 }
 
+// The stream-ordered pool of the current device (null where the device has
+// none); made on first use, one per device and process.
+static cudaMemPool_t device_pool() {
+    static std::mutex mu;
+    static cudaMemPool_t pools[64] = {};
+    static bool tried[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    std::lock_guard<std::mutex> lock(mu);
+    if (!tried[dev]) {
+        tried[dev] = true;
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        uint64_t keep = kPoolKeepBytes;
+        if (cudaMemPoolCreate(&pools[dev], &props) != cudaSuccess ||
+            cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+            cudaGetLastError();
+            pools[dev] = nullptr;
+        }
+    }
+    return pools[dev];
+}
+
+void trim_pool() {
+    if (cudaMemPool_t p = device_pool()) cudaMemPoolTrimTo(p, 0);
+    cudaGetLastError();
+}
+
 int DeviceBuffer::reserve(size_t n) {
     if (n <= bytes && ptr) return SIEB200_OK;
     release();
     if (n == 0) n = 16;
-    cudaError_t e = cudaMalloc(&ptr, n);
+    cudaMemPool_t pool = order && n <= kPoolMaxBytes ? device_pool() : nullptr;
+    cudaError_t e = cudaErrorMemoryAllocation;
+    if (pool) {
+        e = cudaMallocFromPoolAsync(&ptr, n, pool, order);
+        pooled = e == cudaSuccess;
+        if (!pooled) cudaGetLastError();
+    }
+    if (e != cudaSuccess) e = cudaMalloc(&ptr, n);
+    if (e == cudaErrorMemoryAllocation) {  // once more without what the pool keeps
+        cudaGetLastError();
+        trim_pool();
+        e = cudaMalloc(&ptr, n);
+    }
     if (e != cudaSuccess) {
         ptr = nullptr;
         bytes = 0;
@@ -133,9 +178,11 @@ int DeviceBuffer::reserve(size_t n) {
 }
 
 void DeviceBuffer::release() {
-    if (ptr) cudaFree(ptr);
+    if (ptr && pooled) cudaFreeAsync(ptr, order);
+    else if (ptr) cudaFree(ptr);
     ptr = nullptr;
     bytes = 0;
+    pooled = false;
 }
 
 // Gauss-Legendre rule with n points on [0, 1], nodes ascending, rounded to
@@ -361,7 +408,7 @@ int solve_dense_common(sieb200_ctx* ctx, const sieb200_mesh* mesh, const sieb200
     SIEB_CHECK(method >= 0 && method <= 3, SIEB200_INVALID_ARG, "unsupported solver method");
     cudaStream_t st = ctx->stream;
 
-    DeviceBuffer Zb, Zcopy, Bb, Srcb, Xb, Rb;
+    DeviceBuffer Zb(st), Zcopy(st), Bb(st), Srcb(st), Rb(st);
     SIEB_RETURN_IF(Zb.reserve(sizeof(cplx) * N * N));
     const auto t_asm = Clock::now();
     SIEB_RETURN_IF(assemble_device(ctx, *mesh, *o, tensors, Zb.as<cplx>(), N));
@@ -391,7 +438,7 @@ int solve_dense_common(sieb200_ctx* ctx, const sieb200_mesh* mesh, const sieb200
         SIEB_TRY_CUDA(cudaMemcpyAsync(Zcopy.ptr, Zb.ptr, sizeof(cplx) * N * N, cudaMemcpyDeviceToDevice, st));
     }
     DenseSolver solver;
-    solver.ctx = ctx;
+    solver.bind(ctx);
     solver.n = N;
     solver.method = method;
     SIEB_TRY_CUDA(cudaStreamSynchronize(st));
@@ -417,7 +464,7 @@ int solve_dense_common(sieb200_ctx* ctx, const sieb200_mesh* mesh, const sieb200
     if (o->compute_residual) {
         const auto t_res = Clock::now();
         const double* Zr = in_place ? Zcopy.as<double>() : Zb.as<double>();
-        DeviceBuffer scratch;
+        DeviceBuffer scratch(st);
         std::vector<double> hr(2 * N);
         if (ncols >= 2) {
             // every column at once: R = B - Z X (one FP64 complex GEMM)
@@ -521,7 +568,7 @@ int lane_solve(sieb200_ctx* ctx, DenseSolver& solver, LaneBuffers& lb, const sie
         SIEB_RETURN_IF(lb.R.reserve(sizeof(cplx) * N * N + sizeof(cplx) * N));
         SIEB_TRY_CUDA(cudaMemcpyAsync(lb.R.ptr, lb.Z.ptr, sizeof(cplx) * N * N, cudaMemcpyDeviceToDevice, st));
     }
-    solver.ctx = ctx;
+    solver.bind(ctx);
     solver.n = N;
     solver.method = o->solver;
     solver.sm_cap = sm_cap;
@@ -621,8 +668,11 @@ int sieb200_ctx_destroy(sieb200_ctx* ctx) {
     ctx->pairs.release(); ctx->near_list.release(); ctx->counter.release(); ctx->inc.release();
     ctx->mass.release(); ctx->zbuf.release(); ctx->rhsbuf.release(); ctx->srcbuf.release();
     ctx->tens.release();
+    if (ctx->side) cudaStreamDestroy(ctx->side);
+    if (ctx->side2) cudaStreamDestroy(ctx->side2);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
+    trim_pool();
     return SIEB200_OK;
 }
 
@@ -849,7 +899,7 @@ int sieb200_matvec_matrix_free(sieb200_ctx* ctx, const sieb200_mesh* mesh, const
         SIEB_TRY_CUDA(cudaStreamSynchronize(ctx->stream));
         return SIEB200_OK;
     }
-    DeviceBuffer tmp;
+    DeviceBuffer tmp(ctx->stream);
     SIEB_RETURN_IF(tmp.reserve(sizeof(cplx) * 2 * N));
     cplx* dx = tmp.as<cplx>();
     cplx* dy = dx + N;
@@ -875,7 +925,7 @@ int sieb200_gstc_tensor_gradient(sieb200_ctx* ctx, const sieb200_mesh* mesh, con
         SIEB_TRY_CUDA(cudaStreamSynchronize(ctx->stream));
         return SIEB200_OK;
     }
-    DeviceBuffer tmp;
+    DeviceBuffer tmp(ctx->stream);
     SIEB_RETURN_IF(tmp.reserve(sizeof(cplx) * (2 * N + ns)));
     cplx* dl = tmp.as<cplx>();
     cplx* dx = dl + N;
@@ -899,7 +949,7 @@ int sieb200_assemble_rhs(sieb200_ctx* ctx, const sieb200_mesh* mesh, const sieb2
         SIEB_TRY_CUDA(cudaStreamSynchronize(ctx->stream));
         return SIEB200_OK;
     }
-    DeviceBuffer tmp;
+    DeviceBuffer tmp(ctx->stream);
     SIEB_RETURN_IF(tmp.reserve(sizeof(cplx) * N * num_sources));
     SIEB_RETURN_IF(assemble_rhs_device(ctx, *mesh, *opt, sources, num_sources, tmp.as<cplx>(), N));
     SIEB_TRY_CUDA(cudaMemcpyAsync(B, tmp.ptr, sizeof(cplx) * N * num_sources, cudaMemcpyDeviceToHost, ctx->stream));
@@ -912,7 +962,7 @@ int sieb200_dense_solver_create(sieb200_ctx* ctx, int64_t n, int method, sieb200
     SIEB_CHECK(method >= 0 && method <= 3, SIEB200_INVALID_ARG, "unsupported dense solver method");
     SIEB_CHECK(n <= std::numeric_limits<int>::max(), SIEB200_OVERFLOW, "matrix dimension exceeds the int limit");
     sieb200_dense_solver* s = new sieb200_dense_solver();
-    s->impl.ctx = ctx;
+    s->impl.bind(ctx);
     s->impl.n = n;
     s->impl.method = method;
     *out = s;
@@ -952,7 +1002,7 @@ int sieb200_matvec(sieb200_ctx* ctx, int64_t n, const void* A, int64_t lda, int 
     SIEB_CHECK(ctx && A && x && y && n > 0 && lda >= n && (prec == 0 || prec == 1),
                SIEB200_INVALID_ARG, "invalid matvec arguments");
     SIEB_TRY_CUDA(cudaSetDevice(ctx->device));
-    DeviceBuffer scratch;
+    DeviceBuffer scratch(ctx->stream);
     SIEB_RETURN_IF(gemv_device(ctx, n, A, lda, prec, reinterpret_cast<const cplx*>(x), beta,
                                reinterpret_cast<cplx*>(y), scratch));
     SIEB_TRY_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -1063,7 +1113,7 @@ int sieb200_gemm_tf32_sub_shifted(sieb200_ctx* ctx, int64_t m2, int64_t n, int k
                "invalid GEMM arguments");
     SIEB_TRY_CUDA(cudaSetDevice(ctx->device));
     GemmTC* g = nullptr;
-    SIEB_RETURN_IF(gemm_tc_create(&g));
+    SIEB_RETURN_IF(gemm_tc_create(&g, ctx->stream));
     gemm_tc_set_mode(g, mode >= 4 ? mode - 2 : mode);
     int st = gemm_tc_sub(g, ctx->stream, C, ldc, A, B, m2, n, k, 0, mode >= 4 ? 1 : 0, col_shift);
     if (st == SIEB200_OK) st = gemm_tc_check(g, ctx->stream);

@@ -1600,11 +1600,18 @@ static int assemble_or_apply(sieb200_ctx* ctx, const sieb200_mesh& mesh, const s
                    "Gauss-Legendre point count must be in [1, 20]");
         SIEB_TRY_CUDA(cudaMemcpyAsync(dgl, glt, sizeof(glt), cudaMemcpyHostToDevice, st));
     }
+    // (The free memory, whose query takes 0.1 to 11 ms, is asked for only where
+    // the workspace of earlier calls is too small.)
     const size_t pair_bytes = sizeof(cplx) * 9 * po.NB;
-    size_t budget = (size_t)8 << 30;
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) budget = std::min(budget, free_b / 3);
-    const int slab = (int)std::max<size_t>(1, std::min<size_t>(nf, budget / (pair_bytes * nf)));
+    const size_t most = (size_t)8 << 30;
+    auto slab_of = [&](size_t budget) {
+        return (int)std::max<size_t>(1, std::min<size_t>(nf, budget / (pair_bytes * nf)));
+    };
+    int slab = slab_of(most);
+    if (ctx->pairs.bytes < pair_bytes * (size_t)slab * nf) {
+        size_t free_b = 0, total_b = 0;
+        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) slab = slab_of(std::min(most, free_b / 3));
+    }
     SIEB_RETURN_IF(ctx->pairs.reserve(pair_bytes * (size_t)slab * nf));
     po.pairs = ctx->pairs.as<cplx>();
     SIEB_RETURN_IF(ctx->counter.reserve(sizeof(unsigned long long)));
@@ -2063,7 +2070,7 @@ int surface_fields_device(sieb200_ctx* ctx, const sieb200_mesh& mesh, const doub
     const int per_chunk = kFieldThreads * (int)((most + std::min<int64_t>(most, want) - 1) / std::min<int64_t>(most, want));
     const int chunks = (nf + per_chunk - 1) / per_chunk;
     const int ld = ((nf + 31) / 32) * 32;
-    DeviceBuffer buf;
+    DeviceBuffer buf(st);
     const size_t b_obs = sizeof(d3) * (size_t)nobs, b_cur = sizeof(cplx) * (size_t)ne;
     const size_t b_out = sizeof(cplx) * 3 * (size_t)nobs;
     const size_t b_fs = sizeof(double) * (size_t)(kFieldRows + 3 * Q) * ld;

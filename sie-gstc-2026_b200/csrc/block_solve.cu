@@ -631,7 +631,10 @@ void block_solve_release(MixedState* st) {
 // packs would not fit in the device's free memory (the caller falls back).
 static int prepare(DenseSolver* s, MixedState* st, int nrhs, bool* fits) {
     *fits = true;
-    if (!st->block) st->block = new BlockSolveState();
+    if (!st->block) {
+        st->block = new BlockSolveState();
+        for (DeviceBuffer* b : {&st->block->packs, &st->block->work, &st->block->krylov}) b->order = s->ctx->stream;
+    }
     BlockSolveState* bs = st->block;
     const int64_t np = st->np, nbl = st->nbl;
     const int64_t l_rows = lower_pack_rows_before(nbl - 1, np);  // every L21 (the last block has none)

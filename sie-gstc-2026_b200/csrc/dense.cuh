@@ -29,6 +29,13 @@ struct DenseSolver {
     // sweep running several systems concurrently gives each its share.
     int sm_cap = 0;
 
+    // Sets the context, and its stream as the order of every buffer.
+    void bind(sieb200_ctx* c) {
+        ctx = c;
+        for (DeviceBuffer* b : {&ipiv, &work, &lu, &perm, &panel, &gemm_a, &gemm_b, &krylov, &vec, &flags,
+                                &gemv_scratch, &couple})
+            if (!b->ptr) b->order = c->stream;
+    }
     int factorize(double* A, int64_t lda);
     int solve(int64_t nrhs, double* B, int64_t ldb, bool adjoint, double tol, int maxit, int* iters);
 };

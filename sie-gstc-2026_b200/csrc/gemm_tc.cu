@@ -833,6 +833,7 @@ int encode_tensor_map_2d(CUtensorMap* map, CUtensorMapDataType type, const void*
 }
 
 struct GemmTC {
+    DeviceBuffer word;
     unsigned* err = nullptr;
     int mode = 3;  // persistent kernel, reduction epilogue
     int c_slots = 4;  // C slots of the persistent kernel's epilogue (1 or 4)
@@ -874,15 +875,18 @@ int launch_persistent(int variant, unsigned grid, cudaStream_t stream, const CUt
     }
 }
 
-int gemm_tc_create(GemmTC** out) {
+int gemm_tc_create(GemmTC** out, cudaStream_t stream) {
     GemmTC* g = new GemmTC();
-    cudaError_t e = cudaMalloc(&g->err, sizeof(unsigned));
-    if (e != cudaSuccess) {
+    g->word.order = stream;
+    const int st = g->word.reserve(sizeof(unsigned));
+    const cudaError_t e = st == SIEB200_OK ? cudaMemsetAsync(g->word.ptr, 0, sizeof(unsigned), stream) : cudaSuccess;
+    if (st != SIEB200_OK || e != cudaSuccess) {
         delete g;
+        if (st != SIEB200_OK) return st;
         set_error(std::string("gemm workspace: ") + cudaGetErrorString(e));
         return SIEB200_CUDA_ERROR;
     }
-    cudaMemset(g->err, 0, sizeof(unsigned));
+    g->err = g->word.as<unsigned>();
     const char* env = getenv("SIEB200_GEMM_SIMT");
     if (env && env[0] == '1') g->mode = 0;
     const char* mode_env = getenv("SIEB200_GEMM_MODE");
@@ -900,8 +904,6 @@ int gemm_tc_create(GemmTC** out) {
 }
 
 void gemm_tc_destroy(GemmTC* g) {
-    if (!g) return;
-    if (g->err) cudaFree(g->err);
     delete g;
 }
 

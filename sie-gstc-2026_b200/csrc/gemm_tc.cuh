@@ -12,7 +12,7 @@ namespace sieb200 {
 
 struct GemmTC;
 
-int gemm_tc_create(GemmTC** out);
+int gemm_tc_create(GemmTC** out, cudaStream_t stream);
 void gemm_tc_destroy(GemmTC* g);
 // Returns a SIEB200_* status; the kernel's bounded waits report through an
 // error word checked on the next synchronization (gemm_tc_check).

@@ -2135,13 +2135,12 @@ void mixed_release(DenseSolver* s) {
         if (st->ev_lcol) cudaEventDestroy(st->ev_lcol);
         if (st->ev_gemm) cudaEventDestroy(st->ev_gemm);
         if (st->ev_head) cudaEventDestroy(st->ev_head);
-        if (st->side) cudaStreamDestroy(st->side);
-        if (st->side2) cudaStreamDestroy(st->side2);
         delete st;
     }
     s->gemm_state = nullptr;
     s->lu.release(); s->perm.release(); s->panel.release(); s->gemm_a.release(); s->gemm_b.release();
     s->krylov.release(); s->vec.release(); s->flags.release(); s->gemv_scratch.release(); s->couple.release();
+    s->ipiv.release(); s->work.release();
 }
 
 static int check_err(DenseSolver* s, const char* what) {
@@ -2161,6 +2160,17 @@ static int check_err(DenseSolver* s, const char* what) {
         set_error(std::string(what) + ": device error word " + std::to_string(e));
         return SIEB200_CUDA_ERROR;
     }
+    return SIEB200_OK;
+}
+
+// The context's high-priority stream `own`, made on first use.
+static int lookahead_stream(cudaStream_t* own, cudaStream_t* out) {
+    if (!*own) {
+        int least = 0, greatest = 0;
+        SIEB_TRY_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+        SIEB_TRY_CUDA(cudaStreamCreateWithPriority(own, cudaStreamNonBlocking, greatest));
+    }
+    *out = *own;
     return SIEB200_OK;
 }
 
@@ -2262,20 +2272,16 @@ int mixed_factorize(DenseSolver* s) {
     st->Apack[0] = s->gemm_a.as<float>();
     st->Apack[1] = reinterpret_cast<float*>(s->gemm_a.as<char>() + bApack);
     st->Bpack = s->gemm_b.as<float>();
-    if (st->use_tc && !st->gemm) SIEB_RETURN_IF(gemm_tc_create(&st->gemm));
-    if (!st->side) {
-        int least = 0, greatest = 0;
-        SIEB_TRY_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-        SIEB_TRY_CUDA(cudaStreamCreateWithPriority(&st->side, cudaStreamNonBlocking, greatest));
+    if (st->use_tc && !st->gemm) SIEB_RETURN_IF(gemm_tc_create(&st->gemm, stream));
+    SIEB_RETURN_IF(lookahead_stream(&ctx->side, &st->side));
+    if (!st->ev_cols) {
         SIEB_TRY_CUDA(cudaEventCreateWithFlags(&st->ev_cols, cudaEventDisableTiming));
         SIEB_TRY_CUDA(cudaEventCreateWithFlags(&st->ev_diag, cudaEventDisableTiming));
         SIEB_TRY_CUDA(cudaEventCreateWithFlags(&st->ev_pan, cudaEventDisableTiming));
     }
-    if (!st->side2) {
-        int least = 0, greatest = 0;
-        SIEB_TRY_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-        SIEB_TRY_CUDA(cudaStreamCreateWithPriority(&st->side2, cudaStreamNonBlocking, greatest));
-        SIEB_TRY_CUDA(cudaEventCreateWithFlags(&st->ev_lcol, cudaEventDisableTiming));
+    if (st->lcol == 2) {
+        SIEB_RETURN_IF(lookahead_stream(&ctx->side2, &st->side2));
+        if (!st->ev_lcol) SIEB_TRY_CUDA(cudaEventCreateWithFlags(&st->ev_lcol, cudaEventDisableTiming));
     }
     if (!st->ev_gemm) {
         SIEB_TRY_CUDA(cudaEventCreateWithFlags(&st->ev_gemm, cudaEventDisableTiming));
@@ -3171,10 +3177,8 @@ static int fp64_factorize(DenseSolver* s) {
     st->diag_panels = diag_panels_env();
     st->diag_compact = diag_compact_env();
     st->diag_rec = 0;  // complex64 only
-    if (!st->side) {
-        int least = 0, greatest = 0;
-        SIEB_TRY_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-        SIEB_TRY_CUDA(cudaStreamCreateWithPriority(&st->side, cudaStreamNonBlocking, greatest));
+    SIEB_RETURN_IF(lookahead_stream(&ctx->side, &st->side));
+    if (!st->ev_cols) {
         SIEB_TRY_CUDA(cudaEventCreateWithFlags(&st->ev_cols, cudaEventDisableTiming));
         SIEB_TRY_CUDA(cudaEventCreateWithFlags(&st->ev_diag, cudaEventDisableTiming));
         SIEB_TRY_CUDA(cudaEventCreateWithFlags(&st->ev_pan, cudaEventDisableTiming));

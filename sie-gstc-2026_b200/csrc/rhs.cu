@@ -543,7 +543,7 @@ int incident_fields_device(sieb200_ctx* ctx, const sieb200_options& opt, const s
     const size_t pbytes = sizeof(double) * 3 * (size_t)n, fbytes = sizeof(cplx) * 3 * (size_t)n;
     const size_t off_s = ((pbytes + 255) / 256) * 256;
     const size_t off_e = off_s + 256, off_h = off_e + ((fbytes + 255) / 256) * 256;
-    DeviceBuffer buf;
+    DeviceBuffer buf(st);
     SIEB_RETURN_IF(buf.reserve(off_h + fbytes));
     char* b = buf.as<char>();
     SIEB_TRY_CUDA(cudaMemcpyAsync(b, points, pbytes, cudaMemcpyHostToDevice, st));
@@ -580,7 +580,7 @@ int far_field_device(sieb200_ctx* ctx, const sieb200_mesh& mesh, const double* j
                  oPart = take(sizeof(double) * 12 * (size_t)chunks * ndir),
                  oDir = take(sizeof(double) * 9 * ndir), oOut = take(sizeof(cplx) * 2 * ndir),
                  oU = take(sizeof(double) * ndir);
-    DeviceBuffer buf;
+    DeviceBuffer buf(st);
     SIEB_RETURN_IF(buf.reserve(off));
     char* b = buf.as<char>();
     double* rec = reinterpret_cast<double*>(b + oRec);
@@ -644,7 +644,7 @@ int far_field_matrix_device(sieb200_ctx* ctx, const sieb200_mesh& mesh, double k
     auto take = [&](size_t bytes) { size_t o = off; off += ((bytes + 255) / 256) * 256; return o; };
     const size_t oV = take(sizeof(double) * 3 * nv), oF = take(sizeof(int) * 3 * nf),
                  oI = take(sizeof(int) * 2 * ne), oDir = take(sizeof(double) * 9 * ndir);
-    DeviceBuffer buf;
+    DeviceBuffer buf(st);
     SIEB_RETURN_IF(buf.reserve(off));
     char* b = buf.as<char>();
     SIEB_TRY_CUDA(cudaMemcpyAsync(b + oV, mesh.vertices, sizeof(double) * 3 * nv, cudaMemcpyHostToDevice, st));
