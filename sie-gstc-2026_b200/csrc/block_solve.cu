@@ -173,7 +173,7 @@ __global__ void rbt_block_N_kernel(const float2* __restrict__ Y, int64_t ldy, in
     }
 }
 
-// Diagonal block k of a triangular solve on Y: X_k = Inv_k Y_k for 16
+// Diagonal block k of a triangular solve on Y: X_k = Inv_k Y_k for 8
 // columns per CTA (FP64 accumulation of the complex64 values), written back
 // into Y and packed as the GEMM's B operand: column j of Xpack is
 // [Re, Im] per row, split [hi | lo | hi] along K. Rows beyond the block's
@@ -183,81 +183,108 @@ __global__ void rbt_block_N_kernel(const float2* __restrict__ Y, int64_t ldy, in
 // with leading dimension ldf; X_prev the previous block's solved rows of Y,
 // kbp of them): the trailing GEMM of the previous step skips this block, so
 // that this kernel and that GEMM run side by side.
-constexpr int DA_COLS = 16;
+// Bound: latency, one of the two kernels on every step's chain. A warp takes a
+// column, its lanes rows l and l + 32, so that the matrix column comes from
+// shared memory without conflicts (row pitch 65 entries) and the vector entry
+// is a broadcast; each thread's global loads go out together before its first
+// shared-memory store. 6.5 us per launch at 64 columns; with 16 columns per
+// CTA and four neighbouring rows per thread every read conflicted 8 ways:
+// 14.5 us.
+constexpr int DA_COLS = 8;
 constexpr int kSmemDiagApply = (2 * NB * (NB + 1) + 2 * DA_COLS * NB) * (int)sizeof(float2);
-__global__ void __launch_bounds__(256) diag_apply_kernel(float2* __restrict__ Y, int64_t ldy, int64_t k0, int kb,
-                                                         int nrhs, const float2* __restrict__ Inv,
-                                                         float* __restrict__ Xpack,
-                                                         const float2* __restrict__ Fb, int64_t ldf,
-                                                         const float2* __restrict__ Xprev, int kbp, int kw,
-                                                         int lo_rn) {
+__global__ void __launch_bounds__(32 * DA_COLS) diag_apply_kernel(float2* __restrict__ Y, int64_t ldy, int64_t k0,
+                                                                  int kb, int nrhs, const float2* __restrict__ Inv,
+                                                                  float* __restrict__ Xpack,
+                                                                  const float2* __restrict__ Fb, int64_t ldf,
+                                                                  const float2* __restrict__ Xprev, int kbp, int kw,
+                                                                  int lo_rn) {
+    constexpr int kThreads = 32 * DA_COLS, kPer = NB * NB / kThreads;
+    static_assert(NB == 64, "two rows per lane");
     extern __shared__ __align__(16) float2 da_smem[];
     float2(*inv)[NB + 1] = reinterpret_cast<float2(*)[NB + 1]>(da_smem);              // [row][col]
     float2(*fb)[NB + 1] = inv + NB;                                                    // [row][col]
     float2(*ys)[NB] = reinterpret_cast<float2(*)[NB]>(da_smem + 2 * NB * (NB + 1));   // [col][row]
     float2(*xp)[NB] = ys + DA_COLS;                                                    // [col][row]
-    const int tid = threadIdx.x;
-    const int c0 = blockIdx.x * DA_COLS;
-    for (int e = tid; e < NB * NB; e += blockDim.x) inv[e % NB][e / NB] = Inv[e];  // Inv[r + c NB]
-    for (int e = tid; e < DA_COLS * NB; e += blockDim.x) {
-        const int r = e % NB, c = e / NB;
-        ys[c][r] = (c0 + c < nrhs && r < kb) ? Y[(k0 + r) + (int64_t)(c0 + c) * ldy] : make_float2(0.f, 0.f);
+    const int tid = threadIdx.x, lane = tid & 31, c = tid >> 5;
+    const int gc = blockIdx.x * DA_COLS + c;
+    const float2 z = make_float2(0.f, 0.f);
+    {
+        float2 m[kPer], y[2];
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) m[i] = Inv[tid + i * kThreads];  // Inv[r + c NB]
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int r = lane + 32 * h;
+            y[h] = (gc < nrhs && r < kb) ? Y[(k0 + r) + (int64_t)gc * ldy] : z;
+        }
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+            const int e = tid + i * kThreads;
+            inv[e % NB][e / NB] = m[i];
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) ys[c][lane + 32 * h] = y[h];
     }
     if (Fb) {
-        for (int e = tid; e < NB * NB; e += blockDim.x) {
-            const int r = e % NB, c = e / NB;
-            fb[r][c] = (r < kb && c < kbp) ? Fb[r + (int64_t)c * ldf] : make_float2(0.f, 0.f);
+        float2 m[kPer];
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+            const int e = tid + i * kThreads, r = e % NB, q = e / NB;
+            m[i] = (r < kb && q < kbp) ? Fb[r + (int64_t)q * ldf] : z;
         }
-        for (int e = tid; e < DA_COLS * NB; e += blockDim.x) {
-            const int r = e % NB, c = e / NB;
-            xp[c][r] = (c0 + c < nrhs && r < kbp) ? Xprev[r + (int64_t)(c0 + c) * ldy] : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int r = lane + 32 * h;
+            xp[c][r] = (gc < nrhs && r < kbp) ? Xprev[r + (int64_t)gc * ldy] : z;
+        }
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+            const int e = tid + i * kThreads;
+            fb[e % NB][e / NB] = m[i];
         }
     }
     __syncthreads();
-    const int c = tid / 16;         // column of this thread
-    const int r0 = (tid % 16) * 4;  // its four rows
-    if (Fb) {
-        double fr[4] = {0, 0, 0, 0}, fi[4] = {0, 0, 0, 0};
-        for (int kk = 0; kk < NB; ++kk) {
-            const float2 x = xp[c][kk];
+    // M v of this warp's column, rows lane and lane + 32
+    auto product = [&](float2(*M)[NB + 1], const float2* v, double (&re)[2], double (&im)[2]) {
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const float2 a = fb[r0 + u][kk];
-                fr[u] += (double)a.x * x.x - (double)a.y * x.y;
-                fi[u] += (double)a.x * x.y + (double)a.y * x.x;
+        for (int h = 0; h < 2; ++h) re[h] = im[h] = 0.0;
+#pragma unroll 8
+        for (int kk = 0; kk < NB; ++kk) {
+            const float2 x = v[kk];
+            const double xr = x.x, xi = x.y;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float2 a = M[lane + 32 * h][kk];
+                re[h] += (double)a.x * xr - (double)a.y * xi;
+                im[h] += (double)a.x * xi + (double)a.y * xr;
             }
         }
-        // each thread owns rows r0 .. r0+3 of column c of ys
+    };
+    double re[2], im[2];
+    if (Fb) {
+        product(fb, xp[c], re, im);
+        // each lane owns its two rows of its column of ys
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const float2 y = ys[c][r0 + u];
-            ys[c][r0 + u] = make_float2((float)((double)y.x - fr[u]), (float)((double)y.y - fi[u]));
+        for (int h = 0; h < 2; ++h) {
+            const float2 y = ys[c][lane + 32 * h];
+            ys[c][lane + 32 * h] = make_float2((float)((double)y.x - re[h]), (float)((double)y.y - im[h]));
         }
-        __syncthreads();
+        __syncwarp();
     }
-    double ar[4] = {0, 0, 0, 0}, ai[4] = {0, 0, 0, 0};
-    for (int kk = 0; kk < NB; ++kk) {
-        const float2 y = ys[c][kk];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const float2 a = inv[r0 + u][kk];
-            ar[u] += (double)a.x * y.x - (double)a.y * y.y;
-            ai[u] += (double)a.x * y.y + (double)a.y * y.x;
-        }
-    }
-    const int gc = c0 + c;
+    product(inv, ys[c], re, im);
     if (gc >= nrhs) return;
     float* col = Xpack + (int64_t)gc * kw;  // [hi | lo] (KH) or [hi | lo | hi] (K3)
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        const int r = r0 + u;
+    for (int h = 0; h < 2; ++h) {
+        const int r = lane + 32 * h;
         const bool in = r < kb;
-        const float vx = in ? (float)ar[u] : 0.f, vy = in ? (float)ai[u] : 0.f;
+        const float vx = in ? (float)re[h] : 0.f, vy = in ? (float)im[h] : 0.f;
         if (in) Y[(k0 + r) + (int64_t)gc * ldy] = make_float2(vx, vy);
         const float h0 = tf32_hi(vx), h1 = tf32_hi(vy);
-        col[2 * r] = h0; col[2 * r + 1] = h1;
-        col[2 * NB + 2 * r] = tf32_lo(vx, h0, lo_rn); col[2 * NB + 2 * r + 1] = tf32_lo(vy, h1, lo_rn);
-        if (kw == K3) { col[4 * NB + 2 * r] = h0; col[4 * NB + 2 * r + 1] = h1; }
+        float2* out = reinterpret_cast<float2*>(col) + r;
+        out[0] = make_float2(h0, h1);
+        out[NB] = make_float2(tf32_lo(vx, h0, lo_rn), tf32_lo(vy, h1, lo_rn));
+        if (kw == K3) out[2 * NB] = make_float2(h0, h1);
     }
 }
 
@@ -710,7 +737,7 @@ static int enqueue_triangular(DenseSolver* s, MixedState* st, BlockSolveState* b
         for (int64_t k = 0; k < nbl; ++k) {
             const int64_t k0 = k * NB;
             const int kb = (int)std::min<int64_t>(NB, np - k0);
-            diag_apply_kernel<<<gda, 256, kSmemDiagApply, stream>>>(bs->Y, bs->ldy, k0, kb, nrhs,
+            diag_apply_kernel<<<gda, 32 * DA_COLS, kSmemDiagApply, stream>>>(bs->Y, bs->ldy, k0, kb, nrhs,
                                                                      st->Linv + (size_t)k * NB * NB, Xbuf[0],
                                                                      nullptr, 0, nullptr, 0, kw, st->lo_rn);
             SIEB_NOTE_LAUNCH();
@@ -725,7 +752,7 @@ static int enqueue_triangular(DenseSolver* s, MixedState* st, BlockSolveState* b
         for (int64_t k = nbl - 1; k >= 0; --k) {
             const int64_t k0 = k * NB;
             const int kb = (int)std::min<int64_t>(NB, np - k0);
-            diag_apply_kernel<<<gda, 256, kSmemDiagApply, stream>>>(bs->Y, bs->ldy, k0, kb, nrhs,
+            diag_apply_kernel<<<gda, 32 * DA_COLS, kSmemDiagApply, stream>>>(bs->Y, bs->ldy, k0, kb, nrhs,
                                                                      st->Uinv + (size_t)k * NB * NB, Xbuf[0],
                                                                      nullptr, 0, nullptr, 0, kw, st->lo_rn);
             SIEB_NOTE_LAUNCH();
@@ -760,7 +787,7 @@ static int enqueue_triangular(DenseSolver* s, MixedState* st, BlockSolveState* b
                 Xprev = bs->Y + p0;
                 kbp = (int)std::min<int64_t>(NB, np - p0);
             }
-            diag_apply_kernel<<<gda, 256, kSmemDiagApply, side>>>(
+            diag_apply_kernel<<<gda, 32 * DA_COLS, kSmemDiagApply, side>>>(
                 bs->Y, bs->ldy, k0, kb, nrhs, (pass == 0 ? st->Linv : st->Uinv) + (size_t)k * NB * NB, Xk, Fb,
                 st->ldw, Xprev, kbp, kw, st->lo_rn);
             SIEB_NOTE_LAUNCH();
