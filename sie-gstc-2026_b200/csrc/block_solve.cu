@@ -578,25 +578,44 @@ __global__ void __launch_bounds__(ZD_THREADS, 2) zgemm_dmma_kernel(int64_t m, in
         }
     }
     cp_async_wait<0>();
+    // Two row blocks at a time: their 16 entries of C per lane are read together
+    // before any is written. Read and written entry by entry, a tile's 32
+    // round trips to memory followed one another, longer than the products of a
+    // short K: at K = 64 (the trailing updates of the FP64 factorization,
+    // 2940 unknowns) 6.4 ms over all steps then, 4.9 ms now.
     const bool use_beta = beta.x != 0.0 || beta.y != 0.0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int64_t gr = row0 + wr + 8 * i + fr;
-        if (gr >= m) continue;
+    for (int i0 = 0; i0 < 4; i0 += 2) {
+        double2 c[2][4][2];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int i = 0; i < 2; ++i) {
+            const int64_t gr = row0 + wr + 8 * (i0 + i) + fr;
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int64_t gc = col0 + wc + 8 * j + 2 * fk + h;
-                if (gc >= nc) continue;
-                const double vr = re[i][j][h], vi = im[i][j][h];
-                double2 out = make_double2(alpha.x * vr - alpha.y * vi, alpha.x * vi + alpha.y * vr);
-                if (use_beta) {
-                    const double2 c = C[gr + gc * ldc];
-                    out.x += beta.x * c.x - beta.y * c.y;
-                    out.y += beta.x * c.y + beta.y * c.x;
+            for (int j = 0; j < 4; ++j) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int64_t gc = col0 + wc + 8 * j + 2 * fk + h;
+                    c[i][j][h] = (use_beta && gr < m && gc < nc) ? C[gr + gc * ldc] : make_double2(0.0, 0.0);
                 }
-                C[gr + gc * ldc] = out;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int64_t gr = row0 + wr + 8 * (i0 + i) + fr;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int64_t gc = col0 + wc + 8 * j + 2 * fk + h;
+                    if (gr >= m || gc >= nc) continue;
+                    const double vr = re[i0 + i][j][h], vi = im[i0 + i][j][h];
+                    double2 out = make_double2(alpha.x * vr - alpha.y * vi, alpha.x * vi + alpha.y * vr);
+                    if (use_beta) {
+                        out.x += beta.x * c[i][j][h].x - beta.y * c[i][j][h].y;
+                        out.y += beta.x * c[i][j][h].y + beta.y * c[i][j][h].x;
+                    }
+                    C[gr + gc * ldc] = out;
+                }
             }
         }
     }
