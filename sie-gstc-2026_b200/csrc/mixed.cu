@@ -1643,6 +1643,20 @@ __global__ void __launch_bounds__(256) trsv_couple_kernel(const float2* __restri
     for (int i = 0; i < NB / 4; ++i) out[r + (c0 + 4 * i) * NB] = make_float2((float)re[i], (float)im[i]);
 }
 
+// An FP64 complex sum as four chains of fused multiply-adds.
+struct CSum {
+    double rr = 0.0, ii = 0.0, ri = 0.0, ir = 0.0;
+    __device__ __forceinline__ void add(const float2& w, const cplx& v) {
+        const double wx = w.x, wy = w.y;
+        rr = fma(wx, v.re, rr);
+        ii = fma(wy, v.im, ii);
+        ri = fma(wx, v.im, ri);
+        ir = fma(wy, v.re, ir);
+    }
+    __device__ __forceinline__ double re() const { return rr - ii; }
+    __device__ __forceinline__ double im() const { return ri + ir; }
+};
+
 // trsv_tma_kernel for 128-row CTAs with the coupling to the newest
 // sub-block folded into precomputed products (trsv_couple_kernel). A CTA's
 // sub-blocks in solve order are s1, s2; p is the one published just before
@@ -1653,11 +1667,15 @@ __global__ void __launch_bounds__(256) trsv_couple_kernel(const float2* __restri
 // published before p, which are streamed and accumulated as before, and
 // Dinv y formed while p is still awaited. Once x_p is in, s1 is one 64 x 64
 // product away from publication and s2 one more, with no coupling tiles
-// (the P slices are read into registers at the start): 203 against 213 us
+// (the P slices are read into registers at the start): 187 against 213 us
 // per solve at N = 6016. Folding the previous CTA's first sub-block as well
 // (P3, one poll for both) measured slower, 246-254 us: the longer FP64
-// product then sits on the chain. The same bounded waits, abort and
-// publication protocol as trsv_tma_kernel.
+// product then sits on the chain. One 128 x 128 step in place of the two
+// halves took 161 us, but x_s2 then no longer follows from the x_s1 that was
+// rounded, and ill-conditioned systems stopped converging. The same bounded
+// waits, abort and publication as trsv_tma_kernel, except that progress[0]
+// is not kept: nothing reads it, and the release stood on the chain (203 us
+// with it and with separate multiplies and adds).
 constexpr int kSmemTrsvFold = kSmemTrsv + NB * (int)sizeof(cplx);
 // Registers are granted to 288 threads in units of four warps (12 warps'
 // worth), which caps a thread at 168.
@@ -1769,7 +1787,7 @@ trsv_fold_kernel(const __grid_constant__ CUtensorMap tmW, int64_t np, int nsb, i
     const int64_t grow = R0 + r;
     cplx b = cx(0, 0);  // written only by this CTA: final from the start
     if (h == 0 && grow < np) b = cx(__ldcg(&x[grow].re), __ldcg(&x[grow].im));
-    double acc_re = 0.0, acc_im = 0.0;
+    CSum acc;
     // Polls the NB entries of sub-block sb, and of sub-block sb2 as well
     // when sb2 >= 0 (warp 0, two entries of each per lane, all in every
     // round) into dst / dst2; false on abort or timeout.
@@ -1837,14 +1855,14 @@ trsv_fold_kernel(const __grid_constant__ CUtensorMap tmW, int64_t np, int nsb, i
                 for (int u = 0; u < CPT; ++u) {
                     const float2 w = tile[(h * CPT + u) * ROWS + r];
                     const cplx xv = xt[u];
-                    acc_re += (double)w.x * xv.re - (double)w.y * xv.im;
-                    acc_im += (double)w.x * xv.im + (double)w.y * xv.re;
+                    acc.add(w, xv);
                 }
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(empty0 + 8 * st);
         }
     }
+    const double acc_re = acc.re(), acc_im = acc.im();
     if (h >= 1) red[(h - 1) * ROWS + r] = cx(acc_re, acc_im);
     consumer_bar();
     if (h == 0) ys[r] = cx(b.re - (acc_re + red[r].re), b.im - (acc_im + red[r].im));
@@ -1855,15 +1873,13 @@ trsv_fold_kernel(const __grid_constant__ CUtensorMap tmW, int64_t np, int nsb, i
     auto dinv_apply = [&](int which) {
         const float2* D = Ds + which * NB * TR_DLD;
         const cplx* y = ys + which * NB;
-        double re = 0.0, im = 0.0;
+        CSum a;
 #pragma unroll
         for (int u = 0; u < NB / 4; ++u) {
             const int c = part + 4 * u;
-            const float2 d = D[c * TR_DLD + dr];
-            const cplx yv = y[c];
-            re += (double)d.x * yv.re - (double)d.y * yv.im;
-            im += (double)d.x * yv.im + (double)d.y * yv.re;
+            a.add(D[c * TR_DLD + dr], y[c]);
         }
+        double re = a.re(), im = a.im();
         re += __shfl_xor_sync(0xffffffffu, re, 1);
         im += __shfl_xor_sync(0xffffffffu, im, 1);
         re += __shfl_xor_sync(0xffffffffu, re, 2);
@@ -1879,15 +1895,12 @@ trsv_fold_kernel(const __grid_constant__ CUtensorMap tmW, int64_t np, int nsb, i
     consumer_bar();
     if (!s_go) return;  // block-uniform
     {
-        double re = 0.0, im = 0.0;
+        CSum a;
         if (use_a) {
 #pragma unroll
-            for (int u = 0; u < NB / 2; ++u) {
-                const cplx xv = xp[c1 + 2 * u];
-                re += (double)pa[u].x * xv.re - (double)pa[u].y * xv.im;
-                im += (double)pa[u].x * xv.im + (double)pa[u].y * xv.re;
-            }
+            for (int u = 0; u < NB / 2; ++u) a.add(pa[u], xp[c1 + 2 * u]);
         }
+        double re = a.re(), im = a.im();
         re += __shfl_xor_sync(0xffffffffu, re, 1);
         im += __shfl_xor_sync(0xffffffffu, im, 1);
         if (c1 == 0) {
@@ -1908,17 +1921,13 @@ trsv_fold_kernel(const __grid_constant__ CUtensorMap tmW, int64_t np, int nsb, i
             }
         }
     }
-    consumer_bar();  // orders the stores of s1 before the release
-    if (tid == 0) st_release_gpu(&progress[0], lower ? (unsigned)s1 + 1u : (unsigned)(nsb - s1));
     if (!has_bot) return;
+    consumer_bar();  // x_s1 and ts in
     {
-        double re = 0.0, im = 0.0;
+        CSum a;
 #pragma unroll
-        for (int u = 0; u < NB / 4; ++u) {
-            const cplx xv = xs[part + 4 * u];
-            re += (double)pb[u].x * xv.re - (double)pb[u].y * xv.im;
-            im += (double)pb[u].x * xv.im + (double)pb[u].y * xv.re;
-        }
+        for (int u = 0; u < NB / 4; ++u) a.add(pb[u], xs[part + 4 * u]);
+        double re = a.re(), im = a.im();
         re += __shfl_xor_sync(0xffffffffu, re, 1);
         im += __shfl_xor_sync(0xffffffffu, im, 1);
         re += __shfl_xor_sync(0xffffffffu, re, 2);
@@ -1934,8 +1943,6 @@ trsv_fold_kernel(const __grid_constant__ CUtensorMap tmW, int64_t np, int nsb, i
             }
         }
     }
-    consumer_bar();
-    if (tid == 0) st_release_gpu(&progress[0], lower ? (unsigned)s2 + 1u : (unsigned)(nsb - s2));
 }
 
 // ------------------------------------------------------------ small vector ops
