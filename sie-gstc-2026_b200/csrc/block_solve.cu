@@ -500,16 +500,31 @@ __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
                  : "d"(a), "d"(b));
 }
 
+// TRAILING: the trailing update of the FP64 factorization (zgemm_trailing), a
+// one-dimensional grid over the tiles of the first `strip` tile columns and,
+// right of them, the first `strip` tile rows, without tile (0, 0).
+template <bool TRAILING>
 __global__ void __launch_bounds__(ZD_THREADS, 2) zgemm_dmma_kernel(int64_t m, int64_t nc, int64_t kdim,
                                                                    const double2* __restrict__ A, int64_t lda,
                                                                    const double2* __restrict__ X, int64_t ldx,
                                                                    double2* __restrict__ C, int64_t ldc,
-                                                                   double2 alpha, double2 beta) {
+                                                                   double2 alpha, double2 beta, int strip) {
     extern __shared__ __align__(16) double2 zd_smem[];
     double2* As = zd_smem;                                // [stage][k][ZD_ALD]
     double2* Xs = zd_smem + ZD_STAGES * ZD_STAGE_A;       // [stage][col][ZD_XLD]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int64_t row0 = (int64_t)blockIdx.x * ZD_BM, col0 = (int64_t)blockIdx.y * ZD_BN;
+    int tr = blockIdx.x, tc = blockIdx.y;
+    if (TRAILING) {
+        const int mt = (int)((m + ZD_BM - 1) / ZD_BM), t = (int)blockIdx.x + 1;
+        if (t < mt * strip) {
+            tr = t % mt;
+            tc = t / mt;
+        } else {
+            tr = (t - mt * strip) % strip;
+            tc = strip + (t - mt * strip) / strip;
+        }
+    }
+    const int64_t row0 = (int64_t)tr * ZD_BM, col0 = (int64_t)tc * ZD_BN;
     const int wr = (warp & 1) * 32, wc = (warp >> 1) * 32;  // warp tile origin in the CTA tile
     const int nk = (int)((kdim + ZD_BK - 1) / ZD_BK);
 
@@ -637,6 +652,25 @@ inline unsigned nblk(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
 }  // namespace
 
+static bool zgemm_dmma_selected() {
+    const char* e = getenv("SIEB200_ZGEMM_DMMA");
+    return !(e && e[0] == '0');
+}
+
+static int zgemm_dmma_attributes() {
+    static bool attr_set[64] = {};
+    int dev = 0;
+    SIEB_TRY_CUDA(cudaGetDevice(&dev));
+    if (!attr_set[dev & 63]) {
+        SIEB_TRY_CUDA(cudaFuncSetAttribute(zgemm_dmma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           kSmemZgemmDmma));
+        SIEB_TRY_CUDA(cudaFuncSetAttribute(zgemm_dmma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           kSmemZgemmDmma));
+        attr_set[dev & 63] = true;
+    }
+    return SIEB200_OK;
+}
+
 // C = alpha A X + beta C (FP64 complex, column-major). Exposed for the
 // residual of the batched refinement and its tests.
 int zgemm_device(cudaStream_t stream, int64_t m, int64_t nc, int64_t kdim, const cplx* A, int64_t lda,
@@ -645,22 +679,14 @@ int zgemm_device(cudaStream_t stream, int64_t m, int64_t nc, int64_t kdim, const
     SIEB_CHECK(nc < 65536ll * ZG_BN && m < (1ll << 40), SIEB200_INVALID_ARG, "zgemm: size out of range");
     // The tensor-core kernel needs 16-byte aligned operands (cp.async of one
     // complex entry); SIEB200_ZGEMM_DMMA=0 selects the FMA kernel.
-    const char* dm_env = getenv("SIEB200_ZGEMM_DMMA");
     const bool aligned = ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(X) |
                            reinterpret_cast<uintptr_t>(C)) & 15) == 0;
-    if (!(dm_env && dm_env[0] == '0') && aligned && nc < 65536ll * ZD_BN) {
-        static bool attr_set[64] = {};
-        int dev = 0;
-        SIEB_TRY_CUDA(cudaGetDevice(&dev));
-        if (!attr_set[dev & 63]) {
-            SIEB_TRY_CUDA(cudaFuncSetAttribute(zgemm_dmma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               kSmemZgemmDmma));
-            attr_set[dev & 63] = true;
-        }
+    if (zgemm_dmma_selected() && aligned && nc < 65536ll * ZD_BN) {
+        SIEB_RETURN_IF(zgemm_dmma_attributes());
         const dim3 grid(nblk(m, ZD_BM), nblk(nc, ZD_BN));
-        zgemm_dmma_kernel<<<grid, ZD_THREADS, kSmemZgemmDmma, stream>>>(
+        zgemm_dmma_kernel<false><<<grid, ZD_THREADS, kSmemZgemmDmma, stream>>>(
             m, nc, kdim, reinterpret_cast<const double2*>(A), lda, reinterpret_cast<const double2*>(X), ldx,
-            reinterpret_cast<double2*>(C), ldc, make_double2(alpha.re, alpha.im), make_double2(beta.re, beta.im));
+            reinterpret_cast<double2*>(C), ldc, make_double2(alpha.re, alpha.im), make_double2(beta.re, beta.im), 0);
         SIEB_NOTE_LAUNCH();
         SIEB_TRY_CUDA(cudaGetLastError());
         return SIEB200_OK;
@@ -673,6 +699,37 @@ int zgemm_device(cudaStream_t stream, int64_t m, int64_t nc, int64_t kdim, const
     SIEB_NOTE_LAUNCH();
     SIEB_TRY_CUDA(cudaGetLastError());
     return SIEB200_OK;
+}
+
+// C -= A X for the m x m trailing matrix C (A m x k, X k x m) in its first w
+// columns and first w rows (w = m: all of it; otherwise a multiple of the
+// 64-entry tile), without the leading 64 x 64 block.
+int zgemm_trailing(cudaStream_t stream, int64_t m, int64_t w, int64_t kdim, const cplx* A, int64_t lda, const cplx* X,
+                   int64_t ldx, cplx* C, int64_t ldc) {
+    constexpr int64_t T = ZD_BM;
+    static_assert(ZD_BM == NB && ZD_BN == NB, "the leading block is one tile");
+    if (m <= T) return SIEB200_OK;
+    SIEB_CHECK(w == m || (w > 0 && w < m && w % T == 0), SIEB200_INVALID_ARG, "trailing update: invalid strip");
+    const int64_t mt = (m + T - 1) / T, wt = (w + T - 1) / T;
+    SIEB_CHECK(mt < 46340, SIEB200_INVALID_ARG, "trailing update: size out of range");
+    const bool aligned = ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(X) |
+                           reinterpret_cast<uintptr_t>(C)) & 15) == 0;
+    if (zgemm_dmma_selected() && aligned) {
+        SIEB_RETURN_IF(zgemm_dmma_attributes());
+        zgemm_dmma_kernel<true><<<(unsigned)(mt * wt + wt * (mt - wt) - 1), ZD_THREADS, kSmemZgemmDmma, stream>>>(
+            m, m, kdim, reinterpret_cast<const double2*>(A), lda, reinterpret_cast<const double2*>(X), ldx,
+            reinterpret_cast<double2*>(C), ldc, make_double2(-1.0, 0.0), make_double2(1.0, 0.0), (int)wt);
+        SIEB_NOTE_LAUNCH();
+        SIEB_TRY_CUDA(cudaGetLastError());
+        return SIEB200_OK;
+    }
+    auto part = [&](int64_t r0, int64_t r1, int64_t c0, int64_t c1) -> int {
+        return zgemm_device(stream, r1 - r0, c1 - c0, kdim, A + r0, lda, X + c0 * ldx, ldx, C + r0 + c0 * ldc, ldc,
+                            cx(-1, 0), cx(1, 0));
+    };
+    SIEB_RETURN_IF(part(T, m, 0, std::min(T, w)));
+    SIEB_RETURN_IF(part(0, m, T, w));
+    return part(0, std::min(w, m), w, m);
 }
 
 void block_solve_release(MixedState* st) {

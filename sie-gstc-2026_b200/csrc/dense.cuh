@@ -62,6 +62,8 @@ void destroy_cusolver(sieb200_ctx* ctx);
 // block_solve.cu).
 int zgemm_device(cudaStream_t stream, int64_t m, int64_t nc, int64_t kdim, const cplx* A, int64_t lda,
                  const cplx* X, int64_t ldx, cplx* C, int64_t ldc, cplx alpha, cplx beta);
+int zgemm_trailing(cudaStream_t stream, int64_t m, int64_t w, int64_t kdim, const cplx* A, int64_t lda, const cplx* X,
+                   int64_t ldx, cplx* C, int64_t ldc);
 
 }  // namespace sieb200
 
