@@ -275,7 +275,9 @@ int gemv_device(sieb200_ctx* ctx, int64_t n, const void* A, int64_t lda, int pre
         row_blocks = (n + threads - 1) / threads;
         // Aim for ~4 CTAs per SM.
         chunks = std::max<int64_t>(1, (int64_t)ctx->sm_count * 4 / std::max<int64_t>(1, row_blocks));
-        chunks = std::min<int64_t>(chunks, std::max<int64_t>(1, n / 64));
+        // At least 16 columns per chunk, at most 64 chunks: a chunk's columns follow one another
+        // (n = 120: 16 us as one chunk, 3.4 us as seven).
+        chunks = std::min<int64_t>(std::min<int64_t>(chunks, 64), std::max<int64_t>(1, n / 16));
         cpc = (n + chunks - 1) / chunks;
         chunks = (n + cpc - 1) / cpc;
     }

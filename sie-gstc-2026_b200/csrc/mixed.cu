@@ -1597,52 +1597,6 @@ trsv_tma_kernel(const __grid_constant__ CUtensorMap tmW, int64_t np, int nsb, in
     solve_sub(second);
 }
 
-// Coupling products for trsv_fold_kernel: for sub-block k and its
-// neighbours at distance d in solve order (lower: k - d, upper: k + d),
-// Pd[k] = Dinv_k F(k, k -/+ d), F the factor (W or its conjugate transpose;
-// rows and columns beyond np read as zero), Dinv_k the sub-block's inverse
-// (NB x NB column-major). grid (nsb, D): blockIdx.y + 1 is d (zero where
-// the neighbour does not exist); P = P1 (nsb blocks), P2, .., each NB x NB
-// column-major complex64, accumulated in FP64.
-constexpr int kSmemCouple = 2 * NB * (NB + 1) * (int)sizeof(float2);
-__global__ void __launch_bounds__(256) trsv_couple_kernel(const float2* __restrict__ M, int64_t ldm, int64_t np,
-                                                          int nsb, int lower, const float2* __restrict__ Dinv,
-                                                          float2* __restrict__ P) {
-    extern __shared__ __align__(16) unsigned char dyn_smem[];
-    float2(*Ds)[NB + 1] = reinterpret_cast<float2(*)[NB + 1]>(dyn_smem);  // [row][q]
-    float2(*Fs)[NB + 1] = Ds + NB;                                           // [q][col]
-    const int k = blockIdx.x, dist = blockIdx.y + 1;
-    const int nb = lower ? k - dist : k + dist;  // neighbour sub-block
-    float2* out = P + ((size_t)blockIdx.y * nsb + k) * NB * NB;
-    const int tid = threadIdx.x;
-    if (nb < 0 || nb >= nsb) {
-        for (int e = tid; e < NB * NB; e += 256) out[e] = make_float2(0.f, 0.f);
-        return;
-    }
-    for (int e = tid; e < NB * NB; e += 256) {
-        const int r = e % NB, c = e / NB;  // rows fastest: coalesced columns
-        Ds[r][c] = Dinv[(size_t)k * NB * NB + e];
-        const int64_t gr = (int64_t)k * NB + r, gc = (int64_t)nb * NB + c;
-        Fs[r][c] = (gr < np && gc < np) ? M[gr + gc * ldm] : make_float2(0.f, 0.f);
-    }
-    __syncthreads();
-    const int r = tid % NB, c0 = tid / NB;  // columns c0 + 4i
-    double re[NB / 4], im[NB / 4];
-#pragma unroll
-    for (int i = 0; i < NB / 4; ++i) re[i] = im[i] = 0.0;
-    for (int q = 0; q < NB; ++q) {
-        const float2 d = Ds[r][q];
-#pragma unroll
-        for (int i = 0; i < NB / 4; ++i) {
-            const float2 f = Fs[q][c0 + 4 * i];
-            re[i] += (double)d.x * f.x - (double)d.y * f.y;
-            im[i] += (double)d.x * f.y + (double)d.y * f.x;
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < NB / 4; ++i) out[r + (c0 + 4 * i) * NB] = make_float2((float)re[i], (float)im[i]);
-}
-
 // An FP64 complex sum as four chains of fused multiply-adds.
 struct CSum {
     double rr = 0.0, ii = 0.0, ri = 0.0, ir = 0.0;
@@ -1656,6 +1610,60 @@ struct CSum {
     __device__ __forceinline__ double re() const { return rr - ii; }
     __device__ __forceinline__ double im() const { return ri + ir; }
 };
+
+// Coupling products for trsv_fold_kernel: for sub-block k and its
+// neighbours at distance d in solve order (lower: k - d, upper: k + d),
+// Pd[k] = Dinv_k F(k, k -/+ d), F the factor (W or its conjugate transpose;
+// rows and columns beyond np read as zero), Dinv_k the sub-block's inverse
+// (NB x NB column-major). grid (nsb, D, NB / CO_COLS): blockIdx.y + 1 is d (zero where
+// the neighbour does not exist), blockIdx.z a chunk of the product's columns;
+// P = P1 (nsb blocks), P2, .., each NB x NB column-major complex64, accumulated in
+// FP64. Latency: one CTA per product took 27 us however small the system,
+// 7.5 us with four.
+constexpr int CO_COLS = NB / 4;
+__global__ void __launch_bounds__(256) trsv_couple_kernel(const float2* __restrict__ M, int64_t ldm, int64_t np,
+                                                          int nsb, int lower, const float2* __restrict__ Dinv,
+                                                          float2* __restrict__ P) {
+    constexpr int PER_D = NB * NB / 256, PER_F = NB * CO_COLS / 256;
+    __shared__ float2 Ds[NB][NB + 1];       // [row][q]
+    __shared__ float2 Fs[CO_COLS][NB + 1];  // [col][q]
+    const int k = blockIdx.x, dist = blockIdx.y + 1, col0 = blockIdx.z * CO_COLS;
+    const int nb = lower ? k - dist : k + dist;  // neighbour sub-block
+    float2* out = P + ((size_t)blockIdx.y * nsb + k) * NB * NB + col0 * NB;
+    const int tid = threadIdx.x;
+    if (nb < 0 || nb >= nsb) {
+        for (int e = tid; e < NB * CO_COLS; e += 256) out[e] = make_float2(0.f, 0.f);
+        return;
+    }
+    float2 d[PER_D], f[PER_F];
+#pragma unroll
+    for (int u = 0; u < PER_D; ++u) d[u] = Dinv[(size_t)k * NB * NB + tid + 256 * u];
+#pragma unroll
+    for (int u = 0; u < PER_F; ++u) {
+        const int e = tid + 256 * u;  // rows fastest: coalesced columns
+        const int64_t gr = (int64_t)k * NB + e % NB, gc = (int64_t)nb * NB + col0 + e / NB;
+        f[u] = (gr < np && gc < np) ? M[gr + gc * ldm] : make_float2(0.f, 0.f);
+    }
+#pragma unroll
+    for (int u = 0; u < PER_D; ++u) Ds[(tid + 256 * u) % NB][(tid + 256 * u) / NB] = d[u];
+#pragma unroll
+    for (int u = 0; u < PER_F; ++u) Fs[(tid + 256 * u) / NB][(tid + 256 * u) % NB] = f[u];
+    __syncthreads();
+    const int r = tid % NB, c0 = tid / NB;  // columns c0 + 4i
+    CSum acc[CO_COLS / 4];
+#pragma unroll 8
+    for (int q = 0; q < NB; ++q) {
+        const float2 w = Ds[r][q];
+#pragma unroll
+        for (int i = 0; i < CO_COLS / 4; ++i) {
+            const float2 v = Fs[c0 + 4 * i][q];
+            acc[i].add(w, cx(v.x, v.y));
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < CO_COLS / 4; ++i)
+        out[r + (c0 + 4 * i) * NB] = make_float2((float)acc[i].re(), (float)acc[i].im());
+}
 
 // trsv_tma_kernel for 128-row CTAs with the coupling to the newest
 // sub-block folded into precomputed products (trsv_couple_kernel). A CTA's
@@ -1971,12 +1979,17 @@ __global__ void dot_partial_kernel(int64_t n, int k, const cplx* __restrict__ V,
     }
 }
 
+// h[j] = sum of the parts of column j, a warp per column: a thread adding
+// them one after the other took 6.2 us per launch, this 1.9 us.
 __global__ void dot_finish_kernel(int k, int parts, const cplx* __restrict__ partial, cplx* __restrict__ h) {
-    const int j = threadIdx.x;
-    if (j >= k) return;
+    const int j = blockIdx.x, lane = threadIdx.x;
     cplx s = cx(0, 0);
-    for (int p = 0; p < parts; ++p) s += partial[(int64_t)p * k + j];
-    h[j] = s;
+    for (int p = lane; p < parts; p += 32) s += partial[(int64_t)p * k + j];
+    for (int o = 16; o > 0; o >>= 1) {
+        s.re += __shfl_xor_sync(0xffffffffu, s.re, o);
+        s.im += __shfl_xor_sync(0xffffffffu, s.im, o);
+    }
+    if (lane == 0) h[j] = s;
 }
 
 // w -= V[:, 0:k] h
@@ -2859,8 +2872,6 @@ static int apply_precond(DenseSolver* s, const cplx* r, cplx* z, cplx* work, boo
                                            trsv_smem(NB)));
         SIEB_TRY_CUDA(cudaFuncSetAttribute(trsv_fold_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            kSmemTrsvFold));
-        SIEB_TRY_CUDA(cudaFuncSetAttribute(trsv_couple_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           kSmemCouple));
         attr_set = true;
     }
     const unsigned ncta = (unsigned)((np + rows - 1) / rows);
@@ -2877,7 +2888,7 @@ static int apply_precond(DenseSolver* s, const cplx* r, cplx* z, cplx* work, boo
         SIEB_RETURN_IF(s->couple.reserve(sizeof(float2) * per_dir * 4));
         for (int lower = 1; lower >= 0; --lower) {
             const float2* dinv = adjoint ? (lower ? st->UinvH : st->LinvH) : (lower ? st->Linv : st->Uinv);
-            trsv_couple_kernel<<<dim3((unsigned)nbl, 2), 256, kSmemCouple, stream>>>(
+            trsv_couple_kernel<<<dim3((unsigned)nbl, 2, NB / CO_COLS), 256, 0, stream>>>(
                 adjoint ? st->WH : st->W, st->ldw, np, nbl, lower, dinv, couple_of(lower));
             SIEB_NOTE_LAUNCH();
             SIEB_TRY_CUDA(cudaGetLastError());
@@ -3019,12 +3030,11 @@ static int gmres_ir(DenseSolver* s, cplx* b, int64_t ldb_unused, double tol, int
             // Classical Gram-Schmidt with one reorthogonalization (CGS2): the
             // two passes' coefficients (h, h + j + 1) and ||w||^2 (h + 2j + 2)
             // stay on the device and come back in one copy.
-            const int fin_threads = std::min(1024, ((j + 1 + 31) / 32) * 32);
             for (int pass = 0; pass < 2; ++pass) {
                 cplx* hp = h + pass * (j + 1);
                 dot_partial_kernel<<<dim3(parts, j + 1), 256, 0, stream>>>(n, j + 1, V, n, w, partial);
                 SIEB_NOTE_LAUNCH();
-                dot_finish_kernel<<<1, fin_threads, 0, stream>>>(j + 1, parts, partial, hp);
+                dot_finish_kernel<<<j + 1, 32, 0, stream>>>(j + 1, parts, partial, hp);
                 SIEB_NOTE_LAUNCH();
                 axpy_multi_kernel<<<blocks_for(n, 256), 256, 0, stream>>>(n, j + 1, V, n, hp, w);
                 SIEB_NOTE_LAUNCH();
