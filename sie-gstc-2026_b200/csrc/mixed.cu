@@ -2121,6 +2121,76 @@ __global__ void __launch_bounds__(256) fp64_diag_apply_kernel(cplx* __restrict__
     }
 }
 
+// Own FP64 LU, few right-hand sides: one block step of a triangular solve in
+// one launch, for FS_COLS columns per blockIdx.y. X_k = Inv_k Y_k is formed by every CTA
+// for itself (CTA 0 writes it to X, another buffer: Y_k is still being read),
+// then CTA b takes Y(rows) -= W(rows, k) X_k for its 64 rows, r_begin + 64 b
+// up to r_end. Bound: latency; all of a thread's loads of both matrices go
+// out before anything waits. Against a diagonal kernel and a tiled GEMM per
+// step (3.5 + 19 us for three columns, most of the GEMM's 64-column tiles empty)
+// 4.6 us (2940 unknowns).
+constexpr int FS_COLS = 4;
+__global__ void __launch_bounds__(256) fp64_step_kernel(const cplx* __restrict__ W, int64_t ldw, int64_t k0, int kb,
+                                                        int64_t r_begin, int64_t r_end,
+                                                        const double2* __restrict__ Inv, cplx* Y,
+                                                        cplx* __restrict__ X, int64_t ldy, int nrhs) {
+    static_assert(NB == 64 && FS_COLS == 4, "256 threads: a row and a quarter of the columns each, then a row and a column");
+    __shared__ cplx v[FS_COLS][NB];      // Y_k, then X_k
+    __shared__ cplx red[4][FS_COLS][NB];
+    const int r = threadIdx.x & (NB - 1), p = threadIdx.x >> 6;
+    const int gc = blockIdx.y * FS_COLS + p;  // this thread's column in the second role
+    const int64_t row = r_begin + (int64_t)blockIdx.x * NB + r;
+    double2 inv[16];
+    cplx w[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) inv[u] = __ldg(&Inv[r + (16 * p + u) * NB]);  // column-major
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+        const int q = 16 * p + u;
+        w[u] = (row < r_end && q < kb) ? W[row + (k0 + q) * ldw] : cx(0, 0);
+    }
+    const bool mine = row < r_end && gc < nrhs;
+    const cplx old = mine ? Y[row + (int64_t)gc * ldy] : cx(0, 0);
+    v[p][r] = (gc < nrhs && r < kb) ? Y[(k0 + r) + (int64_t)gc * ldy] : cx(0, 0);
+    __syncthreads();
+    auto sum = [&]() {
+        return cx((red[0][p][r].re + red[1][p][r].re) + (red[2][p][r].re + red[3][p][r].re),
+                  (red[0][p][r].im + red[1][p][r].im) + (red[2][p][r].im + red[3][p][r].im));
+    };
+#pragma unroll
+    for (int c = 0; c < FS_COLS; ++c) {
+        double re = 0.0, im = 0.0;
+#pragma unroll
+        for (int u = 0; u < 16; ++u) {
+            const cplx y = v[c][16 * p + u];
+            re = fma(inv[u].x, y.re, fma(-inv[u].y, y.im, re));
+            im = fma(inv[u].x, y.im, fma(inv[u].y, y.re, im));
+        }
+        red[p][c][r] = cx(re, im);
+    }
+    __syncthreads();
+    const cplx xk = r < kb ? sum() : cx(0, 0);
+    v[p][r] = xk;
+    if (blockIdx.x == 0 && gc < nrhs && r < kb) X[(k0 + r) + (int64_t)gc * ldy] = xk;
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < FS_COLS; ++c) {
+        double re = 0.0, im = 0.0;
+#pragma unroll
+        for (int u = 0; u < 16; ++u) {
+            const cplx y = v[c][16 * p + u];
+            re = fma(w[u].re, y.re, fma(-w[u].im, y.im, re));
+            im = fma(w[u].re, y.im, fma(w[u].im, y.re, im));
+        }
+        red[p][c][r] = cx(re, im);
+    }
+    __syncthreads();
+    if (mine) {
+        const cplx d = sum();
+        Y[row + (int64_t)gc * ldy] = cx(old.re - d.re, old.im - d.im);
+    }
+}
+
 // X(:, c) += D(:, c)
 __global__ void add_cols_kernel(int64_t n, const cplx* __restrict__ D, int64_t ldd, cplx* __restrict__ X,
                                 int64_t ldx) {
@@ -3311,11 +3381,38 @@ static int fp64_factorize(DenseSolver* s) {
     return SIEB200_OK;
 }
 
-// Y (np x nrhs, ldy) <- W^{-1} Y with the complex128 factors.
-static int fp64_triangular(DenseSolver* s, MixedState* st, cplx* Y, int64_t ldy, int nrhs) {
+// Up to this many right-hand sides fp64_triangular runs one kernel per block
+// step (fp64_step_kernel, FS_COLS columns per CTA, every CTA reading its
+// block of W for them); above, a diagonal kernel and a GEMM over all columns.
+// Both solves with 16 columns against the GEMM form with 17: 0.63 and 2.34 ms
+// at 2940 unknowns, 1.73 and 4.79 ms at 6000, growing by 0.2 ms for every
+// four columns there; the GEMM form's time is the same up to 64 columns. The
+// line leaves a margin for larger systems, whose blocks of W are read again
+// from L2.
+constexpr int kFp64StepCols = 32;
+
+// Y (np x nrhs, ldy) <- W^{-1} Y with the complex128 factors; T: np x nrhs
+// scratch (ldy) when nrhs <= kFp64StepCols.
+static int fp64_triangular(DenseSolver* s, MixedState* st, cplx* Y, cplx* T, int64_t ldy, int nrhs) {
     cudaStream_t stream = s->ctx->stream;
     const int64_t np = st->np, nbl = st->nbl, ldw = st->ldw;
     const cplx* W = reinterpret_cast<const cplx*>(st->W64);
+    if (nrhs <= kFp64StepCols) {
+        for (int lower = 1; lower >= 0; --lower) {
+            for (int64_t t = 0; t < nbl; ++t) {
+                const int64_t k = lower ? t : nbl - 1 - t, k0 = k * NB;
+                const int kb = (int)std::min<int64_t>(NB, np - k0);
+                const int64_t r0 = lower ? k0 + kb : 0, r1 = lower ? np : k0;  // rows updated
+                const dim3 grid(std::max(1u, blocks_for(r1 - r0, NB)), blocks_for(nrhs, FS_COLS));
+                const double2* inv = (lower ? st->Linv64 : st->Uinv64) + (size_t)k * NB * NB;
+                fp64_step_kernel<<<grid, 256, 0, stream>>>(W, ldw, k0, kb, r0, r1, inv, lower ? Y : T, lower ? T : Y,
+                                                           ldy, nrhs);
+                SIEB_NOTE_LAUNCH();
+                SIEB_TRY_CUDA(cudaGetLastError());
+            }
+        }
+        return SIEB200_OK;
+    }
     const unsigned g = blocks_for(nrhs, 16);
     for (int64_t k = 0; k < nbl; ++k) {
         const int64_t k0 = k * NB;
@@ -3351,13 +3448,15 @@ static int fp64_solve(DenseSolver* s, int64_t nrhs64, double* Bd, int64_t ldb, d
     const int64_t ldy = ((np + 31) / 32) * 32;
     if (!(tol > 0)) tol = 1e-10;
     if (maxit <= 0) maxit = 5;
-    // Y (ldy x nrhs) | X | R | B0 (n x nrhs each)
+    // Y (ldy x nrhs) | X | R | B0 (n x nrhs each) | T (ldy x nrhs, few columns)
     const size_t blk = (size_t)n * nrhs;
-    SIEB_RETURN_IF(s->krylov.reserve(sizeof(cplx) * ((size_t)ldy * nrhs + 3 * blk)));
+    const size_t t_entries = nrhs <= kFp64StepCols ? (size_t)ldy * nrhs : 0;
+    SIEB_RETURN_IF(s->krylov.reserve(sizeof(cplx) * ((size_t)ldy * nrhs + 3 * blk + t_entries)));
     cplx* Y = s->krylov.as<cplx>();
     cplx* X = Y + (size_t)ldy * nrhs;
     cplx* R = X + blk;
     cplx* B0 = R + blk;
+    cplx* T = B0 + blk;
     cplx* B = reinterpret_cast<cplx*>(Bd);
     const dim3 gv(blocks_for(n, 256), (unsigned)nrhs);
     copy_cols_kernel<<<gv, 256, 0, stream>>>(n, B, ldb, B0, n);
@@ -3390,7 +3489,7 @@ static int fp64_solve(DenseSolver* s, int64_t nrhs64, double* Bd, int64_t ldb, d
         }
         cudaEvent_t ev;
         ctx->prof.begin(stream, 1, 0.0, 16.0 * (double)np * np, &ev);
-        SIEB_RETURN_IF(fp64_triangular(s, st, Y, ldy, nrhs));
+        SIEB_RETURN_IF(fp64_triangular(s, st, Y, T, ldy, nrhs));
         ctx->prof.end(stream, ev);
         for (int c = 0; c < nrhs; ++c) {
             rbt_vec_N_kernel<<<blocks_for(q, 256), 256, 0, stream>>>(Y + (size_t)c * ldy, n, np, st->diag + 4 * np,

@@ -32,3 +32,24 @@ def test_fp64_lu_groups(gpu_ctx, monkeypatch, n, dmma):
     ref = np.linalg.solve(A, B)
     assert np.linalg.norm(X.cpu().numpy().T - ref) <= 2e-12 * np.linalg.norm(ref)
     s.close()
+
+
+@pytest.mark.parametrize("n,nrhs", [(n, c) for n in (7, 64, 130, 323) for c in (1, 4, 5, 32, 33)] + [(1300, 33)])
+def test_fp64_triangular_columns(gpu_ctx, n, nrhs):
+    """Column counts around a CTA's columns of the one-kernel step and around
+    the count above which a diagonal kernel and a GEMM take over."""
+    import torch
+    import sieb200
+    rng = np.random.default_rng(1000 * n + nrhs)
+    A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)) + 4.0 * np.sqrt(n) * np.eye(n)
+    B = rng.standard_normal((n, nrhs)) + 1j * rng.standard_normal((n, nrhs))
+    Z = torch.from_numpy(A.T.copy()).cuda()
+    X = torch.from_numpy(B.T.copy()).cuda()
+    torch.cuda.synchronize()
+    s = sieb200.DenseLuSolver(n, "lu_fp64", ctx=gpu_ctx)
+    s.factorize(Z.data_ptr())
+    s.solve(X.data_ptr(), nrhs=nrhs, tolerance=1e-13, max_iterations=2)
+    gpu_ctx.synchronize()
+    ref = np.linalg.solve(A, B)
+    assert np.linalg.norm(X.cpu().numpy().T - ref) <= 2e-12 * np.linalg.norm(ref)
+    s.close()
