@@ -2191,12 +2191,12 @@ __global__ void __launch_bounds__(256) fp64_step_kernel(const cplx* __restrict__
     }
 }
 
-// X(:, c) += D(:, c)
-__global__ void add_cols_kernel(int64_t n, const cplx* __restrict__ D, int64_t ldd, cplx* __restrict__ X,
+// X(:, c) += s D(:, c)
+__global__ void add_cols_kernel(int64_t n, const cplx* __restrict__ D, int64_t ldd, double s, cplx* __restrict__ X,
                                 int64_t ldx) {
     const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int c = blockIdx.y;
-    if (r < n) X[r + c * ldx] += D[r + c * ldd];
+    if (r < n) X[r + c * ldx] += D[r + c * ldd] * s;
 }
 
 // Y(:, c) = X(:, c) (rectangular copy between leading dimensions)
@@ -3391,6 +3391,13 @@ static int fp64_factorize(DenseSolver* s) {
 // from L2.
 constexpr int kFp64StepCols = 32;
 
+// The refinement's residual as one matvec per column, each at the rate Z
+// comes from memory (34 us a column at 2940 unknowns, 95 at 6000), or as one
+// GEMM, a CTA per 64 rows with all of K (0.46 and 0.93 ms however few the
+// columns): up to about 13 and 9 columns the matvecs are faster, and the line falls
+// as 1/n, n^2 bytes a column against a loop over n.
+static bool fp64_residual_by_column(int64_t n, int64_t nrhs) { return nrhs == 1 || nrhs * n <= 40000; }
+
 // Y (np x nrhs, ldy) <- W^{-1} Y with the complex128 factors; T: np x nrhs
 // scratch (ldy) when nrhs <= kFp64StepCols.
 static int fp64_triangular(DenseSolver* s, MixedState* st, cplx* Y, cplx* T, int64_t ldy, int nrhs) {
@@ -3479,6 +3486,8 @@ static int fp64_solve(DenseSolver* s, int64_t nrhs64, double* Bd, int64_t ldb, d
                    "right-hand side norm must be finite and nonzero");
     }
     int it = 0;
+    double sign = 1.0;  // of the residual in R
+    const bool by_column = fp64_residual_by_column(n, nrhs);
     std::vector<cplx> hr(blk);
     for (;;) {
         // correction D = V W^{-1} U^T R, X += D
@@ -3496,16 +3505,24 @@ static int fp64_solve(DenseSolver* s, int64_t nrhs64, double* Bd, int64_t ldb, d
                                                                      R + (size_t)c * n);
             SIEB_NOTE_LAUNCH();
         }
-        add_cols_kernel<<<gv, 256, 0, stream>>>(n, R, n, X, n);
+        add_cols_kernel<<<gv, 256, 0, stream>>>(n, R, n, sign, X, n);
         SIEB_NOTE_LAUNCH();
         ++it;
-        // R = B - A X in FP64 against the intact matrix
+        // The residual in FP64 against the intact matrix: R = B - A X, or, column by column,
+        // A X - B (the next correction is then subtracted).
         copy_cols_kernel<<<gv, 256, 0, stream>>>(n, B0, n, R, n);
         SIEB_NOTE_LAUNCH();
-        ctx->prof.begin(stream, 2, 8.0 * (double)n * n * nrhs, 16.0 * (double)n * n, &ev);
-        SIEB_RETURN_IF(zgemm_device(stream, n, nrhs, n, reinterpret_cast<const cplx*>(s->A), s->lda, X, n, R, n,
-                                    cx(-1, 0), cx(1, 0)));
-        ctx->prof.end(stream, ev);
+        if (by_column) {
+            for (int c = 0; c < nrhs; ++c)
+                SIEB_RETURN_IF(gemv_device(ctx, n, s->A, s->lda, 0, X + (size_t)c * n, -1.0, R + (size_t)c * n,
+                                           s->gemv_scratch));
+            sign = -1.0;
+        } else {
+            ctx->prof.begin(stream, 2, 8.0 * (double)n * n * nrhs, 16.0 * (double)n * n, &ev);
+            SIEB_RETURN_IF(zgemm_device(stream, n, nrhs, n, reinterpret_cast<const cplx*>(s->A), s->lda, X, n, R, n,
+                                        cx(-1, 0), cx(1, 0)));
+            ctx->prof.end(stream, ev);
+        }
         SIEB_TRY_CUDA(cudaMemcpyAsync(hr.data(), R, sizeof(cplx) * blk, cudaMemcpyDeviceToHost, stream));
         SIEB_TRY_CUDA(cudaStreamSynchronize(stream));
         bool done = true;
