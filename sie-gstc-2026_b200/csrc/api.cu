@@ -471,7 +471,7 @@ int solve_dense_common(sieb200_ctx* ctx, const sieb200_mesh* mesh, const sieb200
             SIEB_RETURN_IF(Rb.reserve(sizeof(cplx) * N * ncols));
             SIEB_TRY_CUDA(cudaMemcpyAsync(Rb.ptr, hb.data(), sizeof(cplx) * N * ncols, cudaMemcpyHostToDevice, st));
             SIEB_RETURN_IF(zgemm_device(st, N, ncols, N, reinterpret_cast<const cplx*>(Zr), N, Bb.as<cplx>(), N,
-                                        Rb.as<cplx>(), N, cx(-1, 0), cx(1, 0)));
+                                        Rb.as<cplx>(), N, cx(-1, 0), cx(1, 0), &scratch));
             std::vector<double> hR(2 * N * ncols);
             SIEB_TRY_CUDA(cudaMemcpyAsync(hR.data(), Rb.ptr, sizeof(cplx) * N * ncols, cudaMemcpyDeviceToHost, st));
             SIEB_TRY_CUDA(cudaStreamSynchronize(st));

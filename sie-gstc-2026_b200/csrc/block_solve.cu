@@ -481,6 +481,7 @@ __global__ void bcopy_kernel(int64_t n, const cplx* __restrict__ X, int64_t ldx,
 // Shared layouts: A as [k][row] with rows padded to 66 (conflict-free
 // 16-byte fragment loads), X as [col][k] with k padded to 20.
 constexpr int ZD_BM = 64, ZD_BN = 64, ZD_BK = 16, ZD_THREADS = 128, ZD_STAGES = 3;
+constexpr int kSms = 148;
 constexpr int ZD_ALD = ZD_BM + 2, ZD_XLD = ZD_BK + 4;
 constexpr int ZD_STAGE_A = ZD_BK * ZD_ALD, ZD_STAGE_X = ZD_BN * ZD_XLD;  // complex entries
 constexpr int kSmemZgemmDmma = ZD_STAGES * (ZD_STAGE_A + ZD_STAGE_X) * 16;
@@ -502,13 +503,15 @@ __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
 
 // TRAILING: the trailing update of the FP64 factorization (zgemm_trailing), a
 // one-dimensional grid over the tiles of the first `strip` tile columns and,
-// right of them, the first `strip` tile rows, without tile (0, 0).
+// right of them, the first `strip` tile rows, without tile (0, 0). Otherwise CTA z
+// takes the products k = z kc .. z kc + kc - 1 into its own C, cz entries further.
 template <bool TRAILING>
 __global__ void __launch_bounds__(ZD_THREADS, 2) zgemm_dmma_kernel(int64_t m, int64_t nc, int64_t kdim,
                                                                    const double2* __restrict__ A, int64_t lda,
                                                                    const double2* __restrict__ X, int64_t ldx,
                                                                    double2* __restrict__ C, int64_t ldc,
-                                                                   double2 alpha, double2 beta, int strip) {
+                                                                   double2 alpha, double2 beta, int strip,
+                                                                   int64_t kc, int64_t cz) {
     extern __shared__ __align__(16) double2 zd_smem[];
     double2* As = zd_smem;                                // [stage][k][ZD_ALD]
     double2* Xs = zd_smem + ZD_STAGES * ZD_STAGE_A;       // [stage][col][ZD_XLD]
@@ -523,6 +526,12 @@ __global__ void __launch_bounds__(ZD_THREADS, 2) zgemm_dmma_kernel(int64_t m, in
             tr = (t - mt * strip) % strip;
             tc = strip + (t - mt * strip) / strip;
         }
+    } else {
+        const int64_t z0 = (int64_t)blockIdx.z * kc;
+        A += z0 * lda;
+        X += z0;
+        C += (int64_t)blockIdx.z * cz;
+        kdim = min(kc, kdim - z0);
     }
     const int64_t row0 = (int64_t)tr * ZD_BM, col0 = (int64_t)tc * ZD_BN;
     const int wr = (warp & 1) * 32, wc = (warp >> 1) * 32;  // warp tile origin in the CTA tile
@@ -648,6 +657,21 @@ __global__ void __launch_bounds__(ZD_THREADS, 2) zgemm_dmma_kernel(int64_t m, in
     }
 }
 
+// C = alpha sum_z P_z + beta C, P_z the m x nc partial products one after the other.
+__global__ void __launch_bounds__(256) zgemm_finish_kernel(int64_t m, int64_t nc, int parts,
+                                                           const cplx* __restrict__ P, cplx* __restrict__ C,
+                                                           int64_t ldc, cplx alpha, cplx beta) {
+    const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (e >= m * nc) return;
+    cplx* c = &C[e % m + (e / m) * ldc];
+    cplx s = cx(0, 0);
+#pragma unroll 4
+    for (int z = 0; z < parts; ++z) s += P[e + (int64_t)z * m * nc];
+    s = alpha * s;
+    if (beta.re != 0.0 || beta.im != 0.0) s += beta * *c;
+    *c = s;
+}
+
 inline unsigned nblk(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
 }  // namespace
@@ -674,7 +698,7 @@ static int zgemm_dmma_attributes() {
 // C = alpha A X + beta C (FP64 complex, column-major). Exposed for the
 // residual of the batched refinement and its tests.
 int zgemm_device(cudaStream_t stream, int64_t m, int64_t nc, int64_t kdim, const cplx* A, int64_t lda,
-                 const cplx* X, int64_t ldx, cplx* C, int64_t ldc, cplx alpha, cplx beta) {
+                 const cplx* X, int64_t ldx, cplx* C, int64_t ldc, cplx alpha, cplx beta, DeviceBuffer* scratch) {
     if (m <= 0 || nc <= 0) return SIEB200_OK;
     SIEB_CHECK(nc < 65536ll * ZG_BN && m < (1ll << 40), SIEB200_INVALID_ARG, "zgemm: size out of range");
     // The tensor-core kernel needs 16-byte aligned operands (cp.async of one
@@ -683,10 +707,33 @@ int zgemm_device(cudaStream_t stream, int64_t m, int64_t nc, int64_t kdim, const
                            reinterpret_cast<uintptr_t>(C)) & 15) == 0;
     if (zgemm_dmma_selected() && aligned && nc < 65536ll * ZD_BN) {
         SIEB_RETURN_IF(zgemm_dmma_attributes());
-        const dim3 grid(nblk(m, ZD_BM), nblk(nc, ZD_BN));
+        dim3 grid(nblk(m, ZD_BM), nblk(nc, ZD_BN));
+        // Few tiles leave SMs idle (two CTAs fit on one): given a scratch
+        // buffer, K is then split over blockIdx.z, at least 128 products each,
+        // and the partial products are added in order. Up to 64 columns,
+        // unsplit and split: K = 1920 300 and 75 us, 2940 463 and 150 us,
+        // 6000 933 and 562 us.
+        const int64_t tiles = (int64_t)grid.x * grid.y;
+        const int64_t parts = scratch ? std::min<int64_t>({16, 2 * kSms / tiles, kdim / 128}) : 1;
+        if (parts >= 2) {
+            const int64_t kc = ((kdim + parts - 1) / parts + ZD_BK - 1) / ZD_BK * ZD_BK;
+            grid.z = (unsigned)((kdim + kc - 1) / kc);
+            SIEB_RETURN_IF(scratch->reserve(sizeof(cplx) * (size_t)m * nc * grid.z));
+            zgemm_dmma_kernel<false><<<grid, ZD_THREADS, kSmemZgemmDmma, stream>>>(
+                m, nc, kdim, reinterpret_cast<const double2*>(A), lda, reinterpret_cast<const double2*>(X), ldx,
+                scratch->as<double2>(), m, make_double2(1.0, 0.0), make_double2(0.0, 0.0), 0, kc, m * nc);
+            SIEB_NOTE_LAUNCH();
+            SIEB_TRY_CUDA(cudaGetLastError());
+            zgemm_finish_kernel<<<nblk(m * nc, 256), 256, 0, stream>>>(m, nc, (int)grid.z, scratch->as<cplx>(), C, ldc,
+                                                                      alpha, beta);
+            SIEB_NOTE_LAUNCH();
+            SIEB_TRY_CUDA(cudaGetLastError());
+            return SIEB200_OK;
+        }
         zgemm_dmma_kernel<false><<<grid, ZD_THREADS, kSmemZgemmDmma, stream>>>(
             m, nc, kdim, reinterpret_cast<const double2*>(A), lda, reinterpret_cast<const double2*>(X), ldx,
-            reinterpret_cast<double2*>(C), ldc, make_double2(alpha.re, alpha.im), make_double2(beta.re, beta.im), 0);
+            reinterpret_cast<double2*>(C), ldc, make_double2(alpha.re, alpha.im), make_double2(beta.re, beta.im), 0,
+            kdim, 0);
         SIEB_NOTE_LAUNCH();
         SIEB_TRY_CUDA(cudaGetLastError());
         return SIEB200_OK;
@@ -718,7 +765,8 @@ int zgemm_trailing(cudaStream_t stream, int64_t m, int64_t w, int64_t kdim, cons
         SIEB_RETURN_IF(zgemm_dmma_attributes());
         zgemm_dmma_kernel<true><<<(unsigned)(mt * wt + wt * (mt - wt) - 1), ZD_THREADS, kSmemZgemmDmma, stream>>>(
             m, m, kdim, reinterpret_cast<const double2*>(A), lda, reinterpret_cast<const double2*>(X), ldx,
-            reinterpret_cast<double2*>(C), ldc, make_double2(-1.0, 0.0), make_double2(1.0, 0.0), (int)wt);
+            reinterpret_cast<double2*>(C), ldc, make_double2(-1.0, 0.0), make_double2(1.0, 0.0), (int)wt, kdim,
+            0);
         SIEB_NOTE_LAUNCH();
         SIEB_TRY_CUDA(cudaGetLastError());
         return SIEB200_OK;
@@ -1027,7 +1075,7 @@ int block_solve(DenseSolver* s, MixedState* st, int64_t nrhs64, double* Bd, int6
             cudaEvent_t ev;
             ctx->prof.begin(stream, 2, 8.0 * (double)n * n * nrhs, 16.0 * (double)n * n, &ev);
             SIEB_RETURN_IF(zgemm_device(stream, n, nrhs, n, reinterpret_cast<const cplx*>(s->A), s->lda, X, n, R, n,
-                                        cx(-1, 0), cx(1, 0)));
+                                        cx(-1, 0), cx(1, 0), &s->gemv_scratch));
             ctx->prof.end(stream, ev);
         }
         bdot_kernel<<<dim3((unsigned)nrhs, 1), 256, 0, stream>>>(n, nrhs, R, 0, n, R, n, hd);
@@ -1064,7 +1112,7 @@ int block_solve(DenseSolver* s, MixedState* st, int64_t nrhs64, double* Bd, int6
             cudaEvent_t ev;
             ctx->prof.begin(stream, 2, 8.0 * (double)n * n * nrhs, 16.0 * (double)n * n, &ev);
             SIEB_RETURN_IF(zgemm_device(stream, n, nrhs, n, reinterpret_cast<const cplx*>(s->A), s->lda, zj, n, W, n,
-                                        cx(1, 0), cx(0, 0)));
+                                        cx(1, 0), cx(0, 0), &s->gemv_scratch));
             ctx->prof.end(stream, ev);
             // CGS2
             std::vector<cplx> hsum((size_t)(j + 1) * nrhs, cx(0, 0));

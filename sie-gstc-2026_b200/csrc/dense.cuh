@@ -58,10 +58,11 @@ int fp64_mma_rate(sieb200_ctx* ctx, double* tflops);
 int gemv_device_static_scratch(sieb200_ctx* ctx, int64_t n, const void* A, int64_t lda, int prec,
                                const cplx* x, double beta, cplx* y);
 void destroy_cusolver(sieb200_ctx* ctx);
-// C = alpha A X + beta C, FP64 complex column-major (hand-written SIMT kernel,
-// block_solve.cu).
+// C = alpha A X + beta C, FP64 complex column-major (block_solve.cu). scratch
+// (optional, ordered on the same stream) lets a product with few tiles split its K.
 int zgemm_device(cudaStream_t stream, int64_t m, int64_t nc, int64_t kdim, const cplx* A, int64_t lda,
-                 const cplx* X, int64_t ldx, cplx* C, int64_t ldc, cplx alpha, cplx beta);
+                 const cplx* X, int64_t ldx, cplx* C, int64_t ldc, cplx alpha, cplx beta,
+                 DeviceBuffer* scratch = nullptr);
 int zgemm_trailing(cudaStream_t stream, int64_t m, int64_t w, int64_t kdim, const cplx* A, int64_t lda, const cplx* X,
                    int64_t ldx, cplx* C, int64_t ldc);
 

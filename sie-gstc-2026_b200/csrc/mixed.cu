@@ -3391,12 +3391,11 @@ static int fp64_factorize(DenseSolver* s) {
 // from L2.
 constexpr int kFp64StepCols = 32;
 
-// The refinement's residual as one matvec per column, each at the rate Z
-// comes from memory (34 us a column at 2940 unknowns, 95 at 6000), or as one
-// GEMM, a CTA per 64 rows with all of K (0.46 and 0.93 ms however few the
-// columns): up to about 13 and 9 columns the matvecs are faster, and the line falls
-// as 1/n, n^2 bytes a column against a loop over n.
-static bool fp64_residual_by_column(int64_t n, int64_t nrhs) { return nrhs == 1 || nrhs * n <= 40000; }
+// Up to this many right-hand sides the refinement's residual is one matvec
+// per column, each at the rate Z comes from memory (18, 34 and 95 us at 1920,
+// 2940 and 6000 unknowns), above it one GEMM, whose 64-column tiles take 75, 150 and
+// 562 us however few of the columns there are.
+constexpr int kFp64MatvecCols = 4;
 
 // Y (np x nrhs, ldy) <- W^{-1} Y with the complex128 factors; T: np x nrhs
 // scratch (ldy) when nrhs <= kFp64StepCols.
@@ -3487,7 +3486,7 @@ static int fp64_solve(DenseSolver* s, int64_t nrhs64, double* Bd, int64_t ldb, d
     }
     int it = 0;
     double sign = 1.0;  // of the residual in R
-    const bool by_column = fp64_residual_by_column(n, nrhs);
+    const bool by_column = nrhs <= kFp64MatvecCols;
     std::vector<cplx> hr(blk);
     for (;;) {
         // correction D = V W^{-1} U^T R, X += D
@@ -3520,7 +3519,7 @@ static int fp64_solve(DenseSolver* s, int64_t nrhs64, double* Bd, int64_t ldb, d
         } else {
             ctx->prof.begin(stream, 2, 8.0 * (double)n * n * nrhs, 16.0 * (double)n * n, &ev);
             SIEB_RETURN_IF(zgemm_device(stream, n, nrhs, n, reinterpret_cast<const cplx*>(s->A), s->lda, X, n, R, n,
-                                        cx(-1, 0), cx(1, 0)));
+                                        cx(-1, 0), cx(1, 0), &s->gemv_scratch));
             ctx->prof.end(stream, ev);
         }
         SIEB_TRY_CUDA(cudaMemcpyAsync(hr.data(), R, sizeof(cplx) * blk, cudaMemcpyDeviceToHost, stream));
