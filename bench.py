@@ -8,7 +8,7 @@ one x-polarised plane wave along +z. Synthetic: the mesh and excitation are
 generated here, the system is assembled by the library.
 
 A step is one solve of the assembled system: randomized-butterfly transform,
-complex64 LU with split-TF32 tensor-core trailing updates, FP64 GMRES
+complex64 LU with split-FP16 tensor-core trailing updates, FP64 GMRES
 refinement against the complex128 Z until the relative residual <= 1e-10.
 Z (576 MB) is resident in HBM and larger than L2 (126 MB), so no separate L2
 flush is needed between steps. The FP64 comparison is cusolverDnZgetrf +
@@ -46,29 +46,26 @@ C0 = 299792458.0
 METRIC = "solves/s mixed-prec+IR vs FP64 LU at rel.res≤1e-10 (1 B200); adjoint grads/s"
 WORKLOAD = ("T-PMCHWT dielectric sphere r=0.5 m, eps_r=4, mu_r=1, ka=pi; geodesic mesh 2000 faces / "
             "3000 RWG edges (N=6000); Dunavant rule 17; 1 plane-wave RHS")
-# DRAM bytes (read + write) per trailing-update launch, mean over the 92
+# DRAM bytes (read + write) per trailing-update launch, mean over the 93
 # launches of one factorization of this workload, from one ncu capture of
 # the trailing GEMM (dram__bytes_read.sum + dram__bytes_write.sum).
-GEMM_DRAM_BYTES_PER_LAUNCH = 158.4e6
+GEMM_DRAM_BYTES_PER_LAUNCH = 47.9e6
 # FP64 flops per Green evaluation (one point pair, one wavenumber) of the
-# T-PMCHWT regular pass, counted from the kernel's source with an FMA as 2:
-# the point-pair geometry shared by the two wavenumbers (distance, r_p.r_q,
-# r_p x r_q, weights: 23 flops, half each), the kernel values (11) and the
-# 8 TL + 10 TK complex moments (72); one sqrt, one reciprocal and one sincos
-# per evaluation are not counted.
-ASSEMBLY_FLOPS_PER_EVAL = 95
-# Rotated-testing (nTL / nTK) pair kernel: per wavenumber 15 flops of kernel
-# values and products with the weight, 30 for the 8 G-weighted and 44 for the
-# 11 g-weighted complex moments; 51 flops of point-pair geometry shared by the
-# two wavenumbers (FMA = 2; sqrt, reciprocal, sincos not counted).
-N_ASSEMBLY_FLOPS_PER_EVAL = 115
+# T-PMCHWT far-pair kernel, counted from its source with an FMA as 2: the
+# point-pair geometry and the reciprocal square root's refinement, shared by
+# the two wavenumbers (19 flops, half each), the phase factor (26), G and g
+# (9), the 4 TL sums over the source points (14) and the TK ones of both
+# wavenumbers together (16, half each). The folds over the test points are
+# per point, not per pair, and are not counted. With RWG testing a face
+# pair is evaluated once for both orders.
+ASSEMBLY_FLOPS_PER_EVAL = 66.5
+# Rotated testing accumulates the same sums over the source points (its folds
+# differ), once for each order of a face pair.
+N_ASSEMBLY_FLOPS_PER_EVAL = 66.5
 # FP64 flops per field evaluation (one observation point, one face, one
-# quadrature point) of the surface-field kernel, counted from its source with
-# an FMA as 2: G and grad G (26), then for each of the three half-RWG
-# functions rho (3), the L vector (36) and the K vector (36), plus the face's
-# edge-length scaling and E/H accumulation spread over the rule's 61 points
-# (~6); one sqrt, two divisions and one sincos are not counted.
-FIELDS_FLOPS_PER_EVAL = 257
+# quadrature point) of the surface-field kernel, counted the same way with one
+# wavenumber: geometry (19), phase (26), G and g (9), the L and K sums (28).
+FIELDS_FLOPS_PER_EVAL = 82
 
 
 def log(*a):
@@ -339,7 +336,10 @@ def measure(args, ctx, rank: int, world: int, local: int, barrier, max_over_rank
     ctx.synchronize()
     t_asm = time.perf_counter() - t0
     Q = 61 if args.rule == 17 else sieb200.lib().sieb200_quadrature_rule(args.rule, None, None)
-    evals = 2.0 * mesh.num_faces ** 2 * Q * Q  # Green evaluations (two wavenumbers)
+    # Green evaluations (two wavenumbers): every ordered face pair with rotated
+    # testing, every unordered one with RWG testing
+    evals_n = 2.0 * mesh.num_faces ** 2 * Q * Q
+    evals = mesh.num_faces * (mesh.num_faces + 1.0) * Q * Q
     fp64_peak = ctx.fp64_fma_peak()
     # The same system with rotated (n x RWG) testing, N-PMCHWT surface form:
     # nTL / nTK face-pair quadrature in place of TL / TK, same placement.
@@ -354,10 +354,10 @@ def measure(args, ctx, rank: int, world: int, local: int, barrier, max_over_rank
         "n_pmchwt": {
             "workload": "N-PMCHWT (n x RWG testing, surface nTL form) of the same sphere, rule 17",
             "assembly_seconds": t_asm_n, "t_pmchwt_assembly_seconds": t_asm,
-            "green_evals_per_s": evals / t_asm_n,
+            "green_evals_per_s": evals_n / t_asm_n,
             "roofline": {"bound": "fp64 pipe", "unit": "TFLOP/s", "flops_per_eval": N_ASSEMBLY_FLOPS_PER_EVAL,
-                         "achieved": evals * N_ASSEMBLY_FLOPS_PER_EVAL / t_asm_n / 1e12, "peak": fp64_peak,
-                         "frac": evals * N_ASSEMBLY_FLOPS_PER_EVAL / t_asm_n / 1e12 / fp64_peak},
+                         "achieved": evals_n * N_ASSEMBLY_FLOPS_PER_EVAL / t_asm_n / 1e12, "peak": fp64_peak,
+                         "frac": evals_n * N_ASSEMBLY_FLOPS_PER_EVAL / t_asm_n / 1e12 / fp64_peak},
         }
     }
     sieb200.assemble_matrix_device(mesh, opts, Z.data_ptr(), ctx=ctx)
@@ -412,11 +412,11 @@ def measure(args, ctx, rank: int, world: int, local: int, barrier, max_over_rank
     prof = {name: ctx.profile_read(i) for i, name in
             [(3, "diag_lu"), (4, "panels"), (6, "factorization"), (7, "refined_solve")]}
     # One more step with the per-launch timeline: the largest trailing update
-    # (block step 0) on its own, against its roofline.
+    # (the first group's) on its own, against its roofline.
     ctx.profile(True, timeline=True)
     step()
     ctx.synchronize()
-    first_gemm = next(((a, b2) for k, a, b2 in sorted(ctx.profile_timeline(), key=lambda v: v[1]) if k == 0), None)
+    longest_gemm = max(((a, b2) for k, a, b2 in ctx.profile_timeline() if k == 0), key=lambda v: v[1] - v[0], default=None)
     ctx.profile(False)
 
     # Accuracy of the mixed solution against the FP64 matrix.
@@ -568,32 +568,32 @@ def measure(args, ctx, rank: int, world: int, local: int, barrier, max_over_rank
         peaks = measured_peaks()
         gemm_s = gemm["ms"] / 1e3
         total_dev_s = t_prof
-        shares = {"tf32_gemm": gemm_s / total_dev_s, "trsv": trsv["ms"] / 1e3 / total_dev_s,
+        shares = {"trailing_gemm": gemm_s / total_dev_s, "trsv": trsv["ms"] / 1e3 / total_dev_s,
                   "fp64_matvec": gemv["ms"] / 1e3 / total_dev_s}
-        tf32_peak = peaks["bf16_tflops"] / 2.0
+        f16_peak = peaks["bf16_tflops"]  # FP16 operands run at the bf16 rate
         gemm_tflops = gemm["flops"] / gemm_s / 1e12 if gemm_s > 0 else 0.0
         gemm_gbs = gemm["bytes"] / gemm_s / 1e9 if gemm_s > 0 else 0.0
         # Which roof binds: the kernel's algorithmic intensity (flops per
         # byte of C read and written plus the packed operands) against the
         # ridge of the two measured peaks.
         intensity = gemm["flops"] / gemm["bytes"] if gemm["bytes"] else 0.0
-        ridge = tf32_peak * 1e12 / (peaks["hbm_gbs"] * 1e9)
+        ridge = f16_peak * 1e12 / (peaks["hbm_gbs"] * 1e9)
         hbm_bound = intensity < ridge
         roofline = {
-            "kernel": "gemm_tf32_sub_persistent_kernel (split-TF32 trailing update, tcgen05)",
+            "kernel": "gemm_f16_sub_kernel (split-FP16 trailing update, tcgen05)",
             "bound": "hbm" if hbm_bound else "tensor",
             "achieved": gemm_gbs if hbm_bound else gemm_tflops,
-            "peak": peaks["hbm_gbs"] if hbm_bound else tf32_peak,
+            "peak": peaks["hbm_gbs"] if hbm_bound else f16_peak,
             "unit": "GB/s" if hbm_bound else "TFLOP/s",
-            "frac": gemm_gbs / peaks["hbm_gbs"] if hbm_bound else gemm_tflops / tf32_peak,
+            "frac": gemm_gbs / peaks["hbm_gbs"] if hbm_bound else gemm_tflops / f16_peak,
             "intensity_flop_per_byte": intensity, "ridge_flop_per_byte": ridge,
-            "tensor_tflops_achieved": gemm_tflops, "tensor_peak_tflops": tf32_peak,
-            "tensor_frac": gemm_tflops / tf32_peak,
+            "tensor_tflops_achieved": gemm_tflops, "tensor_peak_tflops": f16_peak,
+            "tensor_frac": gemm_tflops / f16_peak,
             "traffic": GEMM_DRAM_BYTES_PER_LAUNCH,
-            "traffic_note": "mean dram read+write bytes per trailing-update launch, ncu over the 92 "
+            "traffic_note": "mean dram read+write bytes per trailing-update launch, ncu over the 93 "
                             "launches of one N=6000 factorization",
             "algorithmic_bytes_per_launch": gemm["bytes"] / gemm["launches"] if gemm["launches"] else None,
-            "peak_note": f"TF32 dense = {peaks['source']} bf16 {peaks['bf16_tflops']} TFLOP/s / 2",
+            "peak_note": f"FP16 dense = {peaks['source']} bf16 {peaks['bf16_tflops']} TFLOP/s",
             "launches": gemm["launches"], "hbm_gbs_achieved": gemm_gbs,
             "hbm_frac": gemm_gbs / peaks["hbm_gbs"], "time_share": shares,
             "trsv_gbs": trsv["bytes"] / (trsv["ms"] / 1e3) / 1e9 if trsv["ms"] > 0 else None,
@@ -601,14 +601,14 @@ def measure(args, ctx, rank: int, world: int, local: int, barrier, max_over_rank
             # mean device time per launch (ms) of the chain kernels and of the
             # two phases of a step (spans on the launching streams)
             "mean_ms": {k: (v["ms"] / v["launches"] if v["launches"] else None)
-                        for k, v in [("tf32_gemm", gemm), ("trsv", trsv), *prof.items()]},
-            "largest_launch": largest_launch_roofline(first_gemm, peaks, tf32_peak),
+                        for k, v in [("trailing_gemm", gemm), ("trsv", trsv), *prof.items()]},
+            "largest_launch": largest_launch_roofline(longest_gemm, peaks, f16_peak),
         }
         value = world * args.steps / t_mixed
         out = {
             "metric": METRIC, "value": value, "unit": "solves/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": 1e3 * t_mixed / args.steps, "higher_is_better": True,
-            "scaling": "weak", "vs_baseline": None, "dtype": "c64+tf32x3/c128", "data": "synthetic",
+            "scaling": "weak", "vs_baseline": None, "dtype": "c64+f16x3/c128", "data": "synthetic",
             "config": bench_config(world),
             "roofline": roofline, "cpu_baseline": cpu,
             "e2e": {"value": world * e2e_steps / t_e2e, "unit": "solves/s",
@@ -894,7 +894,7 @@ def multi_rhs_section(ctx, fp64_peak: float, max_over_ranks) -> dict:
     timed(mixed_step, 2)
     ctx.profile(True)
     mixed_step()
-    prof = {name: ctx.profile_read(i) for i, name in [(0, "tf32_gemm"), (2, "fp64_gemm"), (5, "block_trsm"),
+    prof = {name: ctx.profile_read(i) for i, name in [(0, "trailing_gemm"), (2, "fp64_gemm"), (5, "block_trsm"),
                                                       (6, "factorization"), (7, "refined_solve")]}
     ctx.profile(False)
     t_mixed = max_over_ranks(statistics.mean(timed(mixed_step, 3)))
@@ -986,7 +986,7 @@ def sweep_section(ctx, max_over_ranks) -> dict:
     t_seq = max_over_ranks(timings[1])
     t_best = max_over_ranks(timings[best])
     res, _ = sieb200.solve_gstc_sweep_batched(insts, concurrency=best, ctx=ctx)
-    flops = sum(8.0 * float(n) ** 3 for n in sizes)  # split-TF32 LU: 3 x (8/3) N^3
+    flops = sum(8.0 * float(n) ** 3 for n in sizes)  # split LU, 3 products: 3 x (8/3) N^3
     return {"workload": SWEEP_WORKLOAD, "instances": len(insts), "N_min": min(sizes), "N_max": max(sizes),
             "sequential_seconds": t_seq, "sequential_solves_per_s": len(insts) / t_seq,
             "batched_seconds": t_best, "batched_solves_per_s": len(insts) / t_best,
@@ -994,7 +994,7 @@ def sweep_section(ctx, max_over_ranks) -> dict:
             "seconds_by_concurrency": {str(k): v for k, v in timings.items()},
             "max_relative_residual": max(r.metrics["relative_residual"] for r in res),
             "max_refinement_iterations": max(r.metrics["refinement_iterations"] for r in res),
-            "tf32_tflops_effective": flops / t_best / 1e12,
+            "tensor_tflops_effective": flops / t_best / 1e12,
             "timing": "wall clock around the library call (host tensors in, host currents out)"}
 
 
@@ -1044,7 +1044,7 @@ def adjoint_section(ctx, steps: int, max_over_ranks):
     t_mx_s = max_over_ranks(statistics.mean(t_mx))
     t_64_s = max_over_ranks(statistics.mean(t_64))
     return {
-        "workload": ADJOINT_WORKLOAD, "N": 4 * m.num_edges, "method": "mixed_ir (split-TF32 LU + FP64 FGMRES, "
+        "workload": ADJOINT_WORKLOAD, "N": 4 * m.num_edges, "method": "mixed_ir (split-FP16 LU + FP64 FGMRES, "
         "adjoint: conjugate-transpose FGMRES on the same factors)",
         "grads_per_s": 1.0 / t_mx_s, "ms_per_grad": 1e3 * t_mx_s, "steps": steps,
         "fp64_grads_per_s": 1.0 / t_64_s, "speedup_vs_fp64": t_64_s / t_mx_s,
@@ -1054,22 +1054,23 @@ def adjoint_section(ctx, steps: int, max_over_ranks):
     }
 
 
-def largest_launch_roofline(span, peaks, tf32_peak):
-    """The first trailing update of the N = 6016 factorization (block step
-    0: C = 2m x (m - 64) real with m = 5952, split packs 256 wide) from its
-    in-situ timeline span: time against max(bytes / HBM, flops / TF32)."""
+def largest_launch_roofline(span, peaks, f16_peak):
+    """The longest trailing update of the N = 6000 factorization (the first
+    group of four block steps: C = 2m x m real with m = 5744 less the next
+    diagonal block, K = 512, split FP16 operands) from its in-situ timeline
+    span: time against max(bytes / HBM, flops / FP16)."""
     if not span:
         return None
-    np_, nb = 6016, 64
-    m = np_ - nb
-    rows, cols, k = 2 * m, m - nb, 256
-    alg_bytes = 4.0 * (2.0 * rows * cols + (rows + cols) * k)
-    flops = 2.0 * rows * cols * 384
+    np_, nb, k = 6000, 64, 512
+    m = np_ - 4 * nb
+    elems = 2.0 * m * m - 2.0 * nb * nb
+    alg_bytes = 8.0 * elems + 4.0 * 3.0 * m * k
+    flops = 2.0 * elems * 3.0 * k
     t = (span[1] - span[0]) / 1e3
-    roof = max(alg_bytes / (peaks["hbm_gbs"] * 1e9), flops / (tf32_peak * 1e12))
-    return {"us": t * 1e6, "algorithmic_bytes": alg_bytes, "tf32_flops": flops, "roofline_us": roof * 1e6,
+    roof = max(alg_bytes / (peaks["hbm_gbs"] * 1e9), flops / (f16_peak * 1e12))
+    return {"us": t * 1e6, "algorithmic_bytes": alg_bytes, "f16_flops": flops, "roofline_us": roof * 1e6,
             "frac_of_roofline": roof / t, "hbm_frac": alg_bytes / t / (peaks["hbm_gbs"] * 1e9),
-            "tensor_frac": flops / t / (tf32_peak * 1e12)}
+            "tensor_frac": flops / t / (f16_peak * 1e12)}
 
 
 def timeline_summary(spans):

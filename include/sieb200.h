@@ -339,7 +339,7 @@ int sieb200_zgemm(sieb200_ctx* ctx, int64_t m, int64_t nc, int64_t k, const doub
 int sieb200_prepare_records(sieb200_ctx* ctx, int64_t faces, const double* maps, double reference_impedance,
                             double* records_out, double* diag_out);
 
-/* Split-TF32 tensor-core contraction used by the mixed LU's trailing update
+/* Split-TF32 tensor-core contraction of the mixed LU's step-by-step schedules
  * (no counterpart in the reference, which calls cuSOLVER): on device data,
  *   C[m2 x n] (fp32, column-major, ldc) -= A[m2 x k] * B[n x k]^T,
  * A and B K-major fp32, k a multiple of 32. mode 3: persistent tcgen05
@@ -366,14 +366,14 @@ int sieb200_gemm_tf32_sub_shifted(sieb200_ctx* ctx, int64_t m2, int64_t n, int k
  * phases with std::chrono): when enabled, the library brackets each launch
  * of the listed kernels with CUDA events on the context stream and
  * accumulates launch count, device milliseconds and algorithmic work.
- * kernel 0: split-TF32 trailing GEMM (work = 2*m2*n*k TF32 flops and
- * 4*(2*m2*n + (m2 + n)*k) bytes per launch); 1: triangular solves
+ * kernel 0: trailing GEMM of a factorization (work = 2 flops per element and
+ * product of the split operands, the bytes of C read and written and of the operands); 1: triangular solves
  * (work = bytes of factors read); 2: FP64 matvec (bytes of Z read);
  * 3: diagonal-block LU + inverses (with the previous block step's update
  * of the block; on the solver's lookahead stream); 4: block-step panels
  * (L21 with the previous step's update of its rows, and U12: one launch per
  * step); 5: the two blocked triangular solves of a multi-right-hand-side
- * preconditioner application (work = 24 np^2 nrhs TF32 flops and 48 np^2
+ * preconditioner application (work = 24 np^2 nrhs TF32 flops and 32 np^2
  * bytes of packed factors); 6: whole mixed factorizations; 7: whole refined
  * solves (spans on the context stream unless stated). Kind 2 also counts the
  * FP64 complex GEMMs (8 m nc k flops). */

@@ -21,23 +21,25 @@
 // complex atomics per pair. Here:
 //   1. face_prep      one thread per face builds a geometry record and the
 //                     face's quadrature points (double) once.
-//   2. pair_regular   one CTA per test face; its 8 warps stream the source
-//                     faces, one warp per face pair, lanes over the Q*Q point
-//                     pairs. Instead of 9 RWG products per point pair, every
-//                     lane accumulates 8 (TL) + 10 (TK) complex moments of the
-//                     kernel in triangle-local coordinates; a warp butterfly
-//                     reduces them and 9 lanes expand them into the 3x3 blocks:
+//   2. far_pairs      a lane (or a few) per face pair: it runs over its test
+//                     points and, for each, sums over the source points only what
+//                     depends on them (G, G q, g, g q), folded once per test
+//                     point into the pair's complex moments in triangle-local
+//                     coordinates, from which the 3x3 blocks follow:
 //                       rho_m . rho_n  = (p-A_j).(q-B_i)
-//                       (rho_m x rho_n) . R = (rho_m x rho_n) . (v_j - v_i),
-//                     so the inner loop is bound by the Green-kernel
-//                     evaluation (sqrt, division, sincos) on the FP64 pipe.
-//   3. pair_singular  one warp per near pair (centroid distance below the
-//                     threshold, decided in float as the reference does) adds
-//                     the analytic (Wilton) part, lanes over outer points.
+//                       (rho_m x rho_n) . R = (rho_m x rho_n) . (v_j - v_i).
+//                     The Green kernel's phase and reciprocal square root
+//                     are written for the FP64 pipe, which binds (phase.cuh).
+//                     With RWG testing (m, n) and (n, m) are one evaluation.
+//   3. near pairs     (centroid distance below the threshold, decided in float
+//                     as the reference does): near_regular, the extracted
+//                     kernel, and pair_singular, the analytic (Wilton) part,
+//                     one warp per pair, lanes over the outer points.
 //   4. mass_face      GSTC only: one thread per (face, tensor).
 //   5. gather         one thread per (test edge, source edge) sums the <= 2x2
 //                     incident face pairs and writes every block of Z exactly
-//                     once per slab: deterministic, no atomics.
+//                     once per slab (with one slab Z is only stored):
+//                     deterministic, no atomics.
 // Face-pair blocks live in a workspace processed in slabs of test faces, so
 // the largest meshes stream through a bounded buffer.
 
@@ -57,7 +59,7 @@ namespace sieb200 {
 namespace {
 
 constexpr int kMaxQ = 80;      // Dunavant rule 20 has 79 points
-constexpr int kWarps = 8;      // warps per CTA in pair_regular
+constexpr int kWarps = 8;      // warps per CTA of the warp-per-pair kernels
 constexpr int kMaxLine = 20;   // Gauss-Legendre points of the nTL line form
 constexpr double kPi = 3.14159265358979323846;
 

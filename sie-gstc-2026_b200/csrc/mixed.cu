@@ -1,5 +1,6 @@
 // Mixed-precision dense solver: randomized butterfly transform + blocked LU
-// without pivoting in complex64 with split-TF32 tensor-core trailing updates,
+// without pivoting in complex64 with split-FP16 tensor-core trailing updates
+// (split TF32 in the step-by-step schedules),
 // wrapped in FP64 restarted GMRES (right preconditioned) against the intact
 // complex128 system. Replaces the cusolverDnZgetrf/Zgetrs path of
 // include/sie_mom/cuda/dense_lu_solver.cuh:42-166 for the solves/s metric.

@@ -253,7 +253,7 @@ __global__ void ff_faces_kernel(const double* __restrict__ V, const int* __restr
 // Far-field operator as a matrix: rows (F_theta of direction d, then F_phi),
 // columns (J of edge e, then M of edge e), row-major with 2*ne columns, so
 // that [F_theta; F_phi] = A [J; M] with the same radiation vectors and
-// coefficients as ff_samples_kernel / ff_directions_kernel. One thread per
+// coefficients as ff_faces_kernel / ff_directions_kernel. One thread per
 // (direction, edge); the edge's incident faces and the 7-point rule are
 // evaluated on the fly.
 __global__ void ff_matrix_kernel(const double* __restrict__ V, const int* __restrict__ F,

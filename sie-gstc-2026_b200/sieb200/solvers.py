@@ -224,7 +224,7 @@ class Context:
         return [(kinds[i], t0[i], t1[i]) for i in range(min(n, count.value))]
 
     def profile_read(self, kernel: int) -> dict:
-        """kernel 0: split-TF32 trailing GEMM, 1: triangular solves, 2: FP64 matvec
+        """kernel 0: trailing GEMM, 1: triangular solves, 2: FP64 matvec
         and complex GEMM, 3: diagonal-block LU, 4: block-step panels (L21 and U12),
         5: multi-right-hand-side block triangular solves,
         6: whole mixed factorizations, 7: whole refined solves."""
