@@ -1250,10 +1250,13 @@ struct GatherParams {
 
 // The region block (1x1 PEC, 2x2 PMCHWT, 4x4 GSTC) of Z at test edge te and
 // source edge se from the face-pair blocks of the test faces in [m0, m1);
-// false when te has no incident face in the slab.
+// false when te has no incident face in the slab. FORM: the formulation, or -1
+// to take it from P.
+template <int FORM>
 __device__ __forceinline__ bool edge_pair_block(const cplx* __restrict__ pairs, const cplx* __restrict__ mass,
                                                 const int* __restrict__ inc, const GatherParams& P, int te, int se,
                                                 cplx (&blk)[4][4]) {
+    const int form = FORM < 0 ? P.formulation : FORM;
     const int it[2] = {inc[2 * te], inc[2 * te + 1]};
     const int is[2] = {inc[2 * se], inc[2 * se + 1]};
     bool any = false;
@@ -1285,7 +1288,7 @@ __device__ __forceinline__ bool edge_pair_block(const cplx* __restrict__ pairs, 
 #pragma unroll
             for (int k = 0; k < 4; ++k)
                 if (k < P.NB) acc[k] += pb[k];
-            if (P.formulation == SIEB200_GSTC && m == n) {
+            if (form == SIEB200_GSTC && m == n) {
                 has_mass = true;
                 const cplx* mb = mass + (size_t)m * 72 + j * 3 + i;
 #pragma unroll
@@ -1300,12 +1303,12 @@ __device__ __forceinline__ bool edge_pair_block(const cplx* __restrict__ pairs, 
     } else if (P.layout == PAIR_TK_ONLY) {
         acc[1] = acc[0];
     }
-    if (P.formulation == SIEB200_PEC_EFIE && P.variant == 2) {
+    if (form == SIEB200_PEC_EFIE && P.variant == 2) {
         // N-MFIE (pec_solver.cu:171-240): 1/2 Gram on the same face, - nTK2.
         blk[0][0] = cx(0.5 * gram_acc, 0.0) - acc[1];
-    } else if (P.formulation == SIEB200_PEC_EFIE) {
+    } else if (form == SIEB200_PEC_EFIE) {
         blk[0][0] = P.c_jj[1] * acc[0];
-    } else if (P.formulation == SIEB200_PMCHWT && P.variant == 2) {
+    } else if (form == SIEB200_PMCHWT && P.variant == 2) {
         // acc: nTL1, nTL2, nTK1, nTK2.
         const cplx jj = acc[1] * cx(0.0, P.w_em[1]) - acc[0] * cx(0.0, P.w_em[0]);
         const cplx jm = acc[3] * P.eps[1] - acc[2] * P.eps[0] - cx(P.eps_f * gram_acc, 0.0);
@@ -1314,7 +1317,7 @@ __device__ __forceinline__ bool edge_pair_block(const cplx* __restrict__ pairs, 
         blk[0][1] = jm * P.s_jm;
         blk[1][0] = mj * P.s_jm;
         blk[1][1] = jj * (-P.s_mm);
-    } else if (P.formulation == SIEB200_PMCHWT) {
+    } else if (form == SIEB200_PMCHWT) {
         // acc: TL1, TL2, TK1, TK2 (or TL1, TL2, TK1 + TK2, 0)
         const cplx tk = acc[2] + acc[3];
         const cplx jm = tk * P.s_jm;
@@ -1346,7 +1349,12 @@ __device__ __forceinline__ int region_count(int formulation) {
 // column-major stores. Sums the incident face pairs with the test face in
 // [m0, m1). ADD: adds into Z (zeroed before the first of several slabs); else
 // the only slab, and every entry of Z is stored once without being read.
-template <bool ADD>
+// Bound: the latency of its pair reads, so by the threads in flight; each
+// formulation is its own instance, since one kernel for all keeps the 4 x 4
+// blocks of SIE-GSTC in registers (36, 48 and 96 a thread now): PEC, 1920 edges
+// 191 -> 103 us; T-PMCHWT, 3000 edges 780 -> 645 us; SIE-GSTC, 4320 edges
+// 1720 -> 1670 us. The shape of the CTA's tile of edges makes no difference.
+template <int FORM, bool ADD>
 __global__ void gather_kernel(const cplx* __restrict__ pairs, const cplx* __restrict__ mass,
                               const int* __restrict__ inc, GatherParams P, cplx* __restrict__ Z,
                               int64_t ldz) {
@@ -1354,9 +1362,9 @@ __global__ void gather_kernel(const cplx* __restrict__ pairs, const cplx* __rest
     const int se = blockIdx.y * blockDim.y + threadIdx.y;
     if (te >= P.ne || se >= P.ne) return;
     cplx blk[4][4];
-    if (!edge_pair_block(pairs, mass, inc, P, te, se, blk) && ADD) return;
+    if (!edge_pair_block<FORM>(pairs, mass, inc, P, te, se, blk) && ADD) return;
     const int64_t E = P.ne;
-    const int nr = region_count(P.formulation);
+    const int nr = region_count(FORM);
 #pragma unroll
     for (int c = 0; c < 4; ++c)
 #pragma unroll
@@ -1383,7 +1391,7 @@ __global__ void gather_matvec_kernel(const cplx* __restrict__ pairs, const cplx*
     bool mine = false;
     for (int se = lane; se < P.ne; se += 32) {
         cplx blk[4][4];
-        if (!edge_pair_block(pairs, mass, inc, P, te, se, blk)) break;  // same answer for every se
+        if (!edge_pair_block<-1>(pairs, mass, inc, P, te, se, blk)) break;  // same answer for every se
         mine = true;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
@@ -1739,10 +1747,14 @@ static int assemble_or_apply(sieb200_ctx* ctx, const sieb200_mesh& mesh, const s
         const dim3 gb(32, 8), gg((ne + 31) / 32, (ne + 7) / 8);
         if (dx)
             gather_matvec_kernel<<<(ne + 7) / 8, 256, 0, st>>>(po.pairs, dmass, ctx->inc.as<int>(), gp, dx, dy);
-        else if (one_slab)
-            gather_kernel<false><<<gg, gb, 0, st>>>(po.pairs, dmass, ctx->inc.as<int>(), gp, dZ, ldz);
-        else
-            gather_kernel<true><<<gg, gb, 0, st>>>(po.pairs, dmass, ctx->inc.as<int>(), gp, dZ, ldz);
+        else {
+            auto* gather = gp.formulation == SIEB200_PEC_EFIE
+                               ? (one_slab ? gather_kernel<SIEB200_PEC_EFIE, false> : gather_kernel<SIEB200_PEC_EFIE, true>)
+                           : gp.formulation == SIEB200_PMCHWT
+                               ? (one_slab ? gather_kernel<SIEB200_PMCHWT, false> : gather_kernel<SIEB200_PMCHWT, true>)
+                               : (one_slab ? gather_kernel<SIEB200_GSTC, false> : gather_kernel<SIEB200_GSTC, true>);
+            gather<<<gg, gb, 0, st>>>(po.pairs, dmass, ctx->inc.as<int>(), gp, dZ, ldz);
+        }
         SIEB_NOTE_LAUNCH();
         SIEB_TRY_CUDA(cudaGetLastError());
     }
