@@ -492,7 +492,9 @@ gemm_tf32_sub_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const _
 // FP16's range, and lo is kept 2^11 up, so that it has hi's exponent range: entries down
 // to 2^-28 of the largest keep all 22 bits. (One scale for a whole operand did not
 // do: on the 20,880-unknown omega spindle entries of L21 beyond 1023 stand beside rows
-// whose lo parts were lost, 17 refinement iterations instead of 15.) The two mixed
+// whose lo parts were lost, 17 refinement iterations instead of 15. Nor do these scales
+// alone: the packs hold L21 and U12 after a balancing per elimination index,
+// row_exponents in mixed.cu, which cancels in the product.) The two mixed
 // products share one accumulator, hi.hi has the other, and the epilogue joins them.
 // The tensor core's own accumulation truncates, so a sum over all of K = 512
 // loses more than the single-step schedule's sums over 128 did. The epilogue

@@ -31,12 +31,11 @@ int gemm_tc_check(GemmTC* g, cudaStream_t stream);
 // Whether the default kernel configuration is selected (no switch).
 bool gemm_tc_default(const GemmTC* g);
 
-// Scale of a row of L21 or a column of U12 in the FP16 split operands: the power of
-// two that brings its largest magnitude (float bits) into [2^14, 2^15), one per
-// block step. Returns its exponent; 0 for a row of zeros or of non-finite values.
-__host__ __device__ inline int half_exponent(unsigned max_bits) {
-    const int e = (int)(max_bits >> 23) - 127;
-    return max_bits == 0u || e > 127 ? 0 : (14 - e > 120 ? 120 : 14 - e);
+// Exponent of the scale of a row of L21 or a column of U12 in the FP16 split operands:
+// with it the largest entry, whose exponent is max_exp, falls into [2^14, 2^15).
+__host__ __device__ inline int half_exponent(int max_exp) {
+    const int e = 14 - max_exp;
+    return e > 126 ? 126 : (e < -126 ? -126 : e);
 }
 // The same update from scaled FP16 split packs (rows of ld FP16 values, hi
 // columns from k0, lo columns from klo, K of each; lo kept 2^11 up; per 128 columns of

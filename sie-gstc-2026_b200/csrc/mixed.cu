@@ -223,6 +223,40 @@ __device__ __forceinline__ double rcp_rn(double x) { return __drcp_rn(x); }
 __device__ __forceinline__ float tiny_pivot(float) { return 1e-30f; }
 __device__ __forceinline__ double tiny_pivot(double) { return 1e-280; }
 
+__device__ __forceinline__ float pow2f(int e) { return __int_as_float((e + 127) << 23); }  // |e| <= 126
+// floor(log2(x)) of the larger magnitude (-127 for zero and subnormals, 128 for
+// infinities and NaN).
+__device__ __forceinline__ int exponent_of(float x) { return (int)((__float_as_uint(x) & 0x7fffffffu) >> 23) - 127; }
+__device__ __forceinline__ float larger(float2 v) { return fmaxf(fabsf(v.x), fabsf(v.y)); }
+__device__ __forceinline__ float larger(double2 v) { return (float)fmax(fabs(v.x), fabs(v.y)); }
+
+// Balancing exponents of a block step's NB elimination indices for the FP16 split
+// operands: column k of L21 is packed times 2^ex[k], row k of U12 times 2^-ex[k], ex[k]
+// the exponent of the largest entry in row k of the (updated) diagonal block about
+// the middle of the block's range. The powers of two cancel in the product. Why: rows
+// of A scaled by d_i give entries d_i / d_k in L21 and d_k in row k of U12, so that
+// the small entry of one operand meets the large one of the other, and one scale
+// per row and column leaves FP16's 2^28 to cover all of d. The row's largest entry
+// carries d_k and a factor the same for all rows, so both operands come out flat,
+// whatever the scaling of the columns (which the scale per column of U12 takes; the
+// pivot's exponent would carry it into L21). Emulated with exact accumulation, 256
+// unknowns, rows or rows and columns scaled within 2^40 (2^48), one preconditioned
+// step: residual 5e-8, as unscaled and as with TF32 operands; without balancing
+// 1e-5 (2e-3). Cost: 7.17 and 7.20 ms, N = 6000 factor and solve. Warp 0: m0 and m1 the largest magnitudes of rows lane and lane + 32.
+constexpr int kBalanceMax = 60;  // keeps every exponent of the packs within pow2f's range twice over
+__device__ __forceinline__ void row_exponents(float m0, float m1, int lane, int* __restrict__ ex) {
+    const int e0 = exponent_of(m0), e1 = exponent_of(m1);
+    int lo = min(e0, e1), hi = max(e0, e1);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    const int mid = (lo + hi) >> 1;
+    ex[lane] = max(-kBalanceMax, min(kBalanceMax, e0 - mid));
+    ex[lane + 32] = max(-kBalanceMax, min(kBalanceMax, e1 - mid));
+}
+
 // Diagonal block: LU without pivoting and both triangular inverses in one
 // pass of NB rank-1 steps over registers. Warp w holds columns
 // [kDiagCols w, kDiagCols (w+1)), lane l rows l and l+32. Step j takes the
@@ -584,7 +618,8 @@ __device__ __forceinline__ void leaf32_store(const float2 (&a)[RB], int lane, co
 // pivot sets the error word and continues with a zero reciprocal.
 __global__ void __launch_bounds__(256) diag_lu_rec_kernel(const float2* __restrict__ W, int64_t ldw, int64_t k0,
                                                           int kb, float2* __restrict__ Linv,
-                                                          float2* __restrict__ Uinv, unsigned* __restrict__ err) {
+                                                          float2* __restrict__ Uinv, unsigned* __restrict__ err,
+                                                          int* __restrict__ rowex) {
     extern __shared__ __align__(16) unsigned char dyn_smem[];
     float2* A = reinterpret_cast<float2*>(dyn_smem);  // NB x (NB + 1), row-major
     float2* blk = A + NB * (NB + 1);
@@ -612,6 +647,12 @@ __global__ void __launch_bounds__(256) diag_lu_rec_kernel(const float2* __restri
         for (int c = 0; c < RB; ++c) a[c] = A[lane * LD + c];
         leaf32(a, lane, rc1, err);
         leaf32_store(a, lane, rc1, IL1, IU1);
+    } else if (w == 1 && rowex) {
+        float mx[2] = {0.f, 0.f};
+        for (int c = 0; c < NB; ++c)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) mx[h] = fmaxf(mx[h], larger(A[(lane + 32 * h) * LD + c]));
+        row_exponents(mx[0], mx[1], lane, rowex);
     }
     __syncthreads();
     if (w < 4) mm32<128, 0>(IL1, kRecLd, A + RB, LD, U12, kRecLd, tid);             // U12 = inv(L11) A12
@@ -692,16 +733,18 @@ __global__ void __launch_bounds__(256) diag_update_kernel(T* __restrict__ W, int
 // half); 1: diag_panel (one named barrier per panel; the coefficient
 // columns then live in the dynamic shared memory, after the update tiles
 // are no longer read); 2: diag_steps_compact (as 0, one code path).
+// rowex (NB entries, optional): the step's row_exponents.
 template <class T, int ELIM>
 __global__ void __launch_bounds__(kDiagThreads) diag_lu_kernel(const T* __restrict__ W, int64_t ldw,
                                                                int64_t k0, int kb, T* __restrict__ Linv,
                                                                T* __restrict__ Uinv,
                                                                unsigned* __restrict__ err, int64_t kp1,
-                                                               int64_t kp2) {
+                                                               int64_t kp2, int* __restrict__ rowex) {
     constexpr int CW = kDiagCols;
     extern __shared__ __align__(16) unsigned char dyn_smem[];
     __shared__ T cbuf[2][NB];  // c_j, double-buffered across the step barrier
     __shared__ T rcps[NB];     // 1 / p_j
+    __shared__ float rmax[kDiagWarps][NB];  // largest magnitude per row and warp, before the elimination
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     T a[CW][2];
 #pragma unroll
@@ -733,6 +776,15 @@ __global__ void __launch_bounds__(kDiagThreads) diag_lu_kernel(const T* __restri
             }
         }
     }
+    if (rowex) {  // read back after the elimination's barriers
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            float mx = 0.f;
+#pragma unroll
+            for (int v = 0; v < CW; ++v) mx = fmaxf(mx, larger(a[v][h]));
+            rmax[w][lane + 32 * h] = mx;
+        }
+    }
     if (ELIM == 2) {
 #pragma unroll 1
         for (int bp = 0; bp < kDiagWarps; ++bp)
@@ -751,6 +803,15 @@ __global__ void __launch_bounds__(kDiagThreads) diag_lu_kernel(const T* __restri
         for (int bp = kDiagWarps / 2; bp < kDiagWarps; ++bp) diag_steps<T, 1>(a, bp, w, lane, cbuf, rcps, err);
     }
     __syncthreads();
+    if (rowex && w == 0) {
+        float m0 = 0.f, m1 = 0.f;
+#pragma unroll
+        for (int u = 0; u < kDiagWarps; ++u) {
+            m0 = fmaxf(m0, rmax[u][lane]);
+            m1 = fmaxf(m1, rmax[u][lane + 32]);
+        }
+        row_exponents(m0, m1, lane, rowex);
+    }
 #pragma unroll
     for (int v = 0; v < CW; ++v) {
         const int c = CW * w + v;
@@ -770,7 +831,7 @@ __global__ void __launch_bounds__(kDiagThreads) diag_lu_kernel(const T* __restri
 
 
 template <class T>
-using DiagKernel = void (*)(const T*, int64_t, int64_t, int, T*, T*, unsigned*, int64_t, int64_t);
+using DiagKernel = void (*)(const T*, int64_t, int64_t, int, T*, T*, unsigned*, int64_t, int64_t, int*);
 
 // The elimination variant the switches select (diag_lu_kernel's ELIM).
 template <class T>
@@ -807,8 +868,9 @@ struct PanelArgs {
     int64_t a_lo = 0, b_lo = 0;
     int lo_rn = 0;  // lo parts rounded to the nearest TF32
     // pack 2: scaled FP16 split instead, strides and offsets in FP16 values (lo
-    // kept 2^11 up); the scale of each row of L21 and column of U12 goes to fa and fb
-    // as its reciprocal
+    // kept 2^11 up), balanced by rowex (row_exponents); the scale of each row of L21
+    // and column of U12 goes to fa and fb as its reciprocal
+    const int* rowex = nullptr;
     __half* Ah = nullptr;
     __half* Bh = nullptr;
     float* fa = nullptr;
@@ -818,31 +880,32 @@ struct PanelArgs {
     int b_first = 0, nl_run = 0;
 };
 
-__device__ __forceinline__ float pow2f(int e) { return __int_as_float((e + 127) << 23); }  // |e| <= 126
-
-// v = h + 2^-11 l in FP16, both rounded to nearest.
-__device__ __forceinline__ void split_half(float2 v, __half2& h, __half2& l) {
+// v times 2^e as h + 2^-11 l in FP16, both rounded to nearest. The power of two in
+// two factors, since e may be out of pow2f's range.
+__device__ __forceinline__ void split_half(float2 v, int e, __half2& h, __half2& l) {
+    const float s0 = pow2f(e >> 1), s1 = pow2f(e - (e >> 1));
+    v = make_float2(v.x * s0 * s1, v.y * s0 * s1);
     h = __floats2half2_rn(v.x, v.y);
     const float2 r = __half22float2(h);
     l = __floats2half2_rn((v.x - r.x) * 2048.f, (v.y - r.y) * 2048.f);
 }
 
 // FP16 scale exponents of the 32 lines (rows of L21, columns of U12) a panels CTA holds in
-// shared memory, line i at lines[i][0 .. NB): eight lanes per line, result in ex[32]; f
-// receives the reciprocals of the `count` first.
+// shared memory, line i at lines[i][0 .. NB), after balancing by 2^bal[k]: eight
+// lanes per line, result in ex[32]; f receives the reciprocals of the `count` first.
 template <class L>
-__device__ __forceinline__ void line_exponents(const L& lines, int* ex, float* f, int64_t count) {
+__device__ __forceinline__ void line_exponents(const L& lines, const int* bal, int* ex, float* f, int64_t count) {
     const int line = threadIdx.x >> 3, part = threadIdx.x & 7;
-    float mx = 0.f;
+    int mx = -1000;
 #pragma unroll
     for (int c = 0; c < NB / 8; ++c) {
-        const float2 v = lines[line][part + 8 * c];
-        mx = fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.y)));
+        const float v = larger(lines[line][part + 8 * c]);
+        if (v > 0.f) mx = max(mx, exponent_of(v) + bal[part + 8 * c]);
     }
 #pragma unroll
-    for (int o = 1; o < 8; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    for (int o = 1; o < 8; o <<= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     if (part == 0) {
-        const int e = half_exponent(__float_as_uint(mx));
+        const int e = mx == -1000 ? 0 : half_exponent(mx);
         ex[line] = e;
         if (line < count) f[line] = pow2f(-e);
     }
@@ -859,7 +922,7 @@ __device__ __forceinline__ void line_exponents(const L& lines, int* ex, float* f
 // triangular, so each column pair's k loop stops at its last column.
 template <class T>
 __device__ __forceinline__ void panel_L_body(T* __restrict__ W, int64_t ldw, const PanelArgs& pa,
-                                             const T* __restrict__ Uinv, int bx) {
+                                             const T* __restrict__ Uinv, const int* bal, int bx) {
     const int64_t k0 = pa.k0, r0 = pa.s0, np = pa.np;
     const int kb = pa.kb;
     extern __shared__ __align__(16) unsigned char dyn_smem[];
@@ -991,15 +1054,14 @@ __device__ __forceinline__ void panel_L_body(T* __restrict__ W, int64_t ldw, con
     if constexpr (std::is_same<T, float2>::value) {
         if (pa.pack == 2) {
             __shared__ int ex[32];
-            line_exponents(Ar, ex, pa.fa + (rb - pa.a_r0), np - rb);
-            for (int e = tid; e < 32 * NB; e += blockDim.x) {
-                const int rr = e / NB, c = e % NB;
+            line_exponents(Ar, bal, ex, pa.fa + (rb - pa.a_r0), np - rb);
+            const int c = tid % NB, bc = bal[c];
+#pragma unroll 2
+            for (int rr = tid / NB; rr < 32; rr += kPanelThreads / NB) {
                 const int64_t gr = rb + rr;
-                if (gr >= np) continue;
-                const float2 v = Ar[rr][c];
-                const float sc = pow2f(ex[rr]);
+                if (gr >= np) break;
                 __half2 h, l;
-                split_half(make_float2(v.x * sc, v.y * sc), h, l);
+                split_half(Ar[rr][c], ex[rr] + bc, h, l);
                 __half2* row0 = reinterpret_cast<__half2*>(pa.Ah + 2 * (gr - pa.a_r0) * pa.a_ld) + c;
                 __half2* row1 = reinterpret_cast<__half2*>(pa.Ah + (2 * (gr - pa.a_r0) + 1) * pa.a_ld) + c;
                 const int64_t lo = pa.a_lo / 2;
@@ -1044,7 +1106,7 @@ __device__ __forceinline__ void panel_L_body(T* __restrict__ W, int64_t ldw, con
 // row pair's k loop stops at its last row.
 template <class T>
 __device__ __forceinline__ void panel_U_body(T* __restrict__ W, int64_t ldw, const PanelArgs& pa,
-                                             const T* __restrict__ Linv, int bx) {
+                                             const T* __restrict__ Linv, const int* bal, int bx) {
     const int64_t k0 = pa.k0, c0 = pa.s0, np = pa.np;
     const int kb = pa.kb;
     extern __shared__ __align__(16) unsigned char dyn_smem[];
@@ -1159,7 +1221,7 @@ __device__ __forceinline__ void panel_U_body(T* __restrict__ W, int64_t ldw, con
     __syncthreads();
     __shared__ int ex[32];
     if constexpr (std::is_same<T, float2>::value) {
-        if (pa.pack == 2) line_exponents(Ac, ex, pa.fb + (cb - pa.b_c0), np - cb);
+        if (pa.pack == 2) line_exponents(Ac, bal, ex, pa.fb + (cb - pa.b_c0), np - cb);
     }
     for (int e = tid; e < 32 * NB; e += blockDim.x) {
         const int r = e % NB, c = e / NB;
@@ -1169,9 +1231,8 @@ __device__ __forceinline__ void panel_U_body(T* __restrict__ W, int64_t ldw, con
         if (r < kb) W[(k0 + r) + gc * ldw] = v;
         if constexpr (std::is_same<T, float2>::value) {
             if (pa.pack == 2) {
-                const float sc = pow2f(ex[c]);
                 __half2 h, l;
-                split_half(make_float2(v.x * sc, v.y * sc), h, l);
+                split_half(v, ex[c] + bal[r], h, l);
                 __half2* col = reinterpret_cast<__half2*>(pa.Bh + (gc - pa.b_c0) * pa.b_ld) + r;
                 col[0] = h;
                 col[pa.b_lo / 2] = l;
@@ -1259,8 +1320,11 @@ template <class T>
 __global__ void __launch_bounds__(256, 3) panels_kernel(T* __restrict__ W, int64_t ldw, const T* __restrict__ Uinv,
                                                         const T* __restrict__ Linv, const PanelArgs pa) {
     const int nl = pa.nl_run > 0 ? pa.nl_run : pa.nL;
-    if ((int)blockIdx.x < nl) panel_L_body(W, ldw, pa, Uinv, pa.b_first + (int)blockIdx.x);
-    else panel_U_body(W, ldw, pa, Linv, pa.b_first + (int)blockIdx.x - nl);
+    const bool lower = (int)blockIdx.x < nl;
+    __shared__ int bal[NB];  // balancing exponents (pack 2); the bodies synchronize before they read it
+    if (pa.pack == 2 && threadIdx.x < NB) bal[threadIdx.x] = lower ? pa.rowex[threadIdx.x] : -pa.rowex[threadIdx.x];
+    if (lower) panel_L_body(W, ldw, pa, Uinv, bal, pa.b_first + (int)blockIdx.x);
+    else panel_U_body(W, ldw, pa, Linv, bal, pa.b_first + (int)blockIdx.x - nl);
 }
 
 // SIMT trailing update C -= L21 U12 in complex64 (checking path).
@@ -2339,13 +2403,14 @@ int mixed_factorize(DenseSolver* s) {
     const char* hsm_env = getenv("SIEB200_PANEL_HEAD_SMEM");
     st->head_smem = hsm_env ? std::max(kSmemPanel, std::min(kSmemPanelHeadMax, atoi(hsm_env))) : kSmemPanel;
 
-    // Workspace layout in s->lu: W | Linv | Uinv | diag | err+flags ; packs separate.
+    // Workspace layout in s->lu: W | Linv | Uinv | diag | err+flags | rowex ; packs separate.
     const size_t bW = sizeof(float2) * ldw * np;
     const size_t bInv = sizeof(float2) * NB * NB * nbl;
     const size_t bDiag = sizeof(double) * 8 * np;
     const size_t bFlags = sizeof(unsigned) * (4 * nbl + 16);
     auto up = [](size_t b) { return ((b + 255) / 256) * 256; };
-    SIEB_RETURN_IF(s->lu.reserve(up(bW) + 2 * up(bInv) + up(bDiag) + up(bFlags)));
+    const size_t bEx = sizeof(int) * NB * nbl;
+    SIEB_RETURN_IF(s->lu.reserve(up(bW) + 2 * up(bInv) + up(bDiag) + up(bFlags) + bEx));
     char* base = s->lu.as<char>();
     st->W = reinterpret_cast<float2*>(base);
     st->Linv = reinterpret_cast<float2*>(base + up(bW));
@@ -2353,6 +2418,7 @@ int mixed_factorize(DenseSolver* s) {
     st->diag = reinterpret_cast<double*>(base + up(bW) + 2 * up(bInv));
     st->err = reinterpret_cast<unsigned*>(base + up(bW) + 2 * up(bInv) + up(bDiag));
     st->tri_flags = st->err + 16;
+    st->rowex = reinterpret_cast<int*>(base + up(bW) + 2 * up(bInv) + up(bDiag) + up(bFlags));
     const int K3 = 6 * NB;
     const size_t bApack = ((sizeof(float) * 2 * np * K3 + 255) / 256) * 256;
     SIEB_RETURN_IF(s->gemm_a.reserve(2 * bApack));
@@ -2475,6 +2541,7 @@ static int mixed_enqueue(DenseSolver* s, MixedState* st, size_t bFlags, int K3) 
         const int64_t k0 = bk * NB;
         const int kb = (int)std::min<int64_t>(NB, np - k0);
         const int nupd = (kp1 >= 0) + (kp2 >= 0);
+        int* rowex = st->blocked ? st->rowex + bk * NB : nullptr;
         cudaEvent_t ev;
         ctx->prof.begin(sm, 3, (8.0 / 3.0 + 8.0 / 3.0) * NB * NB * NB + nupd * 8.0 * NB * NB * NB,
                         8.0 * NB * NB * (3.0 + 2.0 * nupd), &ev);
@@ -2486,14 +2553,15 @@ static int mixed_enqueue(DenseSolver* s, MixedState* st, size_t bFlags, int K3) 
         }
         if (st->diag_rec) {
             diag_lu_rec_kernel<<<1, 256, kSmemDiagRec, sm>>>(st->W, ldw, k0, kb, st->Linv + (size_t)bk * NB * NB,
-                                                             st->Uinv + (size_t)bk * NB * NB, st->err);
+                                                             st->Uinv + (size_t)bk * NB * NB, st->err, rowex);
             SIEB_NOTE_LAUNCH();
             ctx->prof.end(sm, ev);
             SIEB_TRY_CUDA(cudaGetLastError());
             return SIEB200_OK;
         }
         diag_kernel_for<float2>(st)<<<1, kDiagThreads, kSmemDiagUpd, sm>>>(
-            st->W, ldw, k0, kb, st->Linv + (size_t)bk * NB * NB, st->Uinv + (size_t)bk * NB * NB, st->err, kp1, kp2);
+            st->W, ldw, k0, kb, st->Linv + (size_t)bk * NB * NB, st->Uinv + (size_t)bk * NB * NB, st->err, kp1, kp2,
+            rowex);
         SIEB_NOTE_LAUNCH();
         ctx->prof.end(sm, ev);
         SIEB_TRY_CUDA(cudaGetLastError());
@@ -2620,6 +2688,7 @@ static int mixed_enqueue(DenseSolver* s, MixedState* st, size_t bFlags, int K3) 
             pa.k0 = k0; pa.kb = kb; pa.s0 = s0; pa.np = np;
             pa.nL = (int)blocks_for(m, 32);
             pa.pack = 2;
+            pa.rowex = st->rowex + bk * NB;
             pa.Ah = Ah + (bk % kGroup) * 2 * NB; pa.a_ld = LD; pa.a_r0 = g0; pa.a_lo = LO;
             pa.Bh = Bh + (bk % kGroup) * 2 * NB; pa.b_ld = LD; pa.b_c0 = g0; pa.b_lo = LO;
             pa.fa = fa + (bk % kGroup) * fs;
@@ -3305,7 +3374,7 @@ static int fp64_factorize(DenseSolver* s) {
         }
         diag_kernel_for<double2>(st)<<<1, kDiagThreads, kSmemDiagUpd64, sm>>>(
             st->W64, ldw, k0, kb, st->Linv64 + (size_t)bk * NB * NB, st->Uinv64 + (size_t)bk * NB * NB, st->err, kp,
-            -1);
+            -1, nullptr);
         SIEB_NOTE_LAUNCH();
         ctx->prof.end(sm, ev);
         SIEB_TRY_CUDA(cudaGetLastError());

@@ -27,6 +27,7 @@ struct MixedState {
     double* diag = nullptr;     // butterfly diagonals: U (level1 a,b; level2 e,f) and V, 4*np each
     unsigned* err = nullptr;    // error word (nonzero = failure code)
     unsigned* tri_flags = nullptr;   // per block progress flags (2 * nbl) + 2 tickets
+    int* rowex = nullptr;       // balancing exponents of the FP16 packs, NB per diagonal block
     cplx* vecs = nullptr;       // FP64 work vectors
     int use_tc = 1;
     int blocked = 0;            // grouped block steps with FP16 split packs (the default schedule)

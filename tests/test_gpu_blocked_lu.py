@@ -1,5 +1,8 @@
 """The blocked schedule of the mixed LU (groups of four block steps, FP16
-split packs) at the edges of its groups, and entries far apart in size."""
+split packs) at the edges of its groups, and entries far apart in size.
+
+A one-step bound of 1e-5 leaves two digits to the single-precision factors of
+these well-conditioned systems (5e-8 by an emulation of the split products)."""
 
 import math
 
@@ -76,3 +79,28 @@ def test_packs_out_of_fp16_range(entry, gpu_ctx):
     b = A @ (rng.standard_normal(n) + 1j * rng.standard_normal(n))
     x, _ = _solve(A, b, gpu_ctx, tolerance=1e-10, max_iterations=30)
     assert np.linalg.norm(A @ x - b) <= 1e-10 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("diag", ["", "REC", "COMPACT", "PANELS", "SPLIT=0"])
+@pytest.mark.parametrize("graded", ["rows", "columns", "both"])
+@pytest.mark.parametrize("n", [256, 772, 1024])
+def test_graded_system_one_step(n, graded, diag, gpu_ctx, monkeypatch):
+    """Rows, columns or both scaled by random powers of two within 2^48: an LU of
+    FP32 operands is the same up to those powers, and FP16 packs with a scale per row
+    and column alone leave a residual of 2e-3. A scale repeats every n / 4 rows,
+    which the butterflies mix, so that it survives them and a block of 64 rows holds
+    the whole range. Every diagonal-block kernel, each of which finds the packs' balancing."""
+    if diag:
+        monkeypatch.setenv("SIEB200_DIAG_" + diag.split("=")[0], diag.split("=")[-1] if "=" in diag else "1")
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)) + 3.0 * math.sqrt(n) * np.eye(n)
+    d = 2.0 ** np.round(48.0 * (rng.random((2, n // 4)) - 0.5))
+    d1, d2 = np.tile(d, 4)
+    d1 = d1 if graded != "columns" else np.ones(n)
+    d2 = d2 if graded != "rows" else np.ones(n)
+    A *= np.outer(d1, d2)
+    b = A @ ((rng.standard_normal(n) + 1j * rng.standard_normal(n)) / d2)
+    x, it = _solve(A, b, gpu_ctx, tolerance=1e-5, max_iterations=1)
+    r = A @ x - b
+    assert it == 1 and np.linalg.norm(r) <= 1e-5 * np.linalg.norm(b)
+    assert np.linalg.norm(r / d1) <= 1e-5 * np.linalg.norm(b / d1)
