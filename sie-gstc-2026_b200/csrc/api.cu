@@ -1131,6 +1131,9 @@ int sieb200_far_field(sieb200_ctx* ctx, const sieb200_mesh* mesh, const double* 
                       const double* r_hat, const double* theta_hat, const double* phi_hat,
                       double* f_theta, double* f_phi, double* intensity) {
     SIEB_CHECK(ctx && mesh && j_cur && ndir >= 0, SIEB200_INVALID_ARG, "invalid far-field arguments");
+    SIEB_CHECK(mesh->vertices && mesh->faces && mesh->faces_edges && mesh->num_vertices > 0 && mesh->num_faces > 0 &&
+                   mesh->num_edges > 0,
+               SIEB200_INVALID_ARG, "far-field mesh must contain vertices, faces, and edges");
     SIEB_CHECK(ndir == 0 || (r_hat && theta_hat && phi_hat && f_theta && f_phi && intensity),
                SIEB200_INVALID_ARG, "far-field direction and output arrays must not be null");
     SIEB_CHECK(k0 > 0 && eta0 > 0, SIEB200_INVALID_ARG, "k0 and eta0 must be positive");

@@ -128,3 +128,15 @@ def test_far_field_chunks(name, ndir, k0, gpu_ctx):
     bound = 1e-12 if k0 < 10 else 1e-6  # the rounding of k0 r.r' at phases of 2e7
     for a, b in zip(got, want):
         assert np.abs(a - b).max() <= bound * np.abs(b).max()
+
+
+@pytest.mark.parametrize("ndir", [0, 3])
+def test_far_field_empty_mesh_refused(ndir, gpu_ctx):
+    """A mesh without faces is an error, as in the field evaluation (the split
+    of its faces into chunks would divide by zero)."""
+    import sieb200
+    mesh = sieb200.MeshData(np.zeros((3, 3)), np.zeros((0, 3), np.int32), np.zeros((1, 2), np.int32),
+                            np.zeros((0, 3), np.int32))
+    frames = sieb200.spherical_frames(np.linspace(0.1, 1.0, ndir), np.zeros(ndir))
+    with pytest.raises(sieb200.InvalidArgument):
+        sieb200.far_field(mesh, np.zeros(1, complex), None, 1.0, 376.73, *frames, ctx=gpu_ctx)
