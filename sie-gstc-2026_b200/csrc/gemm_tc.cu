@@ -911,8 +911,6 @@ void gemm_tc_destroy(GemmTC* g) {
 
 void gemm_tc_set_mode(GemmTC* g, int mode) { g->mode = mode; }
 
-bool gemm_tc_default(const GemmTC* g) { return g->mode == 3 && g->c_slots == 4 && g->lolo == 0; }
-
 int gemm_tc_sub(GemmTC* g, cudaStream_t stream, float* C, int64_t ldc, const float* A, const float* B,
                 int64_t M2, int64_t N, int K, int max_ctas, int layout, int64_t shift0) {
     SIEB_CHECK(K % BK == 0 && K > 0, SIEB200_INVALID_ARG, "GEMM K must be a positive multiple of 32");

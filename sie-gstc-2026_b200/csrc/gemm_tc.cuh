@@ -28,8 +28,6 @@ int gemm_tc_sub(GemmTC* g, cudaStream_t stream, float* C, int64_t ldc, const flo
                 const float* B, int64_t M2, int64_t N, int K, int max_ctas = 0, int layout = 0,
                 int64_t shift0 = 0);
 int gemm_tc_check(GemmTC* g, cudaStream_t stream);
-// Whether the default kernel configuration is selected (no switch).
-bool gemm_tc_default(const GemmTC* g);
 
 // Exponent of the scale of a row of L21 or a column of U12 in the FP16 split operands:
 // with it the largest entry, whose exponent is max_exp, falls into [2^14, 2^15).

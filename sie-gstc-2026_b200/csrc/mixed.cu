@@ -81,6 +81,16 @@ static int diag_compact_env() {
     return (e && e[0] == '1') ? 1 : 0;
 }
 
+// Whether a switch of the step-by-step schedules or of their trailing GEMM is
+// set, to whatever value: each asks for those schedules (mixed_enqueue).
+static bool step_schedule_env() {
+    for (const char* name : {"SIEB200_PAIR_UPDATE", "SIEB200_PAIR_MIN", "SIEB200_OVERLAP_MIN", "SIEB200_GEMM_LCOL",
+                             "SIEB200_PANEL_HEAD_MAX", "SIEB200_GEMM_HILO", "SIEB200_TF32_LO_RN", "SIEB200_GEMM_MODE",
+                             "SIEB200_GEMM_SIMT", "SIEB200_GEMM_C_SLOTS", "SIEB200_GEMM_LOLO"})
+        if (getenv(name)) return true;
+    return false;
+}
+
 static void drop_graphs(MixedState* st) {
     for (auto& g : st->graphs) {
         if (g.exec) cudaGraphExecDestroy(g.exec);
@@ -2382,7 +2392,6 @@ int mixed_factorize(DenseSolver* s) {
     st->pair = (pair_env && pair_env[0] == '1') ? 1 : 0;
     const char* pmin_env = getenv("SIEB200_PAIR_MIN");
     st->pair_min = pmin_env ? std::max(0, atoi(pmin_env)) : kPairMinDefault;
-    const bool pmin_env_on = pmin_env && st->pair_min > 0;
     const char* hilo_env = getenv("SIEB200_GEMM_HILO");
     st->hilo = (hilo_env && hilo_env[0] == '0') ? 0 : 1;
     const char* ovl_env = getenv("SIEB200_OVERLAP_MIN");
@@ -2458,9 +2467,8 @@ int mixed_factorize(DenseSolver* s) {
     }
 
     // The blocked schedule (see mixed_enqueue) unless a switch asks for one of
-    // the single-step or pair schedules.
-    st->blocked = st->use_tc && gemm_tc_default(st->gemm) && st->hilo && st->lcol == 1 && !st->pair && !pmin_env_on &&
-                  st->ovl_min == 0 && !st->lo_rn;
+    // the step-by-step schedules.
+    st->blocked = st->use_tc && !step_schedule_env();
 
     // Replay, capture or run eagerly (see MixedState::graphs).
     MixedState::GraphKey key;
@@ -2750,6 +2758,7 @@ static int mixed_enqueue(DenseSolver* s, MixedState* st, size_t bFlags, int K3) 
         return SIEB200_OK;
     }
 
+    // The step-by-step schedules, with split-TF32 operands (step_schedule_env).
     // Right-looking block LU with a lookahead of one block. Step bk: the
     // panels of block bk are formed on the context stream; the next
     // diagonal block takes its update(s) from them and is factored on the
@@ -2774,7 +2783,7 @@ static int mixed_enqueue(DenseSolver* s, MixedState* st, size_t bFlags, int K3) 
     // and runs after odd steps only, for both steps of the pair at once
     // (half the C traffic per flop). The persistent GEMM leaves one SM to
     // the diagonal kernel (whose shared memory keeps it off the GEMM's SMs).
-    // The single-step schedule is the default (SIEB200_PAIR_UPDATE=1 selects
+    // Single steps are the default of these schedules (SIEB200_PAIR_UPDATE=1 selects
     // the pair schedule): on the 6016-unknown system the pair schedule's
     // GEMM runs at 360 TFLOP/s against 297, but the steps without a GEMM put
     // the panels and the diagonal block back to back and the extra updates

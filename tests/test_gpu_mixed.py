@@ -148,6 +148,8 @@ def _pmchwt(level=2, solver="lu_cusolver", rule=5):
 @pytest.mark.parametrize("trailing", ["tc", "tc_pair", "tc_three_product", "tc_load_store", "tc_reduce",
                                       "tc_overlap", "tc_no_lcol", "tc_lcol_gemm", "tc_simt_gemm", "simt"])
 def test_mixed_solver_matches_fp64(trailing, gpu_ctx, monkeypatch):
+    """The grouped schedule (tc), the step-by-step schedules (each other case sets
+    one of their switches) and the SIMT updates."""
     import sieb200
     if trailing == "tc_no_lcol":  # the next panels update the next block column
         monkeypatch.setenv("SIEB200_GEMM_LCOL", "0")
@@ -222,7 +224,13 @@ def test_dense_solver_object_on_device_memory(gpu_ctx):
     s.close()
 
 
-@pytest.mark.parametrize("schedule", ["pair_split", "single_split", "pair_three", "single_three",
+def _set(monkeypatch, **switches):
+    for name, value in switches.items():
+        monkeypatch.setenv("SIEB200_" + name, value)
+
+
+@pytest.mark.parametrize("schedule", ["grouped", "grouped_trsv64", "grouped_diag_rec",
+                                      "pair_split", "single_split", "pair_three", "single_three",
                                       "single_split_overlap", "single_split_trsv64", "pair_then_single",
                                       "single_split_no_lcol", "single_split_lcol_gemm",
                                       "single_split_lcol_side", "single_split_diag_rec",
@@ -230,8 +238,8 @@ def test_dense_solver_object_on_device_memory(gpu_ctx):
 @pytest.mark.parametrize("n", [5, 64, 100, 129, 190, 256, 300, 1000, 2100])
 def test_mixed_ragged_sizes_one_step(n, schedule, gpu_ctx, monkeypatch):
     """Sizes that leave partial sub-blocks, a last row block with one
-    sub-block, and fewer rows than one block, under both trailing-update
-    schedules (pair / single step), both pack layouts (split [hi | lo] /
+    sub-block, and fewer rows than one block, under every trailing-update
+    schedule (grouped, pair, single step), both TF32 pack layouts (split [hi | lo] /
     three-product), the next block column's update in single steps from the
     GEMM (default), the column kernel before or beside it or the panels,
     diagonal blocks by the one-pass 64 x 64 kernel (unrolled or compact)
@@ -243,31 +251,30 @@ def test_mixed_ragged_sizes_one_step(n, schedule, gpu_ctx, monkeypatch):
     triangular solve fails the first bound."""
     import torch
     import sieb200
-    monkeypatch.setenv("SIEB200_PAIR_UPDATE", "1" if schedule.startswith("pair_") and schedule != "pair_then_single"
-                       else "0")
-    # pair steps while the paired update is at least 128 columns wide, single steps after
-    monkeypatch.setenv("SIEB200_PAIR_MIN", "128" if schedule == "pair_then_single" else "0")
-    monkeypatch.setenv("SIEB200_GEMM_HILO", "0" if "_three" in schedule else "1")
-    # overlapped steps: every trailing update at least 64 columns wide skips
-    # the next block row, whose update the next panels take on the side stream
-    monkeypatch.setenv("SIEB200_OVERLAP_MIN", "64" if schedule.endswith("overlap") else "0")
-    monkeypatch.setenv("SIEB200_OVERLAP_SMS", "16")
-    # triangular solves with 64-row CTAs (one sub-block each) or 128-row ones
-    monkeypatch.setenv("SIEB200_TRSV_ROWS", "64" if schedule.endswith("trsv64") else "128")
-    # 128-row triangular solves with the newest coupling folded into
-    # precomputed products (default) or streamed as tiles
-    monkeypatch.setenv("SIEB200_TRSV_FOLD", "0" if schedule.endswith("trsv_stream") else "1")
-    # who updates the next block column below its diagonal block in a single
-    # step: the next panels (0), the GEMM (1, default), col_update_kernel on
-    # the third stream (2) or before the GEMM (3)
-    monkeypatch.setenv("SIEB200_GEMM_LCOL", "0" if schedule.endswith("no_lcol")
-                       else "1" if schedule.endswith("lcol_gemm")
-                       else "2" if schedule.endswith("lcol_side") else "1")
-    # diagonal blocks by the one-pass 64 x 64 kernel, fully unrolled
-    # (default) or in one code path, or by the 2 x 2 recursion over 32 x 32
-    # warp factorizations
-    monkeypatch.setenv("SIEB200_DIAG_REC", "1" if schedule.endswith("diag_rec") else "0")
-    monkeypatch.setenv("SIEB200_DIAG_COMPACT", "1" if schedule.endswith("diag_compact") else "0")
+    if not schedule.startswith("grouped"):
+        _set(monkeypatch,
+             PAIR_UPDATE="1" if schedule.startswith("pair_") and schedule != "pair_then_single" else "0",
+             # pair steps while the paired update is at least 128 columns wide, single steps after
+             PAIR_MIN="128" if schedule == "pair_then_single" else "0",
+             GEMM_HILO="0" if "_three" in schedule else "1",
+             # overlapped steps: every trailing update at least 64 columns wide skips
+             # the next block row, whose update the next panels take on the side stream
+             OVERLAP_MIN="64" if schedule.endswith("overlap") else "0", OVERLAP_SMS="16",
+             # who updates the next block column below its diagonal block in a single
+             # step: the next panels (0), the GEMM (1, default), col_update_kernel on
+             # the third stream (2) or before the GEMM (3)
+             GEMM_LCOL="0" if schedule.endswith("no_lcol") else "2" if schedule.endswith("lcol_side") else "1")
+    _set(monkeypatch,
+         # triangular solves with 64-row CTAs (one sub-block each) or 128-row ones
+         TRSV_ROWS="64" if schedule.endswith("trsv64") else "128",
+         # 128-row triangular solves with the newest coupling folded into
+         # precomputed products (default) or streamed as tiles
+         TRSV_FOLD="0" if schedule.endswith("trsv_stream") else "1",
+         # diagonal blocks by the one-pass 64 x 64 kernel, fully unrolled
+         # (default) or in one code path, or by the 2 x 2 recursion over 32 x 32
+         # warp factorizations
+         DIAG_REC="1" if schedule.endswith("diag_rec") else "0",
+         DIAG_COMPACT="1" if schedule.endswith("diag_compact") else "0")
     rng = np.random.default_rng(n)
     A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)) + 3.0 * math.sqrt(n) * np.eye(n)
     b = rng.standard_normal(n) + 1j * rng.standard_normal(n)
@@ -310,24 +317,28 @@ def test_mixed_split_panels_bit_identical(n, gpu_ctx, monkeypatch):
     code whichever launch it is in, so the factors, and with them the
     one-step solution, are the same bit for bit as with one panels launch:
     for every step split, for the narrower steps only (the switch inside
-    the factorization), and with the head's larger shared-memory request."""
+    the factorization), and with the head's larger shared-memory request. The
+    switch alone selects the step-by-step schedule (in every other variant two
+    more do); the grouped schedule's factors differ in their last bits."""
     import torch
     import sieb200
     rng = np.random.default_rng(400 + n)
     A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)) + 3.0 * math.sqrt(n) * np.eye(n)
     b = rng.standard_normal(n) + 1j * rng.standard_normal(n)
     Z = torch.from_numpy(np.asfortranarray(A).T.copy()).cuda()
-    monkeypatch.setenv("SIEB200_PAIR_MIN", "0")
-    monkeypatch.setenv("SIEB200_GEMM_LCOL", "1")
-    variants = {"one_launch": ("0", "0"), "all_split": ("1000000", "0"),
-                "narrow_split": (str(max(1, n // 2)), "0"), "all_split_big_smem": ("1000000", str(200 * 1024))}
+    variants = {"one_launch": ("0", "0"), "all_split": ("1000000", "0"), "only_switch": ("1000000", "0"),
+                "narrow_split": (str(max(1, n // 2)), "0"), "all_split_big_smem": ("1000000", str(200 * 1024)),
+                "grouped": None}
     out = {}
-    for name, (head_max, smem) in variants.items():
-        monkeypatch.setenv("SIEB200_PANEL_HEAD_MAX", head_max)
-        if smem == "0":
-            monkeypatch.delenv("SIEB200_PANEL_HEAD_SMEM", raising=False)
-        else:
-            monkeypatch.setenv("SIEB200_PANEL_HEAD_SMEM", smem)
+    for name, head in variants.items():
+        for switch in ("PAIR_MIN", "GEMM_LCOL", "PANEL_HEAD_MAX", "PANEL_HEAD_SMEM"):
+            monkeypatch.delenv("SIEB200_" + switch, raising=False)
+        if head:
+            _set(monkeypatch, PANEL_HEAD_MAX=head[0])
+            if name != "only_switch":
+                _set(monkeypatch, PAIR_MIN="0", GEMM_LCOL="1")
+            if head[1] != "0":
+                _set(monkeypatch, PANEL_HEAD_SMEM=head[1])
         s = sieb200.DenseLuSolver(n, "mixed_ir", ctx=gpu_ctx)
         xs = []
         for _ in range(3):  # eager, captured, replayed
@@ -341,6 +352,8 @@ def test_mixed_split_panels_bit_identical(n, gpu_ctx, monkeypatch):
         for x in xs[1:]:
             assert np.array_equal(x, xs[0]), name
         out[name] = xs[0]
+    grouped = out.pop("grouped")
+    assert n < 1000 or not np.array_equal(grouped, out["one_launch"])
     assert np.linalg.norm(A @ out["one_launch"] - b) / np.linalg.norm(b) <= 1e-5
     for name, xs in out.items():
         assert np.array_equal(xs, out["one_launch"]), name
@@ -444,16 +457,19 @@ def test_mixed_adjoint_matches_cusolver_on_pmchwt(gpu_ctx):
     mix.close()
 
 
-@pytest.mark.parametrize("pair", ["0", "1"])
+@pytest.mark.parametrize("pair", ["0", "1", None])
 def test_profile_timeline_orders_the_block_steps(pair, gpu_ctx, monkeypatch):
     """The profiler's timeline: one span per hot launch with start <= end,
     every chain kernel inside the factorization span, one diagonal-block
     kernel per block, one panels launch per block step and one tensor-core
-    trailing update per step but the last two (single-step schedule) or per
-    odd step among those (pair schedule)."""
+    trailing update per step but the last two (single-step schedule, and the
+    grouped one: pair None) or per odd step among those (pair schedule). The
+    single-step schedule moves the whole trailing matrix in every step, the
+    grouped one in every fourth."""
     import torch
     import sieb200
-    monkeypatch.setenv("SIEB200_PAIR_UPDATE", pair)
+    if pair is not None:
+        monkeypatch.setenv("SIEB200_PAIR_UPDATE", pair)
     n = 1000
     rng = np.random.default_rng(7)
     A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)) + 3.0 * math.sqrt(n) * np.eye(n)
@@ -463,6 +479,7 @@ def test_profile_timeline_orders_the_block_steps(pair, gpu_ctx, monkeypatch):
     s.factorize(Z.data_ptr())
     gpu_ctx.synchronize()
     spans = gpu_ctx.profile_timeline()
+    moved = gpu_ctx.profile_read(0)["bytes"]
     gpu_ctx.profile(False)
     s.close()
     assert spans and all(t0 <= t1 for _, t0, t1 in spans)
@@ -477,6 +494,9 @@ def test_profile_timeline_orders_the_block_steps(pair, gpu_ctx, monkeypatch):
     # the last two steps have no columns right of the next block
     expect = (nbl - 2) // 2 if pair == "1" else nbl - 2
     assert sum(1 for sp in spans if sp[0] == 0) == expect
+    m = n - 64 * np.arange(1.0, nbl - 1)
+    single = (4.0 * (2.0 * (2.0 * m * m - 128 * 64) + 3.0 * m * 256)).sum()
+    assert moved == pytest.approx(single, rel=1e-12) if pair == "0" else moved < 0.8 * single
     diag = sorted(t0 for k, t0, _ in spans if k == 3)
     assert diag == [t0 for k, t0, _ in spans if k == 3]  # recorded in step order
 
