@@ -1112,13 +1112,21 @@ int sieb200_gemm_tf32_sub_shifted(sieb200_ctx* ctx, int64_t m2, int64_t n, int k
     SIEB_CHECK(ctx && A && B && C && ldc >= m2 && mode >= 0 && mode <= 5, SIEB200_INVALID_ARG,
                "invalid GEMM arguments");
     SIEB_TRY_CUDA(cudaSetDevice(ctx->device));
+    DeviceBuffer word(ctx->stream);
+    SIEB_RETURN_IF(word.reserve(sizeof(unsigned)));
+    SIEB_TRY_CUDA(cudaMemsetAsync(word.ptr, 0, sizeof(unsigned), ctx->stream));
     GemmTC* g = nullptr;
-    SIEB_RETURN_IF(gemm_tc_create(&g, ctx->stream));
+    SIEB_RETURN_IF(gemm_tc_create(&g));
+    gemm_tc_error_word(g, word.as<unsigned>());
     gemm_tc_set_mode(g, mode >= 4 ? mode - 2 : mode);
-    int st = gemm_tc_sub(g, ctx->stream, C, ldc, A, B, m2, n, k, 0, mode >= 4 ? 1 : 0, col_shift);
-    if (st == SIEB200_OK) st = gemm_tc_check(g, ctx->stream);
+    const int st = gemm_tc_sub(g, ctx->stream, C, ldc, A, B, m2, n, k, 0, mode >= 4 ? 1 : 0, col_shift);
     gemm_tc_destroy(g);
-    return st;
+    SIEB_RETURN_IF(st);
+    unsigned e = 0;
+    SIEB_TRY_CUDA(cudaMemcpyAsync(&e, word.ptr, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
+    SIEB_TRY_CUDA(cudaStreamSynchronize(ctx->stream));
+    SIEB_CHECK(e == 0u, SIEB200_TIMEOUT, "tensor-core GEMM: a pipeline wait exceeded its bound");
+    return SIEB200_OK;
 }
 
 int sieb200_gemm_tf32_sub(sieb200_ctx* ctx, int64_t m2, int64_t n, int k, const float* A,

@@ -1198,8 +1198,7 @@ int block_solve(DenseSolver* s, MixedState* st, int64_t nrhs64, double* Bd, int6
             SIEB_NOTE_LAUNCH();
             SIEB_TRY_CUDA(cudaGetLastError());
         }
-        SIEB_TRY_CUDA(cudaStreamSynchronize(stream));
-        SIEB_RETURN_IF(gemm_tc_check(st->gemm, stream));
+        SIEB_RETURN_IF(mixed_check(s, "batched GMRES refinement"));
     }
     bcopy_kernel<<<gv, 256, 0, stream>>>(n, X, n, B, ldb);
     SIEB_NOTE_LAUNCH();

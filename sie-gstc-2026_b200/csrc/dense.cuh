@@ -41,6 +41,9 @@ struct DenseSolver {
 };
 
 int mixed_factorize(DenseSolver* s);
+// Waits for the context's stream and reports what the mixed solver's kernels left
+// in its error word.
+int mixed_check(DenseSolver* s, const char* what);
 int gmres_c64_prepare(DenseSolver* s);
 int mixed_solve(DenseSolver* s, int64_t nrhs, double* B, int64_t ldb, bool adjoint, double tol,
                 int maxit, int* iters);

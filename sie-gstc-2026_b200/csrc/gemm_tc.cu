@@ -45,7 +45,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigne
     long long it = 0;
     while (!mbar_try_wait(bar, parity)) {
         if (++it > kSpinLimit) {
-            atomicCAS(err, 0u, 3u);
+            atomicCAS(err, 0u, kGemmTimeout);
             return false;
         }
         if ((it & 1023) == 0 && *reinterpret_cast<volatile unsigned*>(err) != 0u) return false;
@@ -835,8 +835,7 @@ int encode_tensor_map_2d(CUtensorMap* map, CUtensorMapDataType type, const void*
 }
 
 struct GemmTC {
-    DeviceBuffer word;
-    unsigned* err = nullptr;
+    unsigned* err = nullptr;  // error word of the kernels' bounded waits (gemm_tc_error_word)
     int mode = 3;  // persistent kernel, reduction epilogue
     int c_slots = 4;  // C slots of the persistent kernel's epilogue (1 or 4)
     int lolo = 0;     // split operands: also the product A_lo B_lo^T
@@ -877,18 +876,10 @@ int launch_persistent(int variant, unsigned grid, cudaStream_t stream, const CUt
     }
 }
 
-int gemm_tc_create(GemmTC** out, cudaStream_t stream) {
+void gemm_tc_error_word(GemmTC* g, unsigned* word) { g->err = word; }
+
+int gemm_tc_create(GemmTC** out) {
     GemmTC* g = new GemmTC();
-    g->word.order = stream;
-    const int st = g->word.reserve(sizeof(unsigned));
-    const cudaError_t e = st == SIEB200_OK ? cudaMemsetAsync(g->word.ptr, 0, sizeof(unsigned), stream) : cudaSuccess;
-    if (st != SIEB200_OK || e != cudaSuccess) {
-        delete g;
-        if (st != SIEB200_OK) return st;
-        set_error(std::string("gemm workspace: ") + cudaGetErrorString(e));
-        return SIEB200_CUDA_ERROR;
-    }
-    g->err = g->word.as<unsigned>();
     const char* env = getenv("SIEB200_GEMM_SIMT");
     if (env && env[0] == '1') g->mode = 0;
     const char* mode_env = getenv("SIEB200_GEMM_MODE");
@@ -1001,17 +992,6 @@ int gemm_half_sub(GemmTC* g, cudaStream_t stream, float* C, int64_t ldc, const _
                                                                    fstride, g->err);
     SIEB_NOTE_LAUNCH();
     SIEB_TRY_CUDA(cudaGetLastError());
-    return SIEB200_OK;
-}
-
-int gemm_tc_check(GemmTC* g, cudaStream_t stream) {
-    unsigned e = 0;
-    SIEB_TRY_CUDA(cudaMemcpyAsync(&e, g->err, sizeof(unsigned), cudaMemcpyDeviceToHost, stream));
-    SIEB_TRY_CUDA(cudaStreamSynchronize(stream));
-    if (e != 0u) {
-        set_error("tensor-core GEMM: a pipeline wait exceeded its bound");
-        return SIEB200_TIMEOUT;
-    }
     return SIEB200_OK;
 }
 

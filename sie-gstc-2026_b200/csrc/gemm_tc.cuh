@@ -12,10 +12,13 @@ namespace sieb200 {
 
 struct GemmTC;
 
-int gemm_tc_create(GemmTC** out, cudaStream_t stream);
+int gemm_tc_create(GemmTC** out);
 void gemm_tc_destroy(GemmTC* g);
-// Returns a SIEB200_* status; the kernel's bounded waits report through an
-// error word checked on the next synchronization (gemm_tc_check).
+// The device word in which the kernels' bounded waits leave kGemmTimeout when
+// they give up (the owner clears and reads it); set before the first launch.
+constexpr unsigned kGemmTimeout = 3;
+void gemm_tc_error_word(GemmTC* g, unsigned* word);
+// Returns a SIEB200_* status.
 // max_ctas > 0 caps the persistent kernel's grid, leaving the other SMs to
 // concurrent work on other streams.
 // layout 0: A and B are one K sweep; layout 1: [hi | lo] halves along K,
@@ -27,7 +30,6 @@ void gemm_tc_destroy(GemmTC* g);
 int gemm_tc_sub(GemmTC* g, cudaStream_t stream, float* C, int64_t ldc, const float* A,
                 const float* B, int64_t M2, int64_t N, int K, int max_ctas = 0, int layout = 0,
                 int64_t shift0 = 0);
-int gemm_tc_check(GemmTC* g, cudaStream_t stream);
 
 // Exponent of the scale of a row of L21 or a column of U12 in the FP16 split operands:
 // with it the largest entry, whose exponent is max_exp, falls into [2^14, 2^15).

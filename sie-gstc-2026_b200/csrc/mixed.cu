@@ -2308,7 +2308,7 @@ void mixed_release(DenseSolver* s) {
     s->ipiv.release(); s->work.release();
 }
 
-static int check_err(DenseSolver* s, const char* what) {
+int mixed_check(DenseSolver* s, const char* what) {
     MixedState* st = state_of(s);
     unsigned e = 0;
     SIEB_TRY_CUDA(cudaMemcpyAsync(&e, st->err, sizeof(unsigned), cudaMemcpyDeviceToHost, s->ctx->stream));
@@ -2319,6 +2319,10 @@ static int check_err(DenseSolver* s, const char* what) {
     }
     if (e == 2u) {
         set_error(std::string(what) + ": a triangular-solve block waited past its bound");
+        return SIEB200_TIMEOUT;
+    }
+    if (e == kGemmTimeout) {
+        set_error(std::string(what) + ": a pipeline wait of the tensor-core GEMM exceeded its bound");
         return SIEB200_TIMEOUT;
     }
     if (e != 0u) {
@@ -2438,7 +2442,8 @@ int mixed_factorize(DenseSolver* s) {
     st->Apack[0] = s->gemm_a.as<float>();
     st->Apack[1] = reinterpret_cast<float*>(s->gemm_a.as<char>() + bApack);
     st->Bpack = s->gemm_b.as<float>();
-    if (st->use_tc && !st->gemm) SIEB_RETURN_IF(gemm_tc_create(&st->gemm, stream));
+    if (st->use_tc && !st->gemm) SIEB_RETURN_IF(gemm_tc_create(&st->gemm));
+    if (st->gemm) gemm_tc_error_word(st->gemm, st->err);
     SIEB_RETURN_IF(lookahead_stream(&ctx->side, &st->side));
     if (!st->ev_cols) {
         SIEB_TRY_CUDA(cudaEventCreateWithFlags(&st->ev_cols, cudaEventDisableTiming));
@@ -2487,7 +2492,7 @@ int mixed_factorize(DenseSolver* s) {
                 g.used = ++st->tick;
                 SIEB_TRY_CUDA(cudaGraphLaunch(g.exec, stream));
                 note_launches(g.launches);
-                return check_err(s, "mixed LU factorization");
+                return mixed_check(s, "mixed LU factorization");
             }
         }
     }
@@ -2522,7 +2527,7 @@ int mixed_factorize(DenseSolver* s) {
     } else {
         SIEB_RETURN_IF(mixed_enqueue(s, st, bFlags, K3));
     }
-    return check_err(s, "mixed LU factorization");
+    return mixed_check(s, "mixed LU factorization");
 }
 
 // Enqueues one mixed factorization on the context stream and the lookahead
@@ -3249,11 +3254,11 @@ static int gmres_ir(DenseSolver* s, cplx* b, int64_t ldb_unused, double tol, int
         add_kernel<<<blocks_for(n, 256), 256, 0, stream>>>(n, w, x);
         SIEB_NOTE_LAUNCH();
         SIEB_TRY_CUDA(cudaGetLastError());
-        SIEB_RETURN_IF(check_err(s, "GMRES refinement"));
+        SIEB_RETURN_IF(mixed_check(s, "GMRES refinement"));
     }
     SIEB_TRY_CUDA(cudaMemcpyAsync(b, x, sizeof(cplx) * n, cudaMemcpyDeviceToDevice, stream));
     if (iters) *iters = total;
-    return check_err(s, "GMRES refinement");
+    return mixed_check(s, "GMRES refinement");
 }
 
 static int fp64_solve(DenseSolver* s, int64_t nrhs, double* B, int64_t ldb, double tol, int maxit, int* iters);
