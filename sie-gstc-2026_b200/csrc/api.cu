@@ -148,6 +148,20 @@ void trim_pool() {
     cudaGetLastError();
 }
 
+int available_memory(size_t* bytes) {
+    size_t free_b = 0, total_b = 0;
+    SIEB_TRY_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    uint64_t reserved = 0, used = 0;
+    cudaMemPool_t p = device_pool();
+    if (p && (cudaMemPoolGetAttribute(p, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+              cudaMemPoolGetAttribute(p, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)) {
+        cudaGetLastError();
+        reserved = used = 0;
+    }
+    *bytes = free_b + (size_t)(reserved > used ? reserved - used : 0);
+    return SIEB200_OK;
+}
+
 int DeviceBuffer::reserve(size_t n) {
     if (n <= bytes && ptr) return SIEB200_OK;
     release();

@@ -1611,7 +1611,8 @@ static int assemble_or_apply(sieb200_ctx* ctx, const sieb200_mesh& mesh, const s
         SIEB_TRY_CUDA(cudaMemcpyAsync(dgl, glt, sizeof(glt), cudaMemcpyHostToDevice, st));
     }
     // (The free memory, whose query takes 0.1 to 11 ms, is asked for only where
-    // the workspace of earlier calls is too small.)
+    // the workspace of earlier calls is too small; that workspace counts as free,
+    // and what it holds is the least a slab takes.)
     const size_t pair_bytes = sizeof(cplx) * 9 * po.NB;
     const size_t most = (size_t)8 << 30;
     auto slab_of = [&](size_t budget) {
@@ -1619,8 +1620,10 @@ static int assemble_or_apply(sieb200_ctx* ctx, const sieb200_mesh& mesh, const s
     };
     int slab = slab_of(most);
     if (ctx->pairs.bytes < pair_bytes * (size_t)slab * nf) {
-        size_t free_b = 0, total_b = 0;
-        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) slab = slab_of(std::min(most, free_b / 3));
+        const size_t held = ctx->pairs.bytes;
+        size_t free_b = 0;
+        if (available_memory(&free_b) == SIEB200_OK)
+            slab = std::max(slab_of(held), slab_of(std::min(most, (free_b + held) / 3)));
     }
     SIEB_RETURN_IF(ctx->pairs.reserve(pair_bytes * (size_t)slab * nf));
     po.pairs = ctx->pairs.as<cplx>();

@@ -810,8 +810,8 @@ static int prepare(DenseSolver* s, MixedState* st, int nrhs, bool* fits) {
     const size_t bU = sizeof(float) * 2 * (size_t)u_rows * kw;
     const size_t need = ((bL + 255) / 256) * 256 + bU;
     if (bs->packs.bytes < need) {
-        size_t free_b = 0, total_b = 0;
-        SIEB_TRY_CUDA(cudaMemGetInfo(&free_b, &total_b));
+        size_t free_b = 0;
+        SIEB_RETURN_IF(available_memory(&free_b));
         const size_t margin = (size_t)2 << 30;
         if (need + margin > free_b + bs->packs.bytes) {
             *fits = false;

@@ -106,6 +106,9 @@ struct DeviceBuffer {
 
 // Returns the pool's unused memory on the current device to the driver.
 void trim_pool();
+// Memory that buffers on the current device can still have: what the driver has
+// free and what the pool keeps unused (which reserve gives back before it fails).
+int available_memory(size_t* bytes);
 
 }  // namespace sieb200
 

@@ -155,3 +155,43 @@ def test_gstc_batch_of_plane_waves_mixed_matches_fp64(gpu_ctx):
         assert np.linalg.norm(a.currents - b.currents) / np.linalg.norm(b.currents) < 1e-9
         assert a.metrics["relative_residual"] <= 1e-10
         assert b.metrics["relative_residual"] <= 1e-10
+
+
+def test_block_solve_counts_pooled_memory_as_free(gpu_ctx):
+    """With the rest of the device taken, the packs (216 MB, and the 2 GB margin) fit only
+    if what closed solvers left in the library's memory pool counts as free:
+    the solve still runs all columns at once (profiled kind 5)."""
+    import torch
+    import sieb200
+    n, nrhs = 2600, 8
+    A = _system(n, 3)
+    B = np.random.default_rng(4).standard_normal((n, nrhs)) + 0j
+    Z = _dev(A)
+
+    def solver():
+        s = sieb200.DenseLuSolver(n, "mixed_ir", ctx=gpu_ctx)
+        s.factorize(Z.data_ptr())
+        X = _dev(B)
+        torch.cuda.synchronize()
+        s.solve(X.data_ptr(), nrhs=nrhs, tolerance=1e-10, max_iterations=30)
+        gpu_ctx.synchronize()
+        return s, X
+
+    for s, _ in [solver() for _ in range(3)]:  # some 900 MB in buffers of the pool, then unused
+        s.close()
+    torch.cuda.empty_cache()
+    packs = 32 * n * n
+    take = torch.cuda.mem_get_info()[0] - (packs + (2 << 30) - (300 << 20))
+    filler = torch.empty(max(take, 0), dtype=torch.uint8, device="cuda")
+    gpu_ctx.profile(True)
+    try:
+        s, X = solver()
+        at_once = gpu_ctx.profile_read(5)["launches"]
+    finally:
+        gpu_ctx.profile(False)
+        del filler
+        torch.cuda.empty_cache()
+    s.close()
+    assert at_once > 0
+    R = B - A @ _host(X, n, nrhs)
+    assert (np.linalg.norm(R, axis=0) <= 2e-10 * np.linalg.norm(B, axis=0)).all()
