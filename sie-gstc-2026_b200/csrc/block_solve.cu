@@ -902,6 +902,7 @@ static int enqueue_triangular(DenseSolver* s, MixedState* st, BlockSolveState* b
         return SIEB200_OK;
     }
     cudaStream_t side = st->side;
+    JoinOnError guard{side};
     const int cap = std::max(1, s->ctx->sm_count - 4);  // SMs left to the diagonal kernels
     SIEB_TRY_CUDA(cudaEventRecord(bs->ev_fork, stream));
     SIEB_TRY_CUDA(cudaStreamWaitEvent(side, bs->ev_fork, 0));
@@ -959,6 +960,7 @@ static int enqueue_triangular(DenseSolver* s, MixedState* st, BlockSolveState* b
     }
     SIEB_TRY_CUDA(cudaEventRecord(bs->ev_join, side));
     SIEB_TRY_CUDA(cudaStreamWaitEvent(stream, bs->ev_join, 0));
+    guard.joined = true;
     return SIEB200_OK;
 }
 

@@ -2535,6 +2535,7 @@ int mixed_factorize(DenseSolver* s) {
 static int mixed_enqueue(DenseSolver* s, MixedState* st, size_t bFlags, int K3) {
     sieb200_ctx* ctx = s->ctx;
     cudaStream_t stream = ctx->stream;
+    JoinOnError guard{st->side, st->side2};
     const int64_t n = st->n, np = st->np, ldw = st->ldw, nbl = st->nbl;
     cudaEvent_t ev_fact;
     ctx->prof.begin(stream, 6, (8.0 / 3.0) * 4.0 * (double)np * np * np, 0.0, &ev_fact);
@@ -2759,6 +2760,7 @@ static int mixed_enqueue(DenseSolver* s, MixedState* st, size_t bFlags, int K3) 
             SIEB_TRY_CUDA(cudaEventRecord(st->ev_pan, st->side));
             SIEB_TRY_CUDA(cudaStreamWaitEvent(stream, st->ev_pan, 0));
         }
+        guard.joined = true;
         ctx->prof.end(stream, ev_fact);
         return SIEB200_OK;
     }
@@ -2919,6 +2921,7 @@ static int mixed_enqueue(DenseSolver* s, MixedState* st, size_t bFlags, int K3) 
         SIEB_TRY_CUDA(cudaEventRecord(st->ev_pan, st->side));
         SIEB_TRY_CUDA(cudaStreamWaitEvent(stream, st->ev_pan, 0));
     }
+    guard.joined = true;
     ctx->prof.end(stream, ev_fact);
     return SIEB200_OK;
 }
@@ -3353,6 +3356,7 @@ static int fp64_factorize(DenseSolver* s) {
     st->diag_compact = diag_compact_env();
     st->diag_rec = 0;  // complex64 only
     SIEB_RETURN_IF(lookahead_stream(&ctx->side, &st->side));
+    JoinOnError guard{st->side};
     if (!st->ev_cols) {
         SIEB_TRY_CUDA(cudaEventCreateWithFlags(&st->ev_cols, cudaEventDisableTiming));
         SIEB_TRY_CUDA(cudaEventCreateWithFlags(&st->ev_diag, cudaEventDisableTiming));
@@ -3453,6 +3457,7 @@ static int fp64_factorize(DenseSolver* s) {
         SIEB_TRY_CUDA(cudaEventRecord(st->ev_pan, st->side));
         SIEB_TRY_CUDA(cudaStreamWaitEvent(stream, st->ev_pan, 0));
     }
+    guard.joined = true;
     ctx->prof.end(stream, ev_fact);
     unsigned e = 0;
     SIEB_TRY_CUDA(cudaMemcpyAsync(&e, st->err, sizeof(unsigned), cudaMemcpyDeviceToHost, stream));

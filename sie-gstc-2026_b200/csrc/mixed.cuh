@@ -107,6 +107,20 @@ struct MixedState {
     double2* Uinv64 = nullptr;
 };
 
+// Waits for the lookahead streams where a call returns before it has joined them: a
+// failed call's buffers go back to the pool in the order of the context's
+// stream, and another stream could have them while the work on these goes on.
+struct JoinOnError {
+    cudaStream_t a = nullptr, b = nullptr;
+    bool joined = false;
+    ~JoinOnError() {
+        if (joined) return;
+        if (a) cudaStreamSynchronize(a);
+        if (b) cudaStreamSynchronize(b);
+        cudaGetLastError();
+    }
+};
+
 // Index quadruple of a depth-2 butterfly: {i, i+q, i+2q, i+3q}, q = np/4.
 // Transposed application T^T = L1^T L2^T (first the two level-2 blocks, then
 // level 1) of a butterfly with diagonals d = [a (h), b (h), e (h), f (h)],
