@@ -481,7 +481,6 @@ __global__ void bcopy_kernel(int64_t n, const cplx* __restrict__ X, int64_t ldx,
 // Shared layouts: A as [k][row] with rows padded to 66 (conflict-free
 // 16-byte fragment loads), X as [col][k] with k padded to 20.
 constexpr int ZD_BM = 64, ZD_BN = 64, ZD_BK = 16, ZD_THREADS = 128, ZD_STAGES = 3;
-constexpr int kSms = 148;
 constexpr int ZD_ALD = ZD_BM + 2, ZD_XLD = ZD_BK + 4;
 constexpr int ZD_STAGE_A = ZD_BK * ZD_ALD, ZD_STAGE_X = ZD_BN * ZD_XLD;  // complex entries
 constexpr int kSmemZgemmDmma = ZD_STAGES * (ZD_STAGE_A + ZD_STAGE_X) * 16;
@@ -681,8 +680,10 @@ static bool zgemm_dmma_selected() {
     return !(e && e[0] == '0');
 }
 
-static int zgemm_dmma_attributes() {
+// Once per device: the kernels' shared memory and the SM count (optional).
+static int zgemm_dmma_attributes(int* sms = nullptr) {
     static bool attr_set[64] = {};
+    static int sm_count[64] = {};
     int dev = 0;
     SIEB_TRY_CUDA(cudaGetDevice(&dev));
     if (!attr_set[dev & 63]) {
@@ -690,8 +691,10 @@ static int zgemm_dmma_attributes() {
                                            kSmemZgemmDmma));
         SIEB_TRY_CUDA(cudaFuncSetAttribute(zgemm_dmma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            kSmemZgemmDmma));
+        SIEB_TRY_CUDA(cudaDeviceGetAttribute(&sm_count[dev & 63], cudaDevAttrMultiProcessorCount, dev));
         attr_set[dev & 63] = true;
     }
+    if (sms) *sms = sm_count[dev & 63];
     return SIEB200_OK;
 }
 
@@ -706,7 +709,8 @@ int zgemm_device(cudaStream_t stream, int64_t m, int64_t nc, int64_t kdim, const
     const bool aligned = ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(X) |
                            reinterpret_cast<uintptr_t>(C)) & 15) == 0;
     if (zgemm_dmma_selected() && aligned && nc < 65536ll * ZD_BN) {
-        SIEB_RETURN_IF(zgemm_dmma_attributes());
+        int sms = 0;
+        SIEB_RETURN_IF(zgemm_dmma_attributes(&sms));
         dim3 grid(nblk(m, ZD_BM), nblk(nc, ZD_BN));
         // Few tiles leave SMs idle (two CTAs fit on one): given a scratch
         // buffer, K is then split over blockIdx.z, at least 128 products each,
@@ -714,7 +718,7 @@ int zgemm_device(cudaStream_t stream, int64_t m, int64_t nc, int64_t kdim, const
         // unsplit and split: K = 1920 300 and 75 us, 2940 463 and 150 us,
         // 6000 933 and 562 us.
         const int64_t tiles = (int64_t)grid.x * grid.y;
-        const int64_t parts = scratch ? std::min<int64_t>({16, 2 * kSms / tiles, kdim / 128}) : 1;
+        const int64_t parts = scratch ? std::min<int64_t>({16, 2 * sms / tiles, kdim / 128}) : 1;
         if (parts >= 2) {
             const int64_t kc = ((kdim + parts - 1) / parts + ZD_BK - 1) / ZD_BK * ZD_BK;
             grid.z = (unsigned)((kdim + kc - 1) / kc);
