@@ -1,14 +1,17 @@
 // Phase factors and reciprocal square roots of the quadrature kernels.
 //
-// exp(j k x) for many x and one k: not a sincos of the rounded product k x.
-// x k kTurn / (2 pi) is split by FMAs into a step number and a remainder in
+// exp(j k x) for many x and one k: not a sincos of the rounded product k x but a
+// table-driven reduction (P. T. P. Tang, "Table-lookup algorithms for elementary
+// functions and their error analysis", 10th IEEE Symposium on Computer Arithmetic,
+// 1991). x k kTurn / (2 pi) is split by FMAs into a step number and a remainder in
 // [-1/2, 1/2] that keeps the product's low bits; the remainder's sine and
 // cosine - 1 are short polynomials (Chebyshev interpolation over the
 // remainder's range, errors 3.3e-17 and 1e-19) and the step's rotation comes
 // from a table of kTurn entries in shared memory. 15 FP64 instructions, one of
-// them rounding at the size of the result. The table is kept kTurnCopies
-// times, copy c in the 16-byte bank group c, so that a lane reading copy
-// lane % kTurnCopies meets no bank conflict whatever the steps are.
+// them rounding at the size of the result; absolute error below 4e-16 whatever the
+// phase. The table is kept kTurnCopies times, copy c in the 16-byte bank group c, so
+// that a lane reading copy lane % kTurnCopies meets no bank conflict whatever the
+// steps are.
 #pragma once
 
 #include <cmath>
@@ -61,8 +64,10 @@ __device__ __forceinline__ void phase_cs(const double2* lane_tab, const Wave& w,
     s = fma(cs.y, cf, fma(cs.x, sf, cs.y));
 }
 
-// 1/sqrt(x): the hardware's approximate reciprocal square root refined by one
-// third-order step, y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2.
+// 1/sqrt(x): the hardware's approximate reciprocal square root (20 bits) refined by one
+// step of Chebyshev's third-order iteration (J. F. Traub, "Iterative Methods for
+// the Solution of Equations", 1964) for y^-2 = x: y (1 + e/2 + 3 e^2/8) with
+// e = 1 - x y^2. Relative error below 1.7e-16.
 __device__ __forceinline__ double rsqrt_refined(double x) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
