@@ -67,9 +67,10 @@ def _butterfly(n, offset):
 
 
 @pytest.mark.parametrize("entry", [500.0, 2000.0])
-def test_packs_out_of_fp16_range(entry, gpu_ctx):
+def test_packs_out_of_fp16_range(entry, gpu_ctx, monkeypatch):
     """A transformed matrix whose L21 holds one entry far above its neighbours in
-    the row: refined to 1e-10 alike."""
+    the row, which leaves FP16's range in an unscaled pack: refined to 1e-10 in as many
+    iterations as with TF32 operands (the step-by-step schedule)."""
     n = 192
     rng = np.random.default_rng(5)
     W = np.eye(n) + 0.01 * (rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)))
@@ -77,8 +78,11 @@ def test_packs_out_of_fp16_range(entry, gpu_ctx):
     L[130, 7] = entry
     A = np.linalg.solve(_butterfly(n, 0), L @ W) @ np.linalg.inv(_butterfly(n, 4 * n)).T
     b = A @ (rng.standard_normal(n) + 1j * rng.standard_normal(n))
-    x, _ = _solve(A, b, gpu_ctx, tolerance=1e-10, max_iterations=30)
+    x, it = _solve(A, b, gpu_ctx, tolerance=1e-10, max_iterations=30)
     assert np.linalg.norm(A @ x - b) <= 1e-10 * np.linalg.norm(b)
+    monkeypatch.setenv("SIEB200_PAIR_UPDATE", "0")
+    _, it_tf32 = _solve(A, b, gpu_ctx, tolerance=1e-10, max_iterations=30)
+    assert it <= it_tf32
 
 
 @pytest.mark.parametrize("diag", ["", "REC", "COMPACT", "PANELS", "SPLIT=0"])
