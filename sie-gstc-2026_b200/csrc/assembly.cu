@@ -431,13 +431,14 @@ constexpr int kFarSmemMax = kTurnBytes + (int)sizeof(double) * 3 * kMaxQ * 32;
 //    other's transposes and both are written from one evaluation (m <= n);
 //  * phase factors and 1/R without library calls (phase.cuh); BIG falls back
 //    to sincos(k R) for meshes whose phases would not fit its step number.
-// Measured: the 2000-face sphere with 61 points and two wavenumbers 54 ms (212 ms
+// Measured: the 2000-face sphere with 61 points and two wavenumbers 54.4 ms (212 ms
 // for the kernel this replaces: a warp per ordered pair, a test point per lane, sincos
 // and division from the math library); the 2880-face SIE-GSTC sphere with
-// equal wavenumbers 70 ms (435 ms). The FP64 pipe is busy 64 % of the cycles; what is
-// left is the latency of dependent FP64 instructions: 128 registers per thread (16 warps
-// per SM) gave 75 and 54 ms, unrolling by four 70 and 55 ms, so neither more
-// warps nor more independent points fill it.
+// equal wavenumbers 69.7 ms (435 ms). The FP64 pipe is busy 66 and 64 % of the cycles;
+// what is left is the latency of dependent FP64 instructions. Three CTAs per SM cap a
+// thread at 168 registers, which spills 732 bytes with two wavenumbers and 36 with
+// one. The same kernel with four CTAs per SM 54.9 and 75.0 ms, with two 57.6 and
+// 65.9 ms, with the source points unrolled by four 51.7 and 70.1 ms.
 template <int NK, int NT, bool ROT, bool BIG>
 __global__ void __launch_bounds__(kFarWarps * 32, 3)
 far_pairs_kernel(const FaceGeom* __restrict__ geom, const d3* __restrict__ qp, const RuleWeights rw, int Q, int nf,
