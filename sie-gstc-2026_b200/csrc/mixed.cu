@@ -252,7 +252,7 @@ __device__ __forceinline__ float larger(double2 v) { return (float)fmax(fabs(v.x
 // pivot's exponent would carry it into L21). Emulated with exact accumulation, 256
 // unknowns, rows or rows and columns scaled within 2^40 (2^48), one preconditioned
 // step: residual 5e-8, as unscaled and as with TF32 operands; without balancing
-// 1e-5 (2e-3). Cost: 7.17 and 7.20 ms, N = 6000 factor and solve. Warp 0: m0 and m1 the largest magnitudes of rows lane and lane + 32.
+// 1e-5 (2e-3). Cost: 7.10 and 7.15 ms, N = 6000 factor and solve. Warp 0: m0 and m1 the largest magnitudes of rows lane and lane + 32.
 constexpr int kBalanceMax = 60;  // keeps every exponent of the packs within pow2f's range twice over
 __device__ __forceinline__ void row_exponents(float m0, float m1, int lane, int* __restrict__ ex) {
     const int e0 = exponent_of(m0), e1 = exponent_of(m1);
