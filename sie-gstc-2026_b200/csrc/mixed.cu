@@ -252,7 +252,8 @@ __device__ __forceinline__ float larger(double2 v) { return (float)fmax(fabs(v.x
 // pivot's exponent would carry it into L21). Emulated with exact accumulation, 256
 // unknowns, rows or rows and columns scaled within 2^40 (2^48), one preconditioned
 // step: residual 5e-8, as unscaled and as with TF32 operands; without balancing
-// 1e-5 (2e-3). Cost: 7.10 and 7.15 ms, N = 6000 factor and solve. Warp 0: m0 and m1 the largest magnitudes of rows lane and lane + 32.
+// 1e-5 (2e-3). Cost: 7.17 and 7.20 ms, N = 6000 factor and solve.
+// Called by one warp, m0 and m1 the largest magnitudes of rows lane and lane + 32.
 constexpr int kBalanceMax = 60;  // keeps every exponent of the packs within pow2f's range twice over
 __device__ __forceinline__ void row_exponents(float m0, float m1, int lane, int* __restrict__ ex) {
     const int e0 = exponent_of(m0), e1 = exponent_of(m1);
@@ -890,21 +891,20 @@ struct PanelArgs {
     int b_first = 0, nl_run = 0;
 };
 
-// v times 2^e as h + 2^-11 l in FP16, both rounded to nearest. The power of two in
-// two factors, since e may be out of pow2f's range.
-__device__ __forceinline__ void split_half(float2 v, int e, __half2& h, __half2& l) {
-    const float s0 = pow2f(e >> 1), s1 = pow2f(e - (e >> 1));
+// v s0 s1 as h + 2^-11 l in FP16, both rounded to nearest (powers of two: a line's
+// scale, then an index's balancing; their product may be out of range).
+__device__ __forceinline__ void split_half(float2 v, float s0, float s1, __half2& h, __half2& l) {
     v = make_float2(v.x * s0 * s1, v.y * s0 * s1);
     h = __floats2half2_rn(v.x, v.y);
     const float2 r = __half22float2(h);
     l = __floats2half2_rn((v.x - r.x) * 2048.f, (v.y - r.y) * 2048.f);
 }
 
-// FP16 scale exponents of the 32 lines (rows of L21, columns of U12) a panels CTA holds in
+// FP16 scales of the 32 lines (rows of L21, columns of U12) a panels CTA holds in
 // shared memory, line i at lines[i][0 .. NB), after balancing by 2^bal[k]: eight
-// lanes per line, result in ex[32]; f receives the reciprocals of the `count` first.
+// lanes per line, result in sc[32]; f receives the reciprocals of the `count` first.
 template <class L>
-__device__ __forceinline__ void line_exponents(const L& lines, const int* bal, int* ex, float* f, int64_t count) {
+__device__ __forceinline__ void line_scales(const L& lines, const int* bal, float* sc, float* f, int64_t count) {
     const int line = threadIdx.x >> 3, part = threadIdx.x & 7;
     int mx = -1000;
 #pragma unroll
@@ -916,7 +916,7 @@ __device__ __forceinline__ void line_exponents(const L& lines, const int* bal, i
     for (int o = 1; o < 8; o <<= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     if (part == 0) {
         const int e = mx == -1000 ? 0 : half_exponent(mx);
-        ex[line] = e;
+        sc[line] = pow2f(e);
         if (line < count) f[line] = pow2f(-e);
     }
     __syncthreads();
@@ -1063,15 +1063,16 @@ __device__ __forceinline__ void panel_L_body(T* __restrict__ W, int64_t ldw, con
     if (!pa.pack) return;
     if constexpr (std::is_same<T, float2>::value) {
         if (pa.pack == 2) {
-            __shared__ int ex[32];
-            line_exponents(Ar, bal, ex, pa.fa + (rb - pa.a_r0), np - rb);
-            const int c = tid % NB, bc = bal[c];
+            __shared__ float sc[32];
+            line_scales(Ar, bal, sc, pa.fa + (rb - pa.a_r0), np - rb);
+            const int c = tid % NB;
+            const float sb = pow2f(bal[c]);
 #pragma unroll 2
             for (int rr = tid / NB; rr < 32; rr += kPanelThreads / NB) {
                 const int64_t gr = rb + rr;
                 if (gr >= np) break;
                 __half2 h, l;
-                split_half(Ar[rr][c], ex[rr] + bc, h, l);
+                split_half(Ar[rr][c], sc[rr], sb, h, l);
                 __half2* row0 = reinterpret_cast<__half2*>(pa.Ah + 2 * (gr - pa.a_r0) * pa.a_ld) + c;
                 __half2* row1 = reinterpret_cast<__half2*>(pa.Ah + (2 * (gr - pa.a_r0) + 1) * pa.a_ld) + c;
                 const int64_t lo = pa.a_lo / 2;
@@ -1229,10 +1230,11 @@ __device__ __forceinline__ void panel_U_body(T* __restrict__ W, int64_t ldw, con
 #pragma unroll
         for (int j = 0; j < 2; ++j) Ac[2 * tx + j][row[i]] = acc[i][j];
     __syncthreads();
-    __shared__ int ex[32];
+    __shared__ float sc[32];
     if constexpr (std::is_same<T, float2>::value) {
-        if (pa.pack == 2) line_exponents(Ac, bal, ex, pa.fb + (cb - pa.b_c0), np - cb);
+        if (pa.pack == 2) line_scales(Ac, bal, sc, pa.fb + (cb - pa.b_c0), np - cb);
     }
+    const float sb = pa.pack == 2 ? pow2f(bal[tid % NB]) : 0.f;  // the row of all of this thread's entries
     for (int e = tid; e < 32 * NB; e += blockDim.x) {
         const int r = e % NB, c = e / NB;
         const int64_t gc = cb + c;
@@ -1242,7 +1244,7 @@ __device__ __forceinline__ void panel_U_body(T* __restrict__ W, int64_t ldw, con
         if constexpr (std::is_same<T, float2>::value) {
             if (pa.pack == 2) {
                 __half2 h, l;
-                split_half(v, ex[c] + bal[r], h, l);
+                split_half(v, sc[c], sb, h, l);
                 __half2* col = reinterpret_cast<__half2*>(pa.Bh + (gc - pa.b_c0) * pa.b_ld) + r;
                 col[0] = h;
                 col[pa.b_lo / 2] = l;
