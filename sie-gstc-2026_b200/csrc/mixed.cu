@@ -3485,8 +3485,12 @@ constexpr int kFp64StepCols = 32;
 // Up to this many right-hand sides the refinement's residual is one matvec
 // per column, each at the rate Z comes from memory (18, 34 and 95 us at 1920,
 // 2940 and 6000 unknowns), above it one GEMM, whose 64-column tiles take 75, 150 and
-// 562 us however few of the columns there are.
+// 562 us however few of the columns there are. Small systems take the GEMM for fewer
+// columns, since a matvec is two launches whatever its size: whole solves by matvecs and
+// by GEMM with 2 and 4 columns 108 and 142, 106 and 127 us at 60 unknowns, 123 and 160, 130
+// and 150 us at 128, 145 and 191, 164 and 191 us at 200.
 constexpr int kFp64MatvecCols = 4;
+inline int fp64_matvec_cols(int64_t n) { return (int)std::min<int64_t>(kFp64MatvecCols, 1 + n / 64); }
 
 // Y (np x nrhs, ldy) <- W^{-1} Y with the complex128 factors; T: np x nrhs
 // scratch (ldy) when nrhs <= kFp64StepCols.
@@ -3577,7 +3581,7 @@ static int fp64_solve(DenseSolver* s, int64_t nrhs64, double* Bd, int64_t ldb, d
     }
     int it = 0;
     double sign = 1.0;  // of the residual in R
-    const bool by_column = nrhs <= kFp64MatvecCols;
+    const bool by_column = nrhs <= fp64_matvec_cols(n);
     std::vector<cplx> hr(blk);
     for (;;) {
         // correction D = V W^{-1} U^T R, X += D
