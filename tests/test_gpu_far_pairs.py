@@ -17,6 +17,7 @@ C0 = 299792458.0
 def _mesh(name):
     import sieb200
     return {"ico20": lambda: sieb200.icosphere(0.5, 0), "geo180": lambda: sieb200.geodesic_sphere(0.5, 3),
+            "geo500": lambda: sieb200.geodesic_sphere(0.5, 5),
             "spindle90": lambda: sieb200.revolved_spindle(0.6, 60.0, n_axial=6, n_azimuth=9)}[name]()
 
 
@@ -155,7 +156,7 @@ def test_surface_fields_large_phase(name, limit, gpu_ctx):
     assert np.abs(H - Ho).max() <= 32 * ULP * phase * np.abs(Ho).max()
 
 
-@pytest.mark.parametrize("name", ["ico20", "geo180", "spindle90"])
+@pytest.mark.parametrize("name", ["ico20", "geo180", "geo500", "spindle90"])
 @pytest.mark.parametrize("ndir", [1, 127, 129, 1000])
 @pytest.mark.parametrize("k0", [3.0, "limit", 4.0e7])
 def test_far_field_chunks(name, ndir, k0, gpu_ctx):
