@@ -1911,7 +1911,8 @@ __device__ void add_near_fields(const FaceGeom& g, d3 r, const cplx* __restrict_
 }
 
 // One CTA per observation point and face chunk (blockIdx.y), one thread per
-// face; the chunk's E and H go to part[point][chunk][12]. Bound: the FP64
+// face; the chunk's E and H go to part[point][chunk][12], or with one chunk to E and H
+// themselves. Bound: the FP64
 // pipe, 52 instructions per kernel value (the sums are those of the assembly,
 // so the three half-RWG integrals cost nothing per value). A face whose
 // centroid is within 0.1 lambda of the point takes the extracted kernel
@@ -1922,7 +1923,7 @@ __global__ void __launch_bounds__(kFieldThreads, 4)
 surface_fields_kernel(const FaceGeom* __restrict__ geom, const d3* __restrict__ qp, const RuleWeights rw, int Q, int nf,
                       const double* __restrict__ fs, int ld, int faces_per_chunk, const d3* __restrict__ obs,
                       const cplx* __restrict__ J, const cplx* __restrict__ M, const FieldConsts fc, const Wave wave,
-                      double* __restrict__ part) {
+                      double* __restrict__ part, double* __restrict__ E, double* __restrict__ H) {
     __shared__ __align__(16) double2 tab[kTurn * kTurnCopies];
     __shared__ double red[kFieldThreads / 32][12];
     fill_turn_table(tab);
@@ -2019,7 +2020,9 @@ surface_fields_kernel(const FaceGeom* __restrict__ geom, const d3* __restrict__ 
     if (threadIdx.x < 12) {
         double t = 0.0;
         for (int w = 0; w < kFieldThreads / 32; ++w) t += red[w][threadIdx.x];
-        part[((size_t)blockIdx.x * gridDim.y + blockIdx.y) * 12 + threadIdx.x] = t;
+        const int j = threadIdx.x;
+        if (gridDim.y == 1) (j < 6 ? E : H)[6 * (size_t)blockIdx.x + j % 6] = t;
+        else part[((size_t)blockIdx.x * gridDim.y + blockIdx.y) * 12 + j] = t;
     }
 }
 
@@ -2092,7 +2095,7 @@ int surface_fields_device(sieb200_ctx* ctx, const sieb200_mesh& mesh, const doub
     const size_t b_obs = sizeof(d3) * (size_t)nobs, b_cur = sizeof(cplx) * (size_t)ne;
     const size_t b_out = sizeof(cplx) * 3 * (size_t)nobs;
     const size_t b_fs = sizeof(double) * (size_t)(kFieldRows + 3 * Q) * ld;
-    const size_t b_part = sizeof(double) * 12 * (size_t)nobs * chunks;
+    const size_t b_part = chunks == 1 ? 0 : sizeof(double) * 12 * (size_t)nobs * chunks;
     SIEB_RETURN_IF(buf.reserve(2 * b_cur + 2 * b_out + b_fs + b_part + b_obs));
     char* b = buf.as<char>();
     cplx* dJ = reinterpret_cast<cplx*>(b);
@@ -2115,12 +2118,15 @@ int surface_fields_device(sieb200_ctx* ctx, const sieb200_mesh& mesh, const doub
     const bool big = !((double)fc.k * 4.0 * far < kPhaseMax);
     auto* kernel = big ? surface_fields_kernel<true> : surface_fields_kernel<false>;
     kernel<<<dim3((unsigned)nobs, (unsigned)chunks), kFieldThreads, 0, st>>>(
-        geom, qp, make_rule_weights(wts, Q), Q, nf, fs, ld, per_chunk, dobs, dJ, dM, fc, make_wave((double)fc.k), part);
+        geom, qp, make_rule_weights(wts, Q), Q, nf, fs, ld, per_chunk, dobs, dJ, dM, fc, make_wave((double)fc.k), part,
+        reinterpret_cast<double*>(dE), reinterpret_cast<double*>(dH));
     SIEB_NOTE_LAUNCH();
     SIEB_TRY_CUDA(cudaGetLastError());
-    surface_fields_finish_kernel<<<(unsigned)((nobs * 12 + 255) / 256), 256, 0, st>>>(part, nobs, chunks, dE, dH);
-    SIEB_NOTE_LAUNCH();
-    SIEB_TRY_CUDA(cudaGetLastError());
+    if (chunks > 1) {
+        surface_fields_finish_kernel<<<(unsigned)((nobs * 12 + 255) / 256), 256, 0, st>>>(part, nobs, chunks, dE, dH);
+        SIEB_NOTE_LAUNCH();
+        SIEB_TRY_CUDA(cudaGetLastError());
+    }
     SIEB_TRY_CUDA(cudaMemcpyAsync(E_out, dE, b_out, cudaMemcpyDeviceToHost, st));
     SIEB_TRY_CUDA(cudaMemcpyAsync(H_out, dH, b_out, cudaMemcpyDeviceToHost, st));
     SIEB_TRY_CUDA(cudaStreamSynchronize(st));
